@@ -1,0 +1,61 @@
+"""Rys quadrature kernels against the FP64 oracle where they can go wrong:
+output blocks with fewer quartets than lanes and with a ragged last batch,
+partner records without a common S or with only some components present (the
+per-component path), very short and very long distances (both branches of the
+root tables), and range separation."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+
+import helpers
+from vlxb import basis, fock, lists
+from vlxb._lib import lib
+
+pytestmark = pytest.mark.gpu
+RTOL = 1e-10  # the suite's FP64 bar: 1e-10 of the largest element
+
+
+def close(got, exp):
+    return not exp.size or float(np.abs(got - exp).max()) <= RTOL * float(np.abs(exp).max()) + 1e-14
+
+
+def system(atoms, degree, side, seed, uneven):
+    """Two shells per type; `uneven`: S and Q differ between the components of
+    a pair (so a pair splits into records with partial component masks)."""
+    lib().init(0)
+    wl = basis.config_custom(atoms, max(side, 3.0), {0: 1, 1: 1, 2: 1}, degree, 0.4, 3.0, max(1, atoms), 1e-12, seed)
+    if atoms == 2:  # a fixed separation: `side` bohr along one diagonal
+        wl.mol.coords[1] = wl.mol.coords[0] + side / np.sqrt(3.0)
+    rl = lists.build_lists(wl.mol, wl.D, wl.threshold, fock.gpu_schwarz_fn())
+    if uneven:
+        for key, kp in rl.kpartners.items():
+            na, nb = lists.NCART[lists.LV[key[0]]], lists.NCART[lists.LV[key[1]]]
+            first = np.repeat(np.arange(len(kp.counts)), kp.counts.astype(np.int64))
+            c = (first % na) * nb + kp.Dinds.astype(np.int64) % nb
+            kp.pdata = kp.pdata * (1.0 + 0.05 * c)
+            kp.Q = kp.Q * np.where(c % 3 == 1, 0.5, 1.0)
+            order = np.lexsort((-kp.Q, first))
+            kp.Dinds, kp.Q, kp.pdata = kp.Dinds[order], kp.Q[order].copy(), kp.pdata[order].copy()
+    return wl, rl
+
+
+@pytest.mark.parametrize("atoms,degree,side,uneven,omega", [
+    (1, 1, 2.0, False, 0.0),    # one quartet per block
+    (1, 1, 2.0, True, 0.4),
+    (2, 2, 1.2, True, 0.0),
+    (2, 2, 30.0, False, 0.0),   # T beyond every root table
+    (3, 3, 4.0, False, 0.33),   # 81 quartets per block: a ragged last batch for every root count
+])
+def test_exchange_rys_vs_oracle(atoms, degree, side, uneven, omega):
+    wl, rl = system(atoms, degree, side, 3 + atoms, uneven)
+    dl = fock.to_device(rl)
+    runs = []
+    for _ in range(2):
+        _, matK = fock.build_jk(dl, do_j=False, omega=omega)
+        torch.cuda.synchronize()
+        runs.append({k: v.cpu().numpy() for k, v in matK.items()})
+    _, oK = helpers.oracle_jk_all(rl, omega=omega)
+    for k in oK:
+        assert np.array_equal(runs[0][k], runs[1][k]), k
+        assert close(runs[0][k], oK[k]), (k, float(np.abs(runs[0][k] - oK[k]).max()), float(np.abs(oK[k]).max()))

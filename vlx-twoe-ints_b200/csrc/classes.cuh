@@ -1,15 +1,8 @@
 // Per-class host drivers: regroup the caller's lists on the device, then
 // launch the class's integral kernel, all on the caller's stream.
 #pragma once
-#include <atomic>
-
-#include "col_kernels.cuh"
 #include "engine.cuh"
-#include "jk_kernels.cuh"
-#include "jtma_kernels.cuh"
-#include "md_kernels.cuh"
-#include "jgrad_kernels.cuh"
-#include "kgrad_kernels.cuh"
+#include "launch.cuh"
 
 namespace vlxb {
 
@@ -63,30 +56,9 @@ struct ExchangeArgs {
     const double* maxD_mol;         // [molecules] max |D| bound of each molecule
 };
 
-// The staged Coulomb kernel's shared memory exceeds the 48 KB default for
-// kets with d functions: raise the limit once per device for each of its
-// two instantiations.
-template <int LA, int LB, int LC, int LD>
-int jtma_prepare_launch()
-{
-    static std::atomic<unsigned long long> done{0};
-    int dev = 0;
-    VLXB_CHECK_CUDA(cudaGetDevice(&dev));
-    const unsigned long long bit = 1ull << (dev & 63);
-    if (done.load(std::memory_order_acquire) & bit) return VLXB_OK;
-    const int smem = (int)JTmaShape<LC, LD>::SMEM;
-    VLXB_CHECK_CUDA(cudaFuncSetAttribute(coulomb_tma_kernel<LA, LB, LC, LD, 0>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    VLXB_CHECK_CUDA(cudaFuncSetAttribute(coulomb_tma_kernel<LA, LB, LC, LD, 1>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    done.fetch_or(bit, std::memory_order_acq_rel);
-    return VLXB_OK;
-}
-
 // Coulomb class call on a given arena (pool, static or measuring) with given
 // Boys tables and quartet counter (may be null).  G = 1: the bra-centre
-// derivatives of J instead (coulomb_grad_kernel), written to
-// a.mat_J[k * gstride + o], k = 0..5.
+// derivatives of J instead, written to a.mat_J[k * gstride + o], k = 0..5.
 template <int LA, int LB, int LC, int LD, int G = 0>
 int run_coulomb_impl(const CoulombArgs& a, cudaStream_t st, Arena& ar, const BoysTabs& tab,
                      unsigned long long* qc, double cut, int64_t gstride = 0)
@@ -134,52 +106,14 @@ int run_coulomb_impl(const CoulombArgs& a, cudaStream_t st, Arena& ar, const Boy
                   kd.Dh, kd.tpre};
     int grid = launch_grid_limit();
     if ((int64_t)grid > (int64_t)a.n_ab) grid = (int)a.n_ab;
-    unsigned long long* kerr = kernel_errors_device();
-    if (jvar == 3 && !kerr) return VLXB_ECUDA;
     for (int pm = 0; pm < (cut > 0.0 ? 2 : 1); pm++) {
-        if constexpr (G == 1) {
-            constexpr int GT = JGradShape<LA, LB, LC, LD>::THREADS;
-            if (pm == 0)
-                coulomb_grad_kernel<LA, LB, LC, LD, 0><<<grid, GT, 0, st>>>(bra, ket, a.mat_J, gstride, a.thr, tab,
-                                                                            cut);
-            else
-                coulomb_grad_kernel<LA, LB, LC, LD, 1><<<grid, GT, 0, st>>>(bra, ket, a.mat_J, gstride, a.thr, tab,
-                                                                            cut);
-        } else if (jvar == 2) {
-            if (pm == 0)
-                coulomb_md_kernel<LA, LB, LC, LD, 0><<<grid, MD_THREADS, 0, st>>>(bra, ket, a.mat_J, a.thr, tab, qc,
-                                                                                  cut, budget);
-            else
-                coulomb_md_kernel<LA, LB, LC, LD, 1><<<grid, MD_THREADS, 0, st>>>(bra, ket, a.mat_J, a.thr, tab, qc,
-                                                                                  cut, budget);
-        } else if (jvar == 3) {
-            using JS = JTmaShape<LC, LD>;
-            int rc2 = jtma_prepare_launch<LA, LB, LC, LD>();
-            if (rc2) return rc2;
-            if (pm == 0)
-                coulomb_tma_kernel<LA, LB, LC, LD, 0><<<grid, JT_TILE, JS::SMEM, st>>>(bra, ket, a.mat_J, a.thr, tab,
-                                                                                      qc, cut, budget, kerr);
-            else
-                coulomb_tma_kernel<LA, LB, LC, LD, 1><<<grid, JT_TILE, JS::SMEM, st>>>(bra, ket, a.mat_J, a.thr, tab,
-                                                                                      qc, cut, budget, kerr);
-        } else if (jvar == 1) {
-            if (pm == 0)
-                coulomb_col_kernel<LA, LB, LC, LD, 0><<<grid, J_THREADS, 0, st>>>(bra, ket, a.mat_J, a.thr, tab, qc,
-                                                                                  cut, budget);
-            else
-                coulomb_col_kernel<LA, LB, LC, LD, 1><<<grid, J_THREADS, 0, st>>>(bra, ket, a.mat_J, a.thr, tab, qc,
-                                                                                  cut, budget);
-        } else {
-            if (pm == 0)
-                coulomb_kernel<LA, LB, LC, LD, 0><<<grid, J_THREADS, 0, st>>>(bra, ket, a.mat_J, a.thr, tab, qc, cut,
-                                                                               budget);
-            else
-                coulomb_kernel<LA, LB, LC, LD, 1><<<grid, J_THREADS, 0, st>>>(bra, ket, a.mat_J, a.thr, tab, qc, cut,
-                                                                               budget);
-        }
+        if constexpr (G == 1)
+            rc = launch_coulomb_grad<LA, LB, LC, LD>(pm, grid, st, bra, ket, a.mat_J, gstride, a.thr, tab, cut);
+        else
+            rc = launch_coulomb<LA, LB, LC, LD>(jvar, pm, grid, st, bra, ket, a.mat_J, a.thr, tab, qc, cut, budget);
+        if (rc) return rc;
         note_launches();
     }
-    VLXB_CHECK_CUDA(cudaGetLastError());
     return VLXB_OK;
 }
 
@@ -207,46 +141,6 @@ int run_coulomb_grad(const CoulombArgs& a, int64_t gstride, cudaStream_t st)
     if (!tab.f64 || !tab.f32) return VLXB_ECUDA;
     Arena ar(st);
     return run_coulomb_impl<LA, LB, LC, LD, 1>(a, st, ar, tab, nullptr, fp32_cut_get(), gstride);
-}
-
-// One contracted-partner column exchange launch of plan kind ORI when that
-// plan is built for the class; false otherwise.
-template <int LA, int LB, int LC, int LD, int ORI>
-bool launch_exchange_colc(int pm, int grid, cudaStream_t st, const KOutBlocks& out, const KPartnerRecs& rab,
-                          const KPartnerRecs& rcd, const KGroups& kgab, const KGroups& kgcd, const KDensity& dm,
-                          const ExchangeArgs& a, const BoysTabs& tab, unsigned long long* qk, double cut, double budget)
-{
-    if constexpr (ColTab<LA, LB, LC, LD, ORI>::K_FITS) {
-        if (pm == 0)
-            exchange_colc_kernel<LA, LB, LC, LD, ORI, 0><<<grid, K_THREADS, 0, st>>>(
-                out, rab, rcd, kgab, kgcd, dm, a.maxD, a.omega, a.thr, a.mat_K, tab, qk, cut, budget);
-        else
-            exchange_colc_kernel<LA, LB, LC, LD, ORI, 1><<<grid, K_THREADS, 0, st>>>(
-                out, rab, rcd, kgab, kgcd, dm, a.maxD, a.omega, a.thr, a.mat_K, tab, qk, cut, budget);
-        return true;
-    } else {
-        return false;
-    }
-}
-
-// One column exchange launch of plan kind ORI when that plan is built for the
-// class (its ColTab fits); false otherwise.
-template <int LA, int LB, int LC, int LD, int ORI>
-bool launch_exchange_col(int pm, int grid, cudaStream_t st, const KOutBlocks& out, const KPartnerRecs& rab,
-                         const KPartnerRecs& rcd, const KDensity& dm, const ExchangeArgs& a, const BoysTabs& tab,
-                         unsigned long long* qk, double cut, double budget)
-{
-    if constexpr (ColTab<LA, LB, LC, LD, ORI>::K_FITS) {
-        if (pm == 0)
-            exchange_col_kernel<LA, LB, LC, LD, ORI, 0><<<grid, K_THREADS, 0, st>>>(
-                out, rab, rcd, dm, a.maxD, a.omega, a.thr, a.mat_K, tab, qk, cut, budget);
-        else
-            exchange_col_kernel<LA, LB, LC, LD, ORI, 1><<<grid, K_THREADS, 0, st>>>(
-                out, rab, rcd, dm, a.maxD, a.omega, a.thr, a.mat_K, tab, qk, cut, budget);
-        return true;
-    } else {
-        return false;
-    }
 }
 
 template <int LA, int LB, int LC, int LD>
@@ -293,18 +187,16 @@ int run_exchange(const ExchangeArgs& a, cudaStream_t st)
         rc = segment_records(ar, NC * ND, npc, npd, gcd, a.pdata_cd);
         if (rc) return rc;
     }
-    const int var = schedule_get(1, LA, LB, LC, LD);
     const double budget = cut > 0.0 ? fp32_budget_get() : 0.0;
-    KGroups kgab{}, kgcd{};
-    const uint32_t key_naos = a.key_naos ? a.key_naos : a.naos;
-    if (var == 3 || var == 4 || var >= 9) {
-        // contracted variants: group partner records by contracted partner shell
-        rc = contract_groups(ar, npa, gab, a.aoinds[LB], key_naos);
+    constexpr bool CONTRACTED = k_rys(LA, LB, LC, LD) && k_contracted(LA, LB, LC, LD);
+    [[maybe_unused]] KGroups kgab{}, kgcd{};
+    if (CONTRACTED && cut > 0.0) {
+        rc = contract_groups(ar, npa, gab, a.aoinds[LB], a.key_naos ? a.key_naos : a.naos);
         if (rc) return rc;
         if (same) {
             gcd = gab;
         } else {
-            rc = contract_groups(ar, npc, gcd, a.aoinds[LD], key_naos);
+            rc = contract_groups(ar, npc, gcd, a.aoinds[LD], a.key_naos ? a.key_naos : a.naos);
             if (rc) return rc;
         }
     }
@@ -319,9 +211,11 @@ int run_exchange(const ExchangeArgs& a, cudaStream_t st)
             if (rc) return rc;
         }
     }
-    if (var == 3 || var == 4 || var >= 9) {
-        kgab = KGroups{gab.gseg, gab.gq, gab.gbeg, gab.gcnt, gab.msp, gab.mq, gab.msu, gab.mmask, gab.gqa, gab.gqpre};
-        kgcd = KGroups{gcd.gseg, gcd.gq, gcd.gbeg, gcd.gcnt, gcd.msp, gcd.mq, gcd.msu, gcd.mmask, gcd.gqa, gcd.gqpre};
+    if (CONTRACTED && cut > 0.0) {
+        kgab = KGroups{gab.gseg, gab.gq, gab.gbeg, gab.gcnt, gab.msp, gab.mq, gab.msu, gab.mmask, gab.gqa, gab.gqpre,
+                       gab.rec_grp};
+        kgcd = KGroups{gcd.gseg, gcd.gq, gcd.gbeg, gcd.gcnt, gcd.msp, gcd.mq, gcd.msu, gcd.mmask, gcd.gqa, gcd.gqpre,
+                       gcd.rec_grp};
     }
     double* blk_maxD = nullptr;
     if (a.prim_mol_a && a.maxD_mol) {
@@ -339,39 +233,20 @@ int run_exchange(const ExchangeArgs& a, cudaStream_t st)
     unsigned long long* qk = qc ? qc + 1 : nullptr;
     const KDensity dm{a.aoinds[LB], a.count[LB], a.aoinds_col[LD] ? a.aoinds_col[LD] : a.aoinds[LD], a.count[LD],
                       a.D, a.D_stride ? a.D_stride : a.naos};
+    if (ar.failed()) return VLXB_ENOMEM;
     for (int pm = 0; pm < (cut > 0.0 ? 2 : 1); pm++) {
-        bool launched = false;
-        // column kernels: variants 1, 2 = plan kinds 0, 1; variants 5..8 = packed kinds 2..5;
-        // contracted-partner column kernels: variants 3, 4 = kinds 0, 1; 9..12 = kinds 2..5
-        switch (var) {
-            case 3: launched = launch_exchange_colc<LA, LB, LC, LD, 0>(pm, grid, st, out, rab, rcd, kgab, kgcd, dm, a, tab, qk, cut, budget); break;
-            case 4: launched = launch_exchange_colc<LA, LB, LC, LD, 1>(pm, grid, st, out, rab, rcd, kgab, kgcd, dm, a, tab, qk, cut, budget); break;
-            case 9: launched = launch_exchange_colc<LA, LB, LC, LD, 2>(pm, grid, st, out, rab, rcd, kgab, kgcd, dm, a, tab, qk, cut, budget); break;
-            case 10: launched = launch_exchange_colc<LA, LB, LC, LD, 3>(pm, grid, st, out, rab, rcd, kgab, kgcd, dm, a, tab, qk, cut, budget); break;
-            case 11: launched = launch_exchange_colc<LA, LB, LC, LD, 4>(pm, grid, st, out, rab, rcd, kgab, kgcd, dm, a, tab, qk, cut, budget); break;
-            case 12: launched = launch_exchange_colc<LA, LB, LC, LD, 5>(pm, grid, st, out, rab, rcd, kgab, kgcd, dm, a, tab, qk, cut, budget); break;
-            default: break;
-        }
-        switch (var) {
-            case 1: launched = launch_exchange_col<LA, LB, LC, LD, 0>(pm, grid, st, out, rab, rcd, dm, a, tab, qk, cut, budget); break;
-            case 2: launched = launch_exchange_col<LA, LB, LC, LD, 1>(pm, grid, st, out, rab, rcd, dm, a, tab, qk, cut, budget); break;
-            case 5: launched = launch_exchange_col<LA, LB, LC, LD, 2>(pm, grid, st, out, rab, rcd, dm, a, tab, qk, cut, budget); break;
-            case 6: launched = launch_exchange_col<LA, LB, LC, LD, 3>(pm, grid, st, out, rab, rcd, dm, a, tab, qk, cut, budget); break;
-            case 7: launched = launch_exchange_col<LA, LB, LC, LD, 4>(pm, grid, st, out, rab, rcd, dm, a, tab, qk, cut, budget); break;
-            case 8: launched = launch_exchange_col<LA, LB, LC, LD, 5>(pm, grid, st, out, rab, rcd, dm, a, tab, qk, cut, budget); break;
-            default: break;
-        }
-        if (!launched) {
-            if (pm == 0)
-                exchange_kernel<LA, LB, LC, LD, 0><<<grid, K_THREADS, 0, st>>>(out, rab, rcd, dm, a.maxD, a.omega,
-                                                                               a.thr, a.mat_K, tab, qk, cut, budget);
-            else
-                exchange_kernel<LA, LB, LC, LD, 1><<<grid, K_THREADS, 0, st>>>(out, rab, rcd, dm, a.maxD, a.omega,
-                                                                               a.thr, a.mat_K, tab, qk, cut, budget);
-        }
+        if constexpr (!k_rys(LA, LB, LC, LD))
+            rc = launch_exchange_thread<LA, LB, LC, LD>(pm, grid, st, out, rab, rcd, dm, a.maxD, a.omega, a.thr,
+                                                        a.mat_K, tab, qk, cut, budget);
+        else if (pm == 1)
+            rc = launch_exchange_mixed<LA, LB, LC, LD>(grid, st, out, rab, rcd, kgab, kgcd, dm, a.maxD, a.omega, a.thr,
+                                                       a.mat_K, tab, qk, cut, budget);
+        else
+            rc = launch_exchange_rys<LA, LB, LC, LD>(grid, st, out, rab, rcd, kgab, kgcd, dm, a.maxD, a.omega, a.thr,
+                                                     a.mat_K, qk, cut, budget);
+        if (rc) return rc;
         note_launches();
     }
-    VLXB_CHECK_CUDA(cudaGetLastError());
     return VLXB_OK;
 }
 
@@ -432,10 +307,10 @@ int run_exchange_grad(const ExchangeArgs& a, int64_t gstride, cudaStream_t st)
     const KGradBlockD bd{a.aoinds[LA], a.count[LA], a.aoinds[LC], a.count[LC], LA == LC ? 1 : 0};
     int grid = launch_grid_limit();
     if ((int64_t)grid > (int64_t)a.n_ik) grid = (int)a.n_ik;
-    exchange_grad_kernel<LA, LB, LC, LD><<<grid, KGradShape<LA, LB, LC, LD>::THREADS, 0, st>>>(
-        out, rab, rcd, dm, bd, a.maxD, a.omega, a.thr, a.mat_K, gstride, tab);
+    rc = launch_exchange_grad<LA, LB, LC, LD>(grid, st, out, rab, rcd, dm, bd, a.maxD, a.omega, a.thr, a.mat_K,
+                                              gstride, tab);
+    if (rc) return rc;
     note_launches();
-    VLXB_CHECK_CUDA(cudaGetLastError());
     return VLXB_OK;
 }
 

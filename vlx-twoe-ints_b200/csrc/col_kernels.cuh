@@ -26,6 +26,7 @@
 #pragma once
 #include "common.cuh"
 #include "jk_kernels.cuh"
+#include "launch.cuh"
 
 namespace vlxb {
 
@@ -335,19 +336,6 @@ exchange_col_kernel(KOutBlocks out, KPartnerRecs ab, KPartnerRecs cd, KDensity d
 // one S is a group of its own and is digested with its per-component S.
 template <int LA, int LB, int LC, int LD, int ORI, typename T>
 __device__ __forceinline__ void col_vrr_acc(const QVT<T>& q, const T* F, const ColLane& ln, T* out, T w);
-
-struct KGroups {
-    const int* seg;          // [n_first + 1] group offsets by first primitive shell
-    const double* q;         // max member q, descending inside a segment
-    const int32_t* beg;      // first member
-    const int32_t* cnt;      // member count
-    const int32_t* msp;      // member shell pair
-    const double* mq;        // member q
-    const double* msu;       // member uniform S, or NaN (member alone in its group)
-    const uint64_t* mmask;   // member component mask
-    const double* qa;        // sum over members of |q| times HRR growth (FP32 error budget), or null
-    const double* qpre;      // inclusive prefix sum of qa, or null
-};
 
 template <int LA, int LB, int LC, int LD, int ORI, typename T>
 __device__ __forceinline__ int kcolc_group(bool act, int jg, int lg, const KPartnerRecs& ab, const KPartnerRecs& cd,

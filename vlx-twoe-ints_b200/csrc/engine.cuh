@@ -151,6 +151,7 @@ struct PairGroups {
     double* mq = nullptr;      // [rec_stride] member q
     double* msu = nullptr;     // [rec_stride] member uniform S or NaN (then alone in its group)
     uint64_t* mmask = nullptr; // [rec_stride] member component mask
+    int32_t* rec_grp = nullptr; // [rec_stride] group of a record
     // FP32 error budget (budget_prefix_records; null when no budget is set):
     // per record / group the amplified bound, and its inclusive prefix sum
     double* rec_qa = nullptr;

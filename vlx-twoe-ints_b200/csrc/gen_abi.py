@@ -21,6 +21,7 @@ NULL = default stream), and returns a status code instead of void.
 """
 from __future__ import annotations
 
+import glob
 import os
 import sys
 
@@ -177,17 +178,10 @@ def header():
          "   shell quartet, 1 warp-cooperative column kernel, 2 McMurchie-Davidson",
          "   kernel (Hermite ket densities, one quartet per warp), 3 one thread per",
          "   quartet with the sorted ket stream staged into shared memory by TMA bulk",
-         "   copies, double-buffered; kind 1 = exchange: 0",
-         "   one thread per quartet, 1 column kernel with bra lanes, 2 column kernel",
-         "   with ket lanes, 3 / 4 the column kernels with bra / ket lanes that sum",
-         "   the primitive partners of one contracted shell before the HRR, 5 / 6",
-         "   packed column kernels with bra / ket lanes (lanes for the target",
-         "   levels only, from d up, so that a warp holds two or five quartets;",
-         "   the lower levels the VRR couples to are derived in each lane), 7 / 8",
-         "   the packed kernels with the lane-side pair built on its second",
-         "   centre (p+d and s+d pairs), 9..12 the contracted-partner kernels of",
-         "   the packed plans 5..8).  A column variant that is not built for",
-         "   the class, or whose kernel does not fit it, falls back to 0.",
+         "   copies, double-buffered; kind 1 = exchange: each class has one kernel,",
+         "   whatever the value (0..12): one thread per shell quartet below a total",
+         "   angular momentum of 5, Rys quadrature with one thread per root from there;",
+         "   FP32 quartets of the latter run on a thread or column kernel).",
          "   Every variant gives the same J/K to rounding; the",
          "   choice only changes speed.  Set by the autotuner.  No reference",
          "   counterpart. */",
@@ -569,26 +563,72 @@ def abi_cu():
     return "\n".join(L)
 
 
+J_LAUNCH = ("const JBraRecs&, const JKetPairs&, double*, double, const BoysTabs&, unsigned long long*, double, double")
+K_LAUNCH = ("const KOutBlocks&, const KPartnerRecs&, const KPartnerRecs&, const KDensity&, double, double, double, "
+            "double*")
+
+
+def k_rys(cls):
+    """Classes of the Rys exchange kernel (k_rys of launch.cuh)."""
+    return sum(LV[x] for x in cls) >= 5
+
+
+def driver_tu():
+    """The class drivers (host code only)."""
+    L = ["// Generated by gen_abi.py -- do not edit.", '#include "../classes.cuh"', "", "namespace vlxb {"]
+    for cls in j_classes():
+        t = ", ".join(str(LV[x]) for x in cls)
+        L.append(f"int coulomb_{cls}(const CoulombArgs& a, cudaStream_t s) {{ return run_coulomb<{t}>(a, s); }}")
+        L.append(f"int coulomb_grad_{cls}(const CoulombArgs& a, int64_t gs, cudaStream_t s) "
+                 f"{{ return run_coulomb_grad<{t}>(a, gs, s); }}")
+    for cls in k_classes():
+        t = ", ".join(str(LV[x]) for x in cls)
+        L.append(f"int exchange_{cls}(const ExchangeArgs& a, cudaStream_t s) {{ return run_exchange<{t}>(a, s); }}")
+        L.append(f"int exchange_grad_{cls}(const ExchangeArgs& a, int64_t gs, cudaStream_t s) "
+                 f"{{ return run_exchange_grad<{t}>(a, gs, s); }}")
+    L += ["}  // namespace vlxb", ""]
+    return "\n".join(L)
+
+
 def class_tu(cls, kind):
-    la, lb, lc, ld = (LV[x] for x in cls)
+    """The generated (straight-line) kernels of one class."""
+    t = ", ".join(str(LV[x]) for x in cls)
     L = ["// Generated by gen_abi.py -- do not edit.",
          '#include "../common.cuh"',
          f'#include "q_{cls}.cuh"',
          '#include "hrr_pairs.cuh"',
          '#include "../col_kernels.cuh"',
          f'#include "col_{cls}.cuh"',
-         '#include "../classes.cuh"', "",
+         '#include "../class_launch.cuh"', "",
          "namespace vlxb {"]
     if kind == "j":
-        L.append(f"int coulomb_{cls}(const CoulombArgs& a, cudaStream_t s) "
-                 f"{{ return run_coulomb<{la}, {lb}, {lc}, {ld}>(a, s); }}")
-        L.append(f"int coulomb_grad_{cls}(const CoulombArgs& a, int64_t gs, cudaStream_t s) "
-                 f"{{ return run_coulomb_grad<{la}, {lb}, {lc}, {ld}>(a, gs, s); }}")
+        L.append(f"template int launch_coulomb<{t}>(int, int, int, cudaStream_t, {J_LAUNCH});")
+        L.append(f"template int launch_coulomb_grad<{t}>(int, int, cudaStream_t, const JBraRecs&, const JKetPairs&, "
+                 "double*, int64_t, double, const BoysTabs&, double);")
     else:
-        L.append(f"int exchange_{cls}(const ExchangeArgs& a, cudaStream_t s) "
-                 f"{{ return run_exchange<{la}, {lb}, {lc}, {ld}>(a, s); }}")
-        L.append(f"int exchange_grad_{cls}(const ExchangeArgs& a, int64_t gs, cudaStream_t s) "
-                 f"{{ return run_exchange_grad<{la}, {lb}, {lc}, {ld}>(a, gs, s); }}")
+        if k_rys(cls):
+            L.append(f"template int launch_exchange_mixed<{t}>(int, cudaStream_t, const KOutBlocks&, "
+                     "const KPartnerRecs&, const KPartnerRecs&, const KGroups&, const KGroups&, const KDensity&, double, "
+                     "double, double, double*, const BoysTabs&, unsigned long long*, double, double);")
+        else:
+            L.append(f"template int launch_exchange_thread<{t}>(int, int, cudaStream_t, {K_LAUNCH}, const BoysTabs&, "
+                     "unsigned long long*, double, double);")
+        L.append(f"template int launch_exchange_grad<{t}>(int, cudaStream_t, const KOutBlocks&, const KPartnerRecs&, "
+                 "const KPartnerRecs&, const KDensity&, const KGradBlockD&, double, double, double, double*, int64_t, "
+                 "const BoysTabs&);")
+    L += ["}  // namespace vlxb", ""]
+    return "\n".join(L)
+
+
+def krys_tu(ab):
+    """Exchange Rys kernels of every class with bra pair `ab`."""
+    L = ["// Generated by gen_abi.py -- do not edit.", '#include "../krys_kernels.cuh"', "", "namespace vlxb {"]
+    for cls in k_classes():
+        if cls[:2] == ab and k_rys(cls):
+            t = ", ".join(str(LV[x]) for x in cls)
+            L.append(f"template int launch_exchange_rys<{t}>(int, cudaStream_t, const KOutBlocks&, const KPartnerRecs&, "
+                     "const KPartnerRecs&, const KGroups&, const KGroups&, const KDensity&, double, double, double, "
+                     "double*, unsigned long long*, double, double);")
     L += ["}  // namespace vlxb", ""]
     return "\n".join(L)
 
@@ -607,10 +647,16 @@ def main(pkg_root, repo_root):
     os.makedirs(gen, exist_ok=True)
     write_if_changed(os.path.join(repo_root, "include", "vlxb.h"), header())
     write_if_changed(os.path.join(gen, "abi.cu"), abi_cu())
+    write_if_changed(os.path.join(gen, "drivers.cu"), driver_tu())
     for cls in j_classes():
         write_if_changed(os.path.join(gen, f"cls_{cls}_j.cu"), class_tu(cls, "j"))
     for cls in k_classes():
         write_if_changed(os.path.join(gen, f"cls_{cls}_k.cu"), class_tu(cls, "k"))
+    for old in glob.glob(os.path.join(gen, "krys_*.cu")):
+        if os.path.basename(old)[5:-3] not in {cls[:2] for cls in k_classes() if k_rys(cls)}:
+            os.remove(old)
+    for ab in sorted({cls[:2] for cls in k_classes() if k_rys(cls)}):
+        write_if_changed(os.path.join(gen, f"krys_{ab}.cu"), krys_tu(ab))
 
 
 if __name__ == "__main__":

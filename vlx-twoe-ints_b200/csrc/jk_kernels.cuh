@@ -304,50 +304,56 @@ struct KChunk {
     int* c32;
 };
 
-// FP32 error budget (budget > 0, aqa / cqpre non-null): the l tail of j runs
-// in FP32 only as far as |q_j| A_j max_D * sum(|q_l| A_l) stays within
-// budget / njtot (njtot = the block's j count, A the HRR growth of a pair).
+// Passing and FP64 prefix lengths of the l list [c0, c1) for one j: nl, n64
+// (n64 = nl without a cutoff).  FP32 error budget (budget > 0, cqpre non-null;
+// qaj = the j bound times its HRR growth): the l tail of j runs in FP32 only as
+// far as |q_j| A_j max_D * sum(|q_l| A_l) stays within budget / njtot (njtot =
+// the block's j count, A the HRR growth of a pair).
+__device__ __forceinline__ void k_prefixes(double qij, double qaj, const double* __restrict__ cq,
+                                           const double* __restrict__ cqpre, int c0, int c1, double maxD, double thr,
+                                           double fp32_cut, int njtot, double budget, int& nl, int& n64)
+{
+    int lo = c0, hi = c1;
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (fabs(qij * __ldg(cq + mid) * maxD) > thr) lo = mid + 1;
+        else hi = mid;
+    }
+    nl = lo - c0;
+    n64 = nl;
+    if (fp32_cut > 0.0) {
+        int lo2 = c0, hi2 = lo;
+        while (lo2 < hi2) {
+            const int mid = (lo2 + hi2) >> 1;
+            if (fabs(qij * __ldg(cq + mid) * maxD) >= fp32_cut) lo2 = mid + 1;
+            else hi2 = mid;
+        }
+        n64 = lo2 - c0;
+        if (budget > 0.0 && cqpre && n64 < nl) {
+            const double qa = qaj * fabs(maxD);
+            const double bj = budget / (double)(njtot > 0 ? njtot : 1);
+            const double pend = __ldg(cqpre + c0 + nl - 1);
+            int lo4 = c0 + n64, hi4 = c0 + nl;
+            while (lo4 < hi4) {
+                const int mid = (lo4 + hi4) >> 1;
+                const double tail = pend - (mid > 0 ? __ldg(cqpre + mid - 1) : 0.0);
+                if (qa * tail <= bj) hi4 = mid;
+                else lo4 = mid + 1;
+            }
+            n64 = lo4 - c0;
+        }
+    }
+}
+
 __device__ __forceinline__ void k_chunk_scan(const double* __restrict__ aq, const double* __restrict__ cq, int jb,
                                              int nj, int c0, int c1, double maxD, double thr, double fp32_cut,
                                              KChunk s, const double* __restrict__ aqa = nullptr,
                                              const double* __restrict__ cqpre = nullptr, int njtot = 1,
                                              double budget = 0.0)
 {
-    for (int t = threadIdx.x; t < nj; t += blockDim.x) {
-        const double qij = __ldg(aq + jb + t);
-        int lo = c0, hi = c1;
-        while (lo < hi) {
-            const int mid = (lo + hi) >> 1;
-            if (fabs(qij * __ldg(cq + mid) * maxD) > thr) lo = mid + 1;
-            else hi = mid;
-        }
-        const int nl = lo - c0;
-        int n64 = nl;
-        if (fp32_cut > 0.0) {
-            int lo2 = c0, hi2 = lo;
-            while (lo2 < hi2) {
-                const int mid = (lo2 + hi2) >> 1;
-                if (fabs(qij * __ldg(cq + mid) * maxD) >= fp32_cut) lo2 = mid + 1;
-                else hi2 = mid;
-            }
-            n64 = lo2 - c0;
-            if (budget > 0.0 && aqa && cqpre && n64 < nl) {
-                const double qa = __ldg(aqa + jb + t) * fabs(maxD);
-                const double bj = budget / (double)(njtot > 0 ? njtot : 1);
-                const double pend = __ldg(cqpre + c0 + nl - 1);
-                int lo4 = c0 + n64, hi4 = c0 + nl;
-                while (lo4 < hi4) {
-                    const int mid = (lo4 + hi4) >> 1;
-                    const double tail = pend - (mid > 0 ? __ldg(cqpre + mid - 1) : 0.0);
-                    if (qa * tail <= bj) hi4 = mid;
-                    else lo4 = mid + 1;
-                }
-                n64 = lo4 - c0;
-            }
-        }
-        s.nl[t] = nl;
-        s.n64[t] = n64;
-    }
+    for (int t = threadIdx.x; t < nj; t += blockDim.x)
+        k_prefixes(__ldg(aq + jb + t), aqa ? __ldg(aqa + jb + t) : 0.0, cq, aqa ? cqpre : nullptr, c0, c1, maxD, thr,
+                   fp32_cut, njtot, budget, s.nl[t], s.n64[t]);
     __syncthreads();
     if (threadIdx.x == 0) {
         s.c64[0] = 0;

@@ -38,19 +38,10 @@
 // block's other positions receive nothing (all of them share the two atoms).
 #pragma once
 #include "jk_kernels.cuh"
+#include "launch.cuh"
 #include "md.cuh"
 
 namespace vlxb {
-
-// D_ik per (i, k) block: rows / columns of the (i, k) components in the AO
-// density (single-molecule calls).
-struct KGradBlockD {
-    const uint32_t* a_aoinds;
-    uint32_t a_count;
-    const uint32_t* c_aoinds;
-    uint32_t c_count;
-    int same_type;  // a == c: the diagonal entries i == k have weight 1
-};
 
 template <int LA, int LB, int LC, int LD>
 struct KGradShape {

@@ -23,11 +23,6 @@
 #include <mutex>
 #include <vector>
 
-#include "common.cuh"
-#include "generated/q_ssss.cuh"
-#include "generated/hrr_pairs.cuh"
-#include "col_kernels.cuh"
-#include "generated/col_ssss.cuh"
 #include "classes.cuh"
 #include "../../include/vlxb.h"
 

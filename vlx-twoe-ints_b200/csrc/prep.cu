@@ -460,6 +460,7 @@ int contract_groups(Arena& ar, int npa, PairGroups& g, const uint32_t* part_aoin
     double* gq0 = ar.alloc<double>(R);
     int* gperm_in = ar.alloc<int>(R);
     int* gperm = ar.alloc<int>(R);
+    g.rec_grp = ar.alloc<int32_t>(R);
     g.gseg = ar.alloc<int>(npa + 1);
     g.gq = ar.alloc<double>(R);
     g.gbeg = ar.alloc<int32_t>(R);
@@ -521,7 +522,8 @@ int contract_groups(Arena& ar, int npa, PairGroups& g, const uint32_t* part_aoin
     if (!ar.measuring()) {
         VLXB_CHECK_CUDA(cub::DeviceSegmentedRadixSort::SortPairsDescending(
             tmp, bytes, gq0, g.gq, gperm_in, gperm, (int)R, npa, g.gseg, g.gseg + 1, 0, 64, st));
-        k_grp_order<<<nb, PREP_THREADS, 0, st>>>(g.gseg + npa, g.n_rec, gperm, gbeg0, g.gbeg, g.gcnt);
+        k_grp_order<<<nb, PREP_THREADS, 0, st>>>(g.gseg + npa, g.n_rec, gperm, gbeg0, perm, g.gbeg, g.gcnt,
+                                                g.rec_grp);
         note_launches();
     }
     VLXB_CHECK_CUDA(cudaGetLastError());

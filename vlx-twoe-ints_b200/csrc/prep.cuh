@@ -402,14 +402,17 @@ __global__ void k_grp_seg(const int* __restrict__ seg, int nseg, const int* __re
 
 __global__ void k_grp_order(const int* __restrict__ n_grp, const int* __restrict__ n_rec,
                             const int* __restrict__ gperm, const int32_t* __restrict__ gbeg_in,
-                            int32_t* __restrict__ gbeg, int32_t* __restrict__ gcnt)
+                            const int* __restrict__ perm, int32_t* __restrict__ gbeg, int32_t* __restrict__ gcnt,
+                            int32_t* __restrict__ rec_grp)
 {
     const int n = *n_grp, nr = *n_rec;
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
         const int g = gperm[t];
         const int b = gbeg_in[g];
+        const int e = g + 1 < n ? gbeg_in[g + 1] : nr;
         gbeg[t] = b;
-        gcnt[t] = (g + 1 < n ? gbeg_in[g + 1] : nr) - b;
+        gcnt[t] = e - b;
+        for (int m = b; m < e; m++) rec_grp[perm[m]] = t;  // member m is record perm[m]
     }
 }
 

@@ -28,8 +28,10 @@ NVCC = os.environ.get("NVCC", "nvcc")
 ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ["-std=c++17", "-O3", "-lineinfo", "-Xcompiler", "-fPIC", "-Xptxas", "-v", "-I", CSRC] + ARCH_FLAGS
 
-COMMON_HEADERS = ["common.cuh", "engine.cuh", "jk_kernels.cuh", "prep.cuh", "classes.cuh", "col_kernels.cuh",
-                  "md.cuh", "md_kernels.cuh", "jgrad_kernels.cuh", "kgrad_kernels.cuh", "tma.cuh", "jtma_kernels.cuh"]
+HOST_HEADERS = ["common.cuh", "engine.cuh", "jk_kernels.cuh", "launch.cuh", "classes.cuh", "prep.cuh", "md.cuh"]
+CLASS_HEADERS = ["common.cuh", "engine.cuh", "jk_kernels.cuh", "launch.cuh", "class_launch.cuh", "col_kernels.cuh",
+                 "md.cuh", "md_kernels.cuh", "jgrad_kernels.cuh", "kgrad_kernels.cuh", "tma.cuh", "jtma_kernels.cuh"]
+RYS_HEADERS = ["common.cuh", "engine.cuh", "jk_kernels.cuh", "launch.cuh", "rys.cuh", "krys_kernels.cuh"]
 
 
 def _run_generators():
@@ -41,15 +43,18 @@ def _run_generators():
 def _sources():
     srcs = [os.path.join(CSRC, "prep.cu"), os.path.join(CSRC, "api.cu"), os.path.join(CSRC, "schwarz.cu"),
             os.path.join(CSRC, "noalloc.cu"), os.path.join(CSRC, "aomap.cu"),
-            os.path.join(CSRC, "listbuild.cu"), os.path.join(CSRC, "fshell.cu"), os.path.join(GEN, "abi.cu")]
-    srcs += sorted(glob.glob(os.path.join(GEN, "cls_*.cu")))
+            os.path.join(CSRC, "listbuild.cu"), os.path.join(CSRC, "fshell.cu"), os.path.join(CSRC, "rys.cu"),
+            os.path.join(GEN, "abi.cu"), os.path.join(GEN, "drivers.cu")]
+    srcs += sorted(glob.glob(os.path.join(GEN, "krys_*.cu"))) + sorted(glob.glob(os.path.join(GEN, "cls_*.cu")))
     return srcs
 
 
 def _deps(src):
-    deps = [src] + [os.path.join(CSRC, h) for h in COMMON_HEADERS] + [os.path.join(GEN, "hrr_pairs.cuh"),
-                                                                     os.path.join(REPO_ROOT, "include", "vlxb.h")]
     base = os.path.basename(src)
+    if base.startswith(("krys_", "rys")):
+        return [src] + [os.path.join(CSRC, h) for h in RYS_HEADERS]
+    deps = [src, os.path.join(GEN, "hrr_pairs.cuh"), os.path.join(REPO_ROOT, "include", "vlxb.h")]
+    deps += [os.path.join(CSRC, h) for h in (CLASS_HEADERS if base.startswith("cls_") else HOST_HEADERS)]
     if base.startswith("cls_"):
         deps.append(os.path.join(GEN, f"col_{base.split('_')[1]}.cuh"))
         with open(src) as fh:  # every generated quartet header the unit includes (its class first)

@@ -1,11 +1,9 @@
-"""Autotuner: pick the kernel variant of every J and K class by timing.
+"""Autotuner: pick the kernel variant of every J class by timing.
 
-For each class and each compiled variant (J: thread-per-quartet, column,
-McMurchie-Davidson, thread-per-quartet with TMA-staged kets;
-K: thread-per-quartet, column with bra or ket lanes, contracted column,
-packed column) the class
+For each class and each compiled variant (thread-per-quartet, column,
+McMurchie-Davidson, thread-per-quartet with TMA-staged kets) the class
 entry point is timed with CUDA events on a given system's lists (best of
-`reps`), and the fastest variant is kept.  The result is a JSON schedule
+`reps`), and the fastest variant is kept; every K class has one kernel.  The result is a JSON schedule
 ({"J": {class: variant}, "K": {...}}) that `apply_schedule` loads into the
 library's table (vlxb_setSchedule).  Every variant computes the same J/K to
 rounding, so the choice only changes speed.
@@ -35,6 +33,7 @@ SPILLING_THREAD_KERNELS = {
 
 
 def compiled_variants(kind: str, cls: str):
+    """Schedule numbers of a class (K: accepted by the library, one kernel each class)."""
     sys.path.insert(0, os.path.join(os.path.dirname(HERE), "csrc"))
     from gen_column import k_variants
 
@@ -78,7 +77,7 @@ def tune(dl, reps: int = 2, log=print):
             saved = L.get_schedule(kind, cls)
             best = None
             timings[kind][cls] = {}
-            variants = compiled_variants(kind, cls)
+            variants = compiled_variants(kind, cls) if kind == "J" else [saved]
             variants.sort(key=lambda v: v != saved)  # current choice first
             for v in variants:
                 L.set_schedule(kind, cls, v)

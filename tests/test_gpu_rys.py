@@ -59,3 +59,20 @@ def test_exchange_rys_vs_oracle(atoms, degree, side, uneven, omega):
     for k in oK:
         assert np.array_equal(runs[0][k], runs[1][k]), k
         assert close(runs[0][k], oK[k]), (k, float(np.abs(runs[0][k] - oK[k]).max()), float(np.abs(oK[k]).max()))
+
+
+@pytest.mark.parametrize("atoms,degree,side,uneven,omega", [
+    (2, 1, 2.0, True, 0.4),
+    (2, 2, 4.0, False, 0.0),
+    (3, 1, 4.0, True, 0.0),
+])
+def test_exchange_gradient_rys_vs_oracle(atoms, degree, side, uneven, omega):
+    from vlxb import gradient
+
+    wl, rl = system(atoms, degree, side, 3 + atoms, uneven)
+    dl = fock.to_device(rl)
+    eg = gradient.ExchangeGradient(dl, wl.mol)
+    g = eg.compute(omega=omega).cpu().numpy()
+    assert np.array_equal(g, eg.compute(omega=omega).cpu().numpy())
+    go, _ = helpers.oracle_exchange_gradient(rl, wl.mol.natoms, omega)
+    assert close(g, go), float(np.abs(g - go).max())

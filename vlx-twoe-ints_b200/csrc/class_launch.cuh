@@ -6,7 +6,6 @@
 #include "engine.cuh"
 #include "jgrad_kernels.cuh"
 #include "jtma_kernels.cuh"
-#include "kgrad_kernels.cuh"
 #include "launch.cuh"
 #include "md_kernels.cuh"
 
@@ -107,17 +106,6 @@ int launch_exchange_mixed(int grid, cudaStream_t st, const KOutBlocks& out, cons
     else
         exchange_kernel<LA, LB, LC, LD, 1><<<grid, K_THREADS, 0, st>>>(out, ab, cd, dm, maxD, omega, thr, mat_K, tab,
                                                                        qk, cut, budget);
-    VLXB_CHECK_CUDA(cudaGetLastError());
-    return VLXB_OK;
-}
-
-template <int LA, int LB, int LC, int LD>
-int launch_exchange_grad(int grid, cudaStream_t st, const KOutBlocks& out, const KPartnerRecs& ab,
-                         const KPartnerRecs& cd, const KDensity& dm, const KGradBlockD& bd, double maxD, double omega,
-                         double thr, double* grad, int64_t gstride, const BoysTabs& tab)
-{
-    exchange_grad_kernel<LA, LB, LC, LD><<<grid, KGradShape<LA, LB, LC, LD>::THREADS, 0, st>>>(
-        out, ab, cd, dm, bd, maxD, omega, thr, grad, gstride, tab);
     VLXB_CHECK_CUDA(cudaGetLastError());
     return VLXB_OK;
 }

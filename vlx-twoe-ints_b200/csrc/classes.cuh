@@ -267,8 +267,6 @@ int run_exchange_grad(const ExchangeArgs& a, int64_t gstride, cudaStream_t st)
     if (gstride < (int64_t)a.n_ik) return VLXB_EINVAL;
     int rc = ensure_pool_configured();
     if (rc) return rc;
-    const BoysTabs tab{boys_table_device(), boys_table32_device()};
-    if (!tab.f64) return VLXB_ECUDA;
     constexpr int NA = ncart(LA), NB = ncart(LB), NC = ncart(LC), ND = ncart(LD);
     Arena ar(st);
     KOutData ko;
@@ -308,7 +306,7 @@ int run_exchange_grad(const ExchangeArgs& a, int64_t gstride, cudaStream_t st)
     int grid = launch_grid_limit();
     if ((int64_t)grid > (int64_t)a.n_ik) grid = (int)a.n_ik;
     rc = launch_exchange_grad<LA, LB, LC, LD>(grid, st, out, rab, rcd, dm, bd, a.maxD, a.omega, a.thr, a.mat_K,
-                                              gstride, tab);
+                                              gstride);
     if (rc) return rc;
     note_launches();
     return VLXB_OK;

@@ -613,9 +613,19 @@ def class_tu(cls, kind):
         else:
             L.append(f"template int launch_exchange_thread<{t}>(int, int, cudaStream_t, {K_LAUNCH}, const BoysTabs&, "
                      "unsigned long long*, double, double);")
-        L.append(f"template int launch_exchange_grad<{t}>(int, cudaStream_t, const KOutBlocks&, const KPartnerRecs&, "
-                 "const KPartnerRecs&, const KDensity&, const KGradBlockD&, double, double, double, double*, int64_t, "
-                 "const BoysTabs&);")
+    L += ["}  // namespace vlxb", ""]
+    return "\n".join(L)
+
+
+def kgrad_tu(ab):
+    """Exchange gradient kernels of every class with bra pair `ab`."""
+    L = ["// Generated by gen_abi.py -- do not edit.", '#include "../kgrad_kernels.cuh"', "", "namespace vlxb {"]
+    for cls in k_classes():
+        if cls[:2] == ab:
+            t = ", ".join(str(LV[x]) for x in cls)
+            L.append(f"template int launch_exchange_grad<{t}>(int, cudaStream_t, const KOutBlocks&, "
+                     "const KPartnerRecs&, const KPartnerRecs&, const KDensity&, const KGradBlockD&, double, double, "
+                     "double, double*, int64_t);")
     L += ["}  // namespace vlxb", ""]
     return "\n".join(L)
 
@@ -652,6 +662,8 @@ def main(pkg_root, repo_root):
         write_if_changed(os.path.join(gen, f"cls_{cls}_j.cu"), class_tu(cls, "j"))
     for cls in k_classes():
         write_if_changed(os.path.join(gen, f"cls_{cls}_k.cu"), class_tu(cls, "k"))
+    for ab in sorted({cls[:2] for cls in k_classes()}):
+        write_if_changed(os.path.join(gen, f"kgrad_{ab}.cu"), kgrad_tu(ab))
     for old in glob.glob(os.path.join(gen, "krys_*.cu")):
         if os.path.basename(old)[5:-3] not in {cls[:2] for cls in k_classes() if k_rys(cls)}:
             os.remove(old)

@@ -1,4 +1,4 @@
-// Exchange nuclear gradient kernel (McMurchie-Davidson form).
+// Exchange nuclear gradient by Rys quadrature (sm_100a).
 //
 // E_K = 1/2 Tr[D K] = 1/2 sum_{ijkl} D_ik D_jl (ij|kl) over all primitive
 // Cartesian indices.  The sum is unchanged by (i <-> j, k <-> l) and by
@@ -12,135 +12,264 @@
 // (Obara-Saika 1986, Eq. 5; the reference generator's gradient='a' / 'c'
 // terms, eri.py:85-152).
 //
-// In Hermite form (md.cuh) (ab|cd) = sum_{e,f} E^{ab}_e Et^{cd}_f R_{e+f},
-// Et = (-1)^{|f|} E, and d/dA turns E^{ab} into
-// E'^{ab,x} = 2 alpha E^{a+1x,b} - a_x E^{a-1x,b} (d/dC the same on Et^{cd}).
-// With Gam_abcd = Dw_ac D_bd S_ab S_cd (Dw_ac = w_ik D_ik) one quartet gives
-//   A side, per b:  Y_{cf}  = sum_d D_bd S_cd Et^{cd}_f
-//                   T_{af}  = S_ab sum_c Dw_ac Y_{cf}
-//                   gA_x   += sum_{a,e} E'^{ab,x}_e sum_f R_{e+f} T_{af}
-//   C side, per d:  Y2_{ae} = sum_b D_bd S_ab E^{ab}_e
-//                   T2_{ce} = S_cd sum_a Dw_ac Y2_{ae}
-//                   gC_x   += sum_{c,f} Et'^{cd,x}_f sum_e R_{e+f} T2_{ce}
-// with R up to level L + 1.  The factorisation keeps every step a small
-// dense loop, so one generic kernel serves all 54 classes (runtime loops over
-// shared-memory tables; no straight-line derivative-class code, whose d-rich
-// instances do not compile in reasonable time).
+// One lane evaluates one root of one quartet (krys_kernels.cuh).  At a root
+// the energy is E = sum Gam_abcd Ix Iy Iz with Gam = Dw_ac D_bd S_ab S_cd
+// (Dw_ac = w_ik D_ik), so all six derivatives come from one reverse sweep:
+// with the sensitivities  Xb(c, d) = dE / dIx(ax, bx; c, d)  of one (a, b),
+//   gA_x += sum_cd Xb(c, d) (2 alpha I(ax + 1, bx; c, d) - ax I(ax - 1, ...))
+//   gC_x += sum_cd Xb(c, d) (2 gamma I(ax, bx; c + 1, d) - c I(ax, bx; c - 1, d)).
+// The sweep costs 24 multiply-adds per (a, b, c) for a d shell d (8 for the
+// energy alone), against 6 x 2 per component and root for separate sums.
+// Loops over b and a are not unrolled; the 27 sensitivities of one (a, b), the
+// 1-D integrals and the six sums are all that a lane keeps in registers.  The
+// VRR table in shared memory has one more row and column than the energy's.
+// Bound: FP64 issue and shared-memory loads together, with eight warps per SM
+// (255 registers).  5 atoms 4s3p2d: 717 -> 70 ms for the 54 classes against the
+// Hermite-table kernel it replaces (shared-memory bound at 91 %), DDDD class
+// call 4.0, PDDD 4.2 ms with the list preparation.
 //
 // Layout follows the exchange kernels: one CTA per (i, k) primitive shell
-// block, its partner-pair quartets spread over groups of SG lanes (SG = 1 ..
-// 32 by class size: one quartet per lane for the smallest classes, one per
-// warp for the largest), the group's lanes over the items of each step, six
-// accumulators per lane, fixed-order reduction, no atomics on the output.
-// Screening is the K kernels' (|Q_ij Q_kl max_D| > thr), FP64.
-// Output: the block's six values are added at the block's lowest (i, k) list
-// position p, grad[x * gstride + p] (x = 0..2: i's centre, 3..5: k's); the
-// block's other positions receive nothing (all of them share the two atoms).
+// block, fixed-order reduction, no atomics on the output.  Screening is the K
+// kernels' (|Q_ij Q_kl max_D| > thr), FP64.  The block's six values are added
+// at the block's lowest (i, k) list position p, grad[x * gstride + p] (x = 0..2:
+// i's centre, 3..5: k's); the block's other positions receive nothing (all of
+// them share the two atoms).
 #pragma once
-#include "jk_kernels.cuh"
-#include "launch.cuh"
-#include "md.cuh"
+#include "krys_kernels.cuh"
 
 namespace vlxb {
 
 template <int LA, int LB, int LC, int LD>
 struct KGradShape {
     static constexpr int L = LA + LB + LC + LD;
-    static constexpr int NA = ncart(LA), NB = ncart(LB), NC = ncart(LC), ND = ncart(LD);
-    static constexpr int NHB = nherm(LA + LB), NHBP = nherm(LA + LB + 1);
-    static constexpr int NHK = nherm(LC + LD), NHKP = nherm(LC + LD + 1);
-    static constexpr int NHL = nherm(L + 1);
-    static constexpr int EB = (LA + 2) * (LB + 1) * (LA + LB + 2);  // herm_e1<LA + 1, LB> per direction
-    static constexpr int EK = (LC + 2) * (LD + 1) * (LC + LD + 2);  // herm_e1<LC + 1, LD>
-    static constexpr int NY = (NC * NHK > NA * NHB) ? NC * NHK : NA * NHB;
-    static constexpr int NT = (NA * NHK > NC * NHB) ? NA * NHK : NC * NHB;
-    // lanes per quartet: a power of two near a quarter of the widest step
-    // (the Y / T items and the Hermite indices of the R contractions), so that
-    // small classes run many quartets per warp (down to one per lane) and
-    // large ones a warp each
-    static constexpr int cmax(int x, int y) { return x > y ? x : y; }
-    static constexpr int WIDE = cmax(cmax(cmax(NC * NHK, NA * NHK), cmax(NA * NHB, NC * NHB)), cmax(NHBP, NHKP));
-    static constexpr int SG = WIDE <= 4 ? 1 : WIDE <= 8 ? 2 : WIDE <= 16 ? 4 : WIDE <= 32 ? 8 : WIDE <= 64 ? 16 : 32;
-    static constexpr int NG = 32 / SG;  // quartet groups per warp
-    // doubles per group: R (two level buffers), R^{(n)}_{000}, E tables, D_bd, S_ab, S_cd, Y, T
-    static constexpr int PER_GROUP = 2 * NHL + (L + 2) + 3 * EB + 3 * EK + NB * ND + NA * NB + NC * ND + NY + NT;
-    static constexpr int FIXED_BYTES = NHKP * NHBP * 2 + NHL * 8 + NA * NC * 8 + 4 * (K_JCHUNK + 1) * 4 + 512;
-    static constexpr int NW = (4 * NG * PER_GROUP * 8 + FIXED_BYTES <= 46 * 1024)   ? 4
-                              : (2 * NG * PER_GROUP * 8 + FIXED_BYTES <= 46 * 1024) ? 2
-                                                                                    : 1;
-    static constexpr int THREADS = NW * 32;
+    static constexpr int NR = (L + 1) / 2 + 1;
+    static constexpr int QW = 32 / NR;
+    static constexpr int BATCH = L >= 3 ? QW : 32 / QW * QW;  // quartets set up together
+    static constexpr int N1 = LA + LB + 2, M1 = LC + LD + 2;
+    // two CTAs of four warps (255 registers); the tables of two d-d pairs leave
+    // room for seven warps, taken as one CTA
+    static constexpr int NW = N1 * M1 >= 36 ? 7 : 4;
+    static constexpr int THREADS = NW * 32, MINB = NW == 7 ? 1 : (L >= 5 ? 2 : 3);
+    static constexpr int SMEM = 3 * N1 * M1 * THREADS * 8;
 };
 
+// v[m], m < NM: the shift of V(a, .) to b exponent bx (krys_row).
+template <int LB, int M1, int NM, int TH>
+__device__ __forceinline__ void kgrad_shift(const double* V, int a, int bx, double R, double* v)
+{
+    const double* p = V + a * M1 * TH;
+    if (LB == 0 || bx == 0) {
+#pragma unroll
+        for (int m = 0; m < NM; m++) v[m] = p[m * TH];
+    } else if (LB == 1 || bx == 1) {
+#pragma unroll
+        for (int m = 0; m < NM; m++) v[m] = fma(R, p[m * TH], p[(M1 + m) * TH]);
+    } else {
+        const double R2 = R * R, RR = R + R;
+#pragma unroll
+        for (int m = 0; m < NM; m++)
+            v[m] = fma(R2, p[m * TH],
+                       fma(RR, p[(M1 + m) * TH], p[(2 * M1 + m) * TH]));
+    }
+}
+
+// The two centres' derivative sums of one direction for sensitivities S(c, d)
+// of the extended integrals H(c, d), c <= LC + 1.
+template <int LB, int LC, int LD, int M1, int TH>
+__device__ __forceinline__ void kgrad_direction(const double* V, int ax, int bx, double R, double Rk, double al2,
+                                                double ga2, const double* S, const double* H, double& gA, double& gC)
+{
+    constexpr int D1 = LD + 1, NM = LC + LD + 1;
+    double p[NM], h[(LC + 1) * D1];
+    kgrad_shift<LB, M1, NM, TH>(V, ax + 1, bx, R, p);
+#pragma unroll
+    for (int m = 0; m < NM; m++) p[m] *= al2;
+    if (ax > 0) {
+        double q[NM];
+        kgrad_shift<LB, M1, NM, TH>(V, ax - 1, bx, R, q);
+#pragma unroll
+        for (int m = 0; m < NM; m++) p[m] = fma(-(double)ax, q[m], p[m]);
+    }
+    shift_ket<LC, LD>(p, Rk, h);
+    double s1 = 0.0, s2 = 0.0;
+#pragma unroll
+    for (int c = 0; c <= LC; c++)
+#pragma unroll
+        for (int d = 0; d <= LD; d++) {
+            gA = fma(S[c * D1 + d], h[c * D1 + d], gA);
+            s1 = fma(S[c * D1 + d], H[(c + 1) * D1 + d], s1);
+            if (c > 0) s2 = fma(-(double)c * S[c * D1 + d], H[(c - 1) * D1 + d], s2);
+        }
+    gC += fma(ga2, s1, s2);
+}
+
+// The six sums of one root with per-component S and component masks.
 template <int LA, int LB, int LC, int LD>
-__global__ void __launch_bounds__(KGradShape<LA, LB, LC, LD>::THREADS)
-exchange_grad_kernel(KOutBlocks out, KPartnerRecs ab, KPartnerRecs cd, KDensity dm, KGradBlockD bd, double maxD,
-                     double omega, double thr, double* __restrict__ grad, int64_t gstride, BoysTabs tabs)
+__device__ __noinline__ void kgrad_masked(const KPartnerRecs& ab, const KPartnerRecs& cd, int jr, int lr,
+                                          const KDensity& dm, const double* Dw, const double* V, double al2,
+                                          double ga2, double* g)
+{
+    constexpr int N1 = LA + LB + 2, M1 = LC + LD + 2, TH = KGradShape<LA, LB, LC, LD>::THREADS;
+    const int spj = __ldg(ab.rec_sp + jr), spl = __ldg(cd.rec_sp + lr);
+    const uint64_t mj = __ldg(ab.rec_mask + jr), ml = __ldg(cd.rec_mask + lr);
+    const double suj = __ldg(ab.su + jr), sul = __ldg(cd.su + lr);
+    const int jsh = __ldg(ab.partner + spj), lsh = __ldg(cd.partner + spl);
+    double R[3], Rk[3];
+    for (int x = 0; x < 3; x++) {
+        R[x] = __ldg(ab.geo + (G_RX + x) * ab.sp_stride + spj);
+        Rk[x] = __ldg(cd.geo + (G_RX + x) * cd.sp_stride + spl);
+    }
+    for (int ij = 0; ij < ncart(LA) * ncart(LB); ij++) {
+        if (!((mj >> ij) & 1ull)) continue;
+        const double Sij = isnan(suj) ? __ldg(ab.S + ij * ab.sp_stride + spj) : suj;
+        const int ca = ij / ncart(LB), cb = ij % ncart(LB);
+        int a[3], b[3], c[3], d[3];
+        cart_exps(LA, ca, a[0], a[1], a[2]);
+        cart_exps(LB, cb, b[0], b[1], b[2]);
+        const uint32_t jao = __ldg(dm.b_aoinds + jsh + (int64_t)dm.b_count * cb);
+        for (int kl = 0; kl < ncart(LC) * ncart(LD); kl++) {
+            if (!((ml >> kl) & 1ull)) continue;
+            const double Skl = isnan(sul) ? __ldg(cd.S + kl * cd.sp_stride + spl) : sul;
+            const int cc = kl / ncart(LD), cdd = kl % ncart(LD);
+            cart_exps(LC, cc, c[0], c[1], c[2]);
+            cart_exps(LD, cdd, d[0], d[1], d[2]);
+            const uint32_t lao = __ldg(dm.d_aoinds + lsh + (int64_t)dm.d_count * cdd);
+            const double w = Dw[ca * ncart(LC) + cc] * Sij * Skl * __ldg(dm.D + (int64_t)jao * dm.naos + lao);
+            double I[3], dA[3], dC[3];
+            for (int x = 0; x < 3; x++) {
+                const double* Vx = V + x * N1 * M1 * TH;
+                I[x] = krys_value<M1, TH>(Vx, a[x], b[x], c[x], d[x], R[x], Rk[x]);
+                dA[x] = al2 * krys_value<M1, TH>(Vx, a[x] + 1, b[x], c[x], d[x], R[x], Rk[x]);
+                if (a[x] > 0) dA[x] -= a[x] * krys_value<M1, TH>(Vx, a[x] - 1, b[x], c[x], d[x], R[x], Rk[x]);
+                dC[x] = ga2 * krys_value<M1, TH>(Vx, a[x], b[x], c[x] + 1, d[x], R[x], Rk[x]);
+                if (c[x] > 0) dC[x] -= c[x] * krys_value<M1, TH>(Vx, a[x], b[x], c[x] - 1, d[x], R[x], Rk[x]);
+            }
+            for (int x = 0; x < 3; x++) {
+                const double o = w * I[(x + 1) % 3] * I[(x + 2) % 3];
+                g[x] = fma(o, dA[x], g[x]);
+                g[3 + x] = fma(o, dC[x], g[3 + x]);
+            }
+        }
+    }
+}
+
+template <int LA, int LB, int LC, int LD>
+__device__ __forceinline__ void kgrad_lane(const KPartnerRecs& ab, const KPartnerRecs& cd, const KWarpSetup<KGradShape<LA, LB, LC, LD>::BATCH>& st,
+                                           int q, int root, const KDensity& dm, const double* Dw,
+                                           const double* __restrict__ rtab, double* V, double* g)
 {
     using S = KGradShape<LA, LB, LC, LD>;
-    constexpr int L1 = S::L + 1;
-    constexpr int NA = S::NA, NB = S::NB, NC = S::NC, ND = S::ND;
-    constexpr int NHB = S::NHB, NHBP = S::NHBP, NHK = S::NHK, NHKP = S::NHKP, NHL = S::NHL;
-    constexpr int NW = S::NW, NT_ = S::THREADS, SG = S::SG, NG = S::NG;
-    constexpr int LSB = LA + LB + 2, LSK = LC + LD + 2;  // t extents of the E tables
+    constexpr int N1 = S::N1, M1 = S::M1, TH = S::THREADS, NS = S::BATCH, VX = N1 * M1 * TH;
+    constexpr int NA = ncart(LA), NB = ncart(LB), NC = ncart(LC), ND = ncart(LD);
+    constexpr int D1 = LD + 1, CD = (LC + 1) * D1, CE = (LC + 2) * D1;
+    const double* sc = st.sc + q;
+    KVTable<N1 * M1, false, TH> Vx{V}, Vy{V + VX}, Vz{V + 2 * VX};
+    krys_tables<S::NR, N1, M1, NS>(sc, root, rtab, Vx, Vy, Vz);
+    const double al2 = 2.0 * sc[KF_AL * NS], ga2 = 2.0 * sc[KF_GA * NS];
+    if (st.jr[q] < 0) {
+        double h[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+        kgrad_masked<LA, LB, LC, LD>(ab, cd, ~st.jr[q], st.lr[q], dm, Dw, V, al2, ga2, h);
+#pragma unroll
+        for (int x = 0; x < 6; x++) g[x] += h[x];
+        return;
+    }
+    const int jsh = st.jsh[q], lsh = st.lsh[q];
+    double R[3], Rk[3];
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        R[k] = sc[(KF_AB + k) * NS];
+        Rk[k] = sc[(KF_CD + k) * NS];
+    }
+    uint32_t lao[ND];
+#pragma unroll
+    for (int k = 0; k < ND; k++) lao[k] = __ldg(dm.d_aoinds + lsh + (int64_t)dm.d_count * k);
+#pragma unroll 1
+    for (int t = 0; t < NB; t++) {
+        int bx, by, bz;
+        krys_b<LB>(t, bx, by, bz);
+        const uint32_t jao = __ldg(dm.b_aoinds + jsh + (int64_t)dm.b_count * cart_index(by, bz));
+        const double* Drow = dm.D + (int64_t)jao * dm.naos;
+        double Dv[ND];
+#pragma unroll
+        for (int k = 0; k < ND; k++) Dv[k] = __ldg(Drow + lao[k]);
+#pragma unroll 1
+        for (int a = 0; a < NA; a++) {
+            int ax, ay, az;
+            cart_exps(LA, a, ax, ay, az);
+            double X[CE], Y[CE], Z[CE], v[M1];
+            kgrad_shift<LB, M1, M1, TH>(V, ax, bx, R[0], v);
+            shift_ket<LC + 1, LD>(v, Rk[0], X);
+            kgrad_shift<LB, M1, M1, TH>(V + VX, ay, by, R[1], v);
+            shift_ket<LC + 1, LD>(v, Rk[1], Y);
+            kgrad_shift<LB, M1, M1, TH>(V + 2 * VX, az, bz, R[2], v);
+            shift_ket<LC + 1, LD>(v, Rk[2], Z);
+            double Xb[CD], Yb[CD], Zb[CD];
+#pragma unroll
+            for (int k = 0; k < CD; k++) Xb[k] = Yb[k] = Zb[k] = 0.0;
+#pragma unroll
+            for (int z = 0; z <= LC; z++) {
+                double T1[ND], Tb[ND];
+#pragma unroll
+                for (int dy = 0; dy <= LD; dy++)
+#pragma unroll
+                    for (int dz = 0; dz <= LD - dy; dz++) {
+                        const int k = cart_index(dy, dz);
+                        T1[k] = Dv[k] * Z[z * D1 + dz];
+                        Tb[k] = 0.0;
+                    }
+#pragma unroll
+                for (int y = 0; y <= LC - z; y++) {
+                    const int x = LC - z - y;
+                    const double wc = Dw[a * NC + cart_index(y, z)];
+#pragma unroll
+                    for (int dx = 0; dx <= LD; dx++) {
+                        const double xw = wc * X[x * D1 + dx];
+                        double s = 0.0;
+#pragma unroll
+                        for (int dy = 0; dy <= LD - dx; dy++) {
+                            const int k = cart_index(dy, LD - dx - dy);
+                            s = fma(T1[k], Y[y * D1 + dy], s);
+                            Yb[y * D1 + dy] = fma(xw, T1[k], Yb[y * D1 + dy]);
+                            Tb[k] = fma(xw, Y[y * D1 + dy], Tb[k]);
+                        }
+                        Xb[x * D1 + dx] = fma(wc, s, Xb[x * D1 + dx]);
+                    }
+                }
+#pragma unroll
+                for (int dy = 0; dy <= LD; dy++)
+#pragma unroll
+                    for (int dz = 0; dz <= LD - dy; dz++) {
+                        const int k = cart_index(dy, dz);
+                        Zb[z * D1 + dz] = fma(Tb[k], Dv[k], Zb[z * D1 + dz]);
+                    }
+            }
+            kgrad_direction<LB, LC, LD, M1, TH>(V, ax, bx, R[0], Rk[0], al2, ga2, Xb, X, g[0], g[3]);
+            kgrad_direction<LB, LC, LD, M1, TH>(V + VX, ay, by, R[1], Rk[1], al2, ga2, Yb, Y, g[1], g[4]);
+            kgrad_direction<LB, LC, LD, M1, TH>(V + 2 * VX, az, bz, R[2], Rk[2], al2, ga2, Zb, Z, g[2], g[5]);
+        }
+    }
+}
+
+template <int LA, int LB, int LC, int LD>
+__global__ void __launch_bounds__((KGradShape<LA, LB, LC, LD>::THREADS), (KGradShape<LA, LB, LC, LD>::MINB))
+exchange_grad_kernel(KOutBlocks out, KPartnerRecs ab, KPartnerRecs cd, KDensity dm, KGradBlockD bd, double maxD,
+                     double omega, double thr, double* __restrict__ grad, int64_t gstride,
+                     const double* __restrict__ rtab)
+{
+    using S = KGradShape<LA, LB, LC, LD>;
+    constexpr int NA = ncart(LA), NC = ncart(LC), NW = S::NW;
+    extern __shared__ double krys_smem[];
     __shared__ int s_nl[K_JCHUNK], s_n64[K_JCHUNK], s_c64[K_JCHUNK + 1], s_c32[K_JCHUNK + 1];
-    __shared__ int16_t sIdx[NHKP][NHBP];  // index of R_{e+f}, -1 above level L + 1
-    __shared__ uint32_t sTuv[NHL];
-    __shared__ uint32_t sRec[NHL];  // R recurrence per entry (as coulomb_md_kernel)
-    __shared__ uint32_t sCart[4][10];  // exponents of component c of shell l: x | y << 4 | z << 8
     __shared__ double sDw[NA * NC];
     __shared__ double red[NW][6];
     __shared__ int s_pmin;
-    __shared__ double sw[NW * NG][S::PER_GROUP];
+    __shared__ KWarpSetup<S::BATCH> s_set[NW];
+    double* V = krys_smem + threadIdx.x;
     const KChunk ch{s_nl, s_n64, s_c64, s_c32};
-
-    for (int i = threadIdx.x; i < 40; i += NT_) {
-        const int l = i / 10, c = i % 10;
-        sCart[l][c] = c < ncart(l) ? (uint32_t)cart_x(l, c) | ((uint32_t)cart_y(l, c) << 4) |
-                                         ((uint32_t)cart_z(l, c) << 8)
-                                   : 0u;
-    }
-    for (int i = threadIdx.x; i < NHL; i += NT_) {
-        int n = 0;
-        while (nherm(n) <= i) n++;
-        const int r = i - (n > 0 ? nherm(n - 1) : 0);
-        int s = 0;
-        while ((s + 1) * (s + 2) / 2 <= r) s++;
-        const int v = r - s * (s + 1) / 2, u = s - v, t = n - s;
-        sTuv[i] = (uint32_t)t | ((uint32_t)u << 8) | ((uint32_t)v << 16);
-        uint32_t rec = 1023u << 10;
-        if (t > 0)
-            rec = herm_idx(t - 1, u, v) | ((t > 1 ? herm_idx(t - 2, u, v) : 1023u) << 10) | ((uint32_t)(t - 1) << 20);
-        else if (u > 0)
-            rec = herm_idx(0, u - 1, v) | ((u > 1 ? herm_idx(0, u - 2, v) : 1023u) << 10) |
-                  ((uint32_t)(u - 1) << 20) | (1u << 28);
-        else if (v > 0)
-            rec = herm_idx(0, 0, v - 1) | ((v > 1 ? herm_idx(0, 0, v - 2) : 1023u) << 10) |
-                  ((uint32_t)(v - 1) << 20) | (2u << 28);
-        sRec[i] = rec;
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < NHKP * NHBP; i += NT_) {
-        const int f = i / NHBP, e = i % NHBP;
-        const uint32_t a = sTuv[e], b = sTuv[f];
-        const int t = (a & 255) + (b & 255), u = ((a >> 8) & 255) + ((b >> 8) & 255), v = (a >> 16) + (b >> 16);
-        sIdx[f][e] = (int16_t)(t + u + v <= L1 ? herm_idx(t, u, v) : -1);
-    }
-    __syncthreads();
-
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int grp = lane / SG, sub = lane % SG;  // quartet group in the warp, lane in the group
-    double* W = sw[warp * NG + grp];
-    double* R0 = W;
-    double* R1 = R0 + NHL;
-    double* Rb = R1 + NHL;        // [L1 + 1] R^{(n)}_{000}
-    double* Eb = Rb + (L1 + 1);   // [3][EB]
-    double* Ek = Eb + 3 * S::EB;  // [3][EK]
-    double* Dbd = Ek + 3 * S::EK;
-    double* Sab = Dbd + NB * ND;
-    double* Scd = Sab + NA * NB;
-    double* Y = Scd + NC * ND;
-    double* T = Y + S::NY;
     const int nout = *out.n;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int root = lane % S::NR, slot = lane / S::NR;
+    KWarpSetup<S::BATCH>& set = s_set[warp];
 
     for (int o = blockIdx.x; o < nout; o += gridDim.x) {
         const int ish = __ldg(out.ish + o), ksh = __ldg(out.ksh + o);
@@ -166,246 +295,20 @@ exchange_grad_kernel(KOutBlocks out, KPartnerRecs ab, KPartnerRecs cd, KDensity 
         for (int jb = a0; jb < a1; jb += K_JCHUNK) {
             const int nj = min(K_JCHUNK, a1 - jb);
             k_chunk_scan(ab, cd, jb, nj, c0, c1, maxD, thr, 0.0, ch);
-            const int nq = s_c64[nj];
-            // every group of a warp walks the same number of slots, so the
-            // warp-wide __syncwarp() calls below stay uniform; a group without a
-            // quartet in its slot skips the work
-            for (int base = warp * NG; base < nq; base += NW * NG) {
-                const int w = base + grp;
-                const bool valid = w < nq;
-                const int jj = valid ? k_find(s_c64, nj, w) : 0;
-                const int jr = jb + jj, lr = valid ? c0 + (w - s_c64[jj]) : c0;
-                const int spj = valid ? __ldg(ab.rec_sp + jr) : 0, spl = valid ? __ldg(cd.rec_sp + lr) : 0;
-                PairGeo bg{}, kg{};
-                double al2 = 0.0, ga2 = 0.0;
-                if (valid) {
-                    bg = load_geo(ab.geo, ab.sp_stride, spj);
-                    kg = load_geo(cd.geo, cd.sp_stride, spl);
-                    al2 = 2.0 * __ldg(ab.geo + G_ALPHA * ab.sp_stride + spj);
-                    ga2 = 2.0 * __ldg(cd.geo + G_ALPHA * cd.sp_stride + spl);
-                    // per-quartet factors: D_bd, S_ab, S_cd, 1-D Hermite tables
-                    const int jsh = __ldg(ab.partner + spj), lsh = __ldg(cd.partner + spl);
-                    for (int t = sub; t < NB * ND; t += SG) {
-                        const int cb = t / ND, cdd = t % ND;
-                        const uint32_t jao = __ldg(dm.b_aoinds + jsh + (int64_t)dm.b_count * cb);
-                        const uint32_t lao = __ldg(dm.d_aoinds + lsh + (int64_t)dm.d_count * cdd);
-                        Dbd[t] = __ldg(dm.D + (int64_t)jao * dm.naos + lao);
-                    }
-                    const double suj = __ldg(ab.su + jr), sul = __ldg(cd.su + lr);
-                    const uint64_t mj = __ldg(ab.rec_mask + jr), ml = __ldg(cd.rec_mask + lr);
-                    for (int t = sub; t < NA * NB; t += SG)
-                        Sab[t] = !isnan(suj) ? suj : (((mj >> t) & 1ull) ? __ldg(ab.S + t * ab.sp_stride + spj) : 0.0);
-                    for (int t = sub; t < NC * ND; t += SG)
-                        Scd[t] = !isnan(sul) ? sul : (((ml >> t) & 1ull) ? __ldg(cd.S + t * cd.sp_stride + spl) : 0.0);
-                    for (int x = sub; x < 6; x += SG) {
-                        if (x < 3) {
-                            const double pa = x == 0 ? bg.Ax : (x == 1 ? bg.Ay : bg.Az);
-                            const double abv = x == 0 ? bg.Rx : (x == 1 ? bg.Ry : bg.Rz);
-                            herm_e1_flat<LA + 1, LB>(pa, pa + abv, bg.i2z, Eb + x * S::EB);
-                        } else {
-                            const double qc = x == 3 ? kg.Ax : (x == 4 ? kg.Ay : kg.Az);
-                            const double cdv = x == 3 ? kg.Rx : (x == 4 ? kg.Ry : kg.Rz);
-                            herm_e1_flat<LC + 1, LD>(qc, qc + cdv, kg.i2z, Ek + (x - 3) * S::EK);
-                        }
-                    }
-                }
-                // R^{(n)}_{000} = 2 sqrt(rho'/pi) (-2 rho')^n F_n(rho' |PQ|^2), rho' = rho d2
-                // (d2 = 1, or w^2 / (rho + w^2) for the attenuated operator), then levels
-                const double PQx = bg.Px - kg.Px, PQy = bg.Py - kg.Py, PQz = bg.Pz - kg.Pz;
-                if (valid && sub == 0) {
-                    const double inv = 1.0 / (bg.z + kg.z);
-                    const double rho = bg.z * kg.z * inv;
-                    const double d2 = omega != 0.0 ? omega * omega / (rho + omega * omega) : 1.0;
-                    const double rp = rho * d2;
-                    double F[L1 + 1];
-                    boys_f64<L1>(rp * fma(PQx, PQx, fma(PQy, PQy, PQz * PQz)), tabs.f64, F);
-                    double s = 2.0 * sqrt(rp * INV_PI_D);
-#pragma unroll
-                    for (int n = 0; n <= L1; n++) {
-                        Rb[n] = F[n] * s;
-                        s *= -2.0 * rp;
-                    }
-                    R0[0] = Rb[L1];
+            const int total = s_c64[nj];
+            const int batch = krys_batch(total, NW, S::QW, S::BATCH);
+            int jj = 0;
+            for (int w0 = warp * batch; w0 < total; w0 += NW * batch) {
+                const int n = min(batch, total - w0), w = w0 + lane;
+                if (lane < n) {
+                    while (s_c64[jj + 1] <= w) jj++;
+                    krys_setup<true>(ab, cd, jb + jj, c0 + w - s_c64[jj], omega, set, lane);
                 }
                 __syncwarp();
-#pragma unroll 1
-                for (int n = L1 - 1; n >= 0; n--) {
-                    double* src = ((L1 - 1 - n) & 1) ? R1 : R0;
-                    double* dst = ((L1 - 1 - n) & 1) ? R0 : R1;
-                    const int cnt = nherm(L1 - n);
-                    if (valid) {
-                        for (int i = sub; i < cnt; i += SG) {
-                            const uint32_t rec = sRec[i];
-                            const uint32_t dir = rec >> 28, s2 = (rec >> 10) & 1023u;
-                            const double pq = dir == 0 ? PQx : (dir == 1 ? PQy : PQz);
-                            double val = pq * src[rec & 1023u];
-                            if (s2 != 1023u) val = fma((double)((rec >> 20) & 255u), src[s2], val);
-                            dst[i] = i == 0 ? Rb[n] : val;
-                        }
-                    }
-                    __syncwarp();
-                }
-                const double* R = (L1 & 1) ? R1 : R0;
-
-                // ---- A side: derivatives on i's centre
-#pragma unroll 1
-                for (int b = 0; b < NB; b++) {
-                    const uint32_t bp_ = sCart[LB][b];
-                    const int bx = bp_ & 15u, by = (bp_ >> 4) & 15u, bz = bp_ >> 8;
-                    if (valid) {
-                        for (int it = sub; it < NC * NHK; it += SG) {
-                            const int c = it / NHK, f = it % NHK;
-                            const uint32_t tf = sTuv[f];
-                            const int t = tf & 255, u = (tf >> 8) & 255, v = tf >> 16;
-                            const uint32_t cp_ = sCart[LC][c];
-                            const int cx = cp_ & 15u, cy = (cp_ >> 4) & 15u, cz = cp_ >> 8;
-                            double y = 0.0;
-                            for (int d = 0; d < ND; d++) {
-                                const uint32_t dp_ = sCart[LD][d];
-                                const int dx = dp_ & 15u, dy = (dp_ >> 4) & 15u, dz = dp_ >> 8;
-                                const double e = Ek[0 * S::EK + (cx * (LD + 1) + dx) * LSK + t] *
-                                                 Ek[1 * S::EK + (cy * (LD + 1) + dy) * LSK + u] *
-                                                 Ek[2 * S::EK + (cz * (LD + 1) + dz) * LSK + v];
-                                y = fma(Dbd[b * ND + d] * Scd[c * ND + d], e, y);
-                            }
-                            Y[it] = ((t + u + v) & 1) ? -y : y;
-                        }
-                    }
-                    __syncwarp();
-                    if (valid) {
-                        for (int it = sub; it < NA * NHK; it += SG) {
-                            const int a = it / NHK, f = it % NHK;
-                            double s = 0.0;
-                            for (int c = 0; c < NC; c++) s = fma(sDw[a * NC + c], Y[c * NHK + f], s);
-                            T[it] = Sab[a * NB + b] * s;
-                        }
-                    }
-                    __syncwarp();
-                    if (valid) {
-                        // lanes over bra Hermite indices e; each R_{e+f} serves all a
-                        for (int e = sub; e < NHBP; e += SG) {
-                            const uint32_t te = sTuv[e];
-                            const int t = te & 255, u = (te >> 8) & 255, v = te >> 16;
-                            double dE[NA][3];
-                            bool any = false;
-#pragma unroll
-                            for (int a = 0; a < NA; a++) {
-                                const uint32_t ap_ = sCart[LA][a];
-                                const int ax = ap_ & 15u, ay = (ap_ >> 4) & 15u, az = ap_ >> 8;
-                                // 1-D factors E^{i,j}_t at i = a_x, a_x + 1, a_x - 1 (0 when i < 0)
-                                const double x0 = Eb[0 * S::EB + (ax * (LB + 1) + bx) * LSB + t];
-                                const double y0 = Eb[1 * S::EB + (ay * (LB + 1) + by) * LSB + u];
-                                const double z0 = Eb[2 * S::EB + (az * (LB + 1) + bz) * LSB + v];
-                                const double xp = Eb[0 * S::EB + ((ax + 1) * (LB + 1) + bx) * LSB + t];
-                                const double yp = Eb[1 * S::EB + ((ay + 1) * (LB + 1) + by) * LSB + u];
-                                const double zp = Eb[2 * S::EB + ((az + 1) * (LB + 1) + bz) * LSB + v];
-                                const double xm = ax > 0 ? Eb[0 * S::EB + ((ax - 1) * (LB + 1) + bx) * LSB + t] : 0.0;
-                                const double ym = ay > 0 ? Eb[1 * S::EB + ((ay - 1) * (LB + 1) + by) * LSB + u] : 0.0;
-                                const double zm = az > 0 ? Eb[2 * S::EB + ((az - 1) * (LB + 1) + bz) * LSB + v] : 0.0;
-                                dE[a][0] = (al2 * xp - ax * xm) * y0 * z0;
-                                dE[a][1] = x0 * (al2 * yp - ay * ym) * z0;
-                                dE[a][2] = x0 * y0 * (al2 * zp - az * zm);
-                                any = any || dE[a][0] != 0.0 || dE[a][1] != 0.0 || dE[a][2] != 0.0;
-                            }
-                            if (!any) continue;
-                            double acc[NA];
-#pragma unroll
-                            for (int a = 0; a < NA; a++) acc[a] = 0.0;
-                            for (int f = 0; f < NHK; f++) {
-                                const double r = R[sIdx[f][e]];
-#pragma unroll
-                                for (int a = 0; a < NA; a++) acc[a] = fma(r, T[a * NHK + f], acc[a]);
-                            }
-#pragma unroll
-                            for (int a = 0; a < NA; a++) {
-                                g[0] = fma(dE[a][0], acc[a], g[0]);
-                                g[1] = fma(dE[a][1], acc[a], g[1]);
-                                g[2] = fma(dE[a][2], acc[a], g[2]);
-                            }
-                        }
-                    }
-                    __syncwarp();
-                }
-
-                // ---- C side: derivatives on k's centre
-#pragma unroll 1
-                for (int d = 0; d < ND; d++) {
-                    const uint32_t dp_ = sCart[LD][d];
-                    const int dx = dp_ & 15u, dy = (dp_ >> 4) & 15u, dz = dp_ >> 8;
-                    if (valid) {
-                        for (int it = sub; it < NA * NHB; it += SG) {
-                            const int a = it / NHB, e = it % NHB;
-                            const uint32_t te = sTuv[e];
-                            const int t = te & 255, u = (te >> 8) & 255, v = te >> 16;
-                            const uint32_t ap_ = sCart[LA][a];
-                            const int ax = ap_ & 15u, ay = (ap_ >> 4) & 15u, az = ap_ >> 8;
-                            double y = 0.0;
-                            for (int b = 0; b < NB; b++) {
-                                const uint32_t bp_ = sCart[LB][b];
-                                const int bx = bp_ & 15u, by = (bp_ >> 4) & 15u, bz = bp_ >> 8;
-                                const double e1 = Eb[0 * S::EB + (ax * (LB + 1) + bx) * LSB + t] *
-                                                  Eb[1 * S::EB + (ay * (LB + 1) + by) * LSB + u] *
-                                                  Eb[2 * S::EB + (az * (LB + 1) + bz) * LSB + v];
-                                y = fma(Dbd[b * ND + d] * Sab[a * NB + b], e1, y);
-                            }
-                            Y[it] = y;
-                        }
-                    }
-                    __syncwarp();
-                    if (valid) {
-                        for (int it = sub; it < NC * NHB; it += SG) {
-                            const int c = it / NHB, e = it % NHB;
-                            double s = 0.0;
-                            for (int a = 0; a < NA; a++) s = fma(sDw[a * NC + c], Y[a * NHB + e], s);
-                            T[it] = Scd[c * ND + d] * s;
-                        }
-                    }
-                    __syncwarp();
-                    if (valid) {
-                        // lanes over ket Hermite indices f; each R_{e+f} serves all c
-                        for (int f = sub; f < NHKP; f += SG) {
-                            const uint32_t tf = sTuv[f];
-                            const int t = tf & 255, u = (tf >> 8) & 255, v = tf >> 16;
-                            const double sg = ((t + u + v) & 1) ? -1.0 : 1.0;
-                            double dE[NC][3];
-                            bool any = false;
-#pragma unroll
-                            for (int c = 0; c < NC; c++) {
-                                const uint32_t cp_ = sCart[LC][c];
-                                const int cx = cp_ & 15u, cy = (cp_ >> 4) & 15u, cz = cp_ >> 8;
-                                const double x0 = Ek[0 * S::EK + (cx * (LD + 1) + dx) * LSK + t];
-                                const double y0 = Ek[1 * S::EK + (cy * (LD + 1) + dy) * LSK + u];
-                                const double z0 = Ek[2 * S::EK + (cz * (LD + 1) + dz) * LSK + v];
-                                const double xp = Ek[0 * S::EK + ((cx + 1) * (LD + 1) + dx) * LSK + t];
-                                const double yp = Ek[1 * S::EK + ((cy + 1) * (LD + 1) + dy) * LSK + u];
-                                const double zp = Ek[2 * S::EK + ((cz + 1) * (LD + 1) + dz) * LSK + v];
-                                const double xm = cx > 0 ? Ek[0 * S::EK + ((cx - 1) * (LD + 1) + dx) * LSK + t] : 0.0;
-                                const double ym = cy > 0 ? Ek[1 * S::EK + ((cy - 1) * (LD + 1) + dy) * LSK + u] : 0.0;
-                                const double zm = cz > 0 ? Ek[2 * S::EK + ((cz - 1) * (LD + 1) + dz) * LSK + v] : 0.0;
-                                dE[c][0] = sg * (ga2 * xp - cx * xm) * y0 * z0;
-                                dE[c][1] = sg * x0 * (ga2 * yp - cy * ym) * z0;
-                                dE[c][2] = sg * x0 * y0 * (ga2 * zp - cz * zm);
-                                any = any || dE[c][0] != 0.0 || dE[c][1] != 0.0 || dE[c][2] != 0.0;
-                            }
-                            if (!any) continue;
-                            double acc[NC];
-#pragma unroll
-                            for (int c = 0; c < NC; c++) acc[c] = 0.0;
-                            for (int e = 0; e < NHB; e++) {
-                                const double r = R[sIdx[f][e]];
-#pragma unroll
-                                for (int c = 0; c < NC; c++) acc[c] = fma(r, T[c * NHB + e], acc[c]);
-                            }
-#pragma unroll
-                            for (int c = 0; c < NC; c++) {
-                                g[3] = fma(dE[c][0], acc[c], g[3]);
-                                g[4] = fma(dE[c][1], acc[c], g[4]);
-                                g[5] = fma(dE[c][2], acc[c], g[5]);
-                            }
-                        }
-                    }
-                    __syncwarp();
-                }
+                if (slot < S::QW)
+                    for (int q = slot; q < n; q += S::QW)
+                        kgrad_lane<LA, LB, LC, LD>(ab, cd, set, q, root, dm, sDw, rtab, V, g);
+                __syncwarp();
             }
             __syncthreads();
         }
@@ -423,6 +326,23 @@ exchange_grad_kernel(KOutBlocks out, KPartnerRecs ab, KPartnerRecs cd, KDensity 
         }
         __syncthreads();
     }
+}
+
+template <int LA, int LB, int LC, int LD>
+int launch_exchange_grad(int grid, cudaStream_t st, const KOutBlocks& out, const KPartnerRecs& ab,
+                         const KPartnerRecs& cd, const KDensity& dm, const KGradBlockD& bd, double maxD, double omega,
+                         double thr, double* grad, int64_t gstride)
+{
+    using S = KGradShape<LA, LB, LC, LD>;
+    static std::atomic<unsigned long long> done;
+    const double* tab = rys_table_device();
+    if (!tab) return VLXB_ECUDA;
+    const int rc = rys_prepare((const void*)exchange_grad_kernel<LA, LB, LC, LD>, S::SMEM, S::MINB, done);
+    if (rc) return rc;
+    exchange_grad_kernel<LA, LB, LC, LD><<<grid, S::THREADS, S::SMEM, st>>>(
+        out, ab, cd, dm, bd, maxD, omega, thr, grad, gstride, tab + rys_offset(S::NR));
+    VLXB_CHECK_CUDA(cudaGetLastError());
+    return VLXB_OK;
 }
 
 }  // namespace vlxb

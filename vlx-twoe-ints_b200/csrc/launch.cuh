@@ -95,6 +95,6 @@ struct KGradBlockD {
 template <int LA, int LB, int LC, int LD>
 int launch_exchange_grad(int grid, cudaStream_t st, const KOutBlocks& out, const KPartnerRecs& ab,
                          const KPartnerRecs& cd, const KDensity& dm, const KGradBlockD& bd, double maxD, double omega,
-                         double thr, double* grad, int64_t gstride, const BoysTabs& tab);
+                         double thr, double* grad, int64_t gstride);
 
 }  // namespace vlxb

@@ -20,11 +20,11 @@ def close(got, exp):
     return not exp.size or float(np.abs(got - exp).max()) <= RTOL * float(np.abs(exp).max()) + 1e-14
 
 
-def system(atoms, degree, side, seed, uneven):
+def system(atoms, degree, side, seed, uneven, threshold=1e-12):
     """Two shells per type; `uneven`: S and Q differ between the components of
     a pair (so a pair splits into records with partial component masks)."""
     lib().init(0)
-    wl = basis.config_custom(atoms, max(side, 3.0), {0: 1, 1: 1, 2: 1}, degree, 0.4, 3.0, max(1, atoms), 1e-12, seed)
+    wl = basis.config_custom(atoms, max(side, 3.0), {0: 1, 1: 1, 2: 1}, degree, 0.4, 3.0, max(1, atoms), threshold, seed)
     if atoms == 2:  # a fixed separation: `side` bohr along one diagonal
         wl.mol.coords[1] = wl.mol.coords[0] + side / np.sqrt(3.0)
     rl = lists.build_lists(wl.mol, wl.D, wl.threshold, fock.gpu_schwarz_fn())
@@ -37,6 +37,14 @@ def system(atoms, degree, side, seed, uneven):
             kp.Q = kp.Q * np.where(c % 3 == 1, 0.5, 1.0)
             order = np.lexsort((-kp.Q, first))
             kp.Dinds, kp.Q, kp.pdata = kp.Dinds[order], kp.Q[order].copy(), kp.pdata[order].copy()
+        for key, jl in rl.jlists.items():
+            na, nb = lists.NCART[lists.LV[key[0]]], lists.NCART[lists.LV[key[1]]]
+            c = (jl.first.astype(np.int64) % na) * nb + jl.second.astype(np.int64) % nb
+            jl.pdata = jl.pdata * (1.0 + 0.05 * c)
+            jl.Q = jl.Q * np.where(c % 3 == 1, 0.5, 1.0)
+            order = np.argsort(-np.abs(jl.Q * jl.D), kind="stable")
+            for n in ("first", "second", "pdata", "Q", "D"):
+                setattr(jl, n, np.ascontiguousarray(getattr(jl, n)[order]))
     return wl, rl
 
 
@@ -75,4 +83,30 @@ def test_exchange_gradient_rys_vs_oracle(atoms, degree, side, uneven, omega):
     g = eg.compute(omega=omega).cpu().numpy()
     assert np.array_equal(g, eg.compute(omega=omega).cpu().numpy())
     go, _ = helpers.oracle_exchange_gradient(rl, wl.mol.natoms, omega)
+    assert close(g, go), float(np.abs(g - go).max())
+
+
+@pytest.mark.parametrize("atoms,degree,side,uneven,threshold", [
+    (1, 1, 2.0, False, 1e-12),   # one ket per bra
+    (2, 2, 1.2, True, 1e-12),
+    (2, 2, 30.0, False, 1e-12),  # T beyond every root table
+    (2, 3, 3.0, False, 1e-4),    # kets with some components screened out
+    (3, 2, 4.0, True, 1e-5),
+])
+def test_coulomb_rys_vs_oracle(atoms, degree, side, uneven, threshold):
+    from vlxb import gradient
+
+    wl, rl = system(atoms, degree, side, 3 + atoms, uneven, threshold)
+    dl = fock.to_device(rl)
+    runs = []
+    for _ in range(2):
+        matJ, _ = fock.build_jk(dl, do_k=False)
+        torch.cuda.synchronize()
+        runs.append({k: v.cpu().numpy() for k, v in matJ.items()})
+    oJ, _ = helpers.oracle_jk_all(rl)
+    for k in oJ:
+        assert np.array_equal(runs[0][k], runs[1][k]), k
+        assert close(runs[0][k], oJ[k]), (k, float(np.abs(runs[0][k] - oJ[k]).max()), float(np.abs(oJ[k]).max()))
+    g = gradient.CoulombGradient(dl, wl.mol).compute().cpu().numpy()
+    go, _ = helpers.oracle_coulomb_gradient(rl, wl.mol.natoms)
     assert close(g, go), float(np.abs(g - go).max())

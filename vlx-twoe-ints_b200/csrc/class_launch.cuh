@@ -4,7 +4,6 @@
 
 #include "col_kernels.cuh"
 #include "engine.cuh"
-#include "jgrad_kernels.cuh"
 #include "jtma_kernels.cuh"
 #include "launch.cuh"
 #include "md_kernels.cuh"
@@ -12,9 +11,9 @@
 namespace vlxb {
 
 // The staged Coulomb kernel's shared memory exceeds the 48 KB default for
-// kets with d functions: raise the limit once per device for each of its
-// two instantiations.
-template <int LA, int LB, int LC, int LD>
+// kets with d functions: raise the limit once per device for each
+// instantiation.
+template <int LA, int LB, int LC, int LD, int PM>
 int jtma_prepare_launch()
 {
     static std::atomic<unsigned long long> done{0};
@@ -22,11 +21,8 @@ int jtma_prepare_launch()
     VLXB_CHECK_CUDA(cudaGetDevice(&dev));
     const unsigned long long bit = 1ull << (dev & 63);
     if (done.load(std::memory_order_acquire) & bit) return VLXB_OK;
-    const int smem = (int)JTmaShape<LC, LD>::SMEM;
-    VLXB_CHECK_CUDA(cudaFuncSetAttribute(coulomb_tma_kernel<LA, LB, LC, LD, 0>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    VLXB_CHECK_CUDA(cudaFuncSetAttribute(coulomb_tma_kernel<LA, LB, LC, LD, 1>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    VLXB_CHECK_CUDA(cudaFuncSetAttribute(coulomb_tma_kernel<LA, LB, LC, LD, PM>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)JTmaShape<LC, LD>::SMEM));
     done.fetch_or(bit, std::memory_order_acq_rel);
     return VLXB_OK;
 }
@@ -41,7 +37,7 @@ int launch_coulomb_pass(int variant, int grid, cudaStream_t st, const JBraRecs& 
     } else if (variant == 3) {
         unsigned long long* kerr = kernel_errors_device();
         if (!kerr) return VLXB_ECUDA;
-        const int rc = jtma_prepare_launch<LA, LB, LC, LD>();
+        const int rc = jtma_prepare_launch<LA, LB, LC, LD, PM>();
         if (rc) return rc;
         coulomb_tma_kernel<LA, LB, LC, LD, PM><<<grid, JT_TILE, JTmaShape<LC, LD>::SMEM, st>>>(
             bra, ket, mat_J, thr, tab, qc, cut, budget, kerr);
@@ -58,21 +54,12 @@ template <int LA, int LB, int LC, int LD>
 int launch_coulomb(int variant, int pm, int grid, cudaStream_t st, const JBraRecs& bra, const JKetPairs& ket,
                    double* mat_J, double thr, const BoysTabs& tab, unsigned long long* qc, double cut, double budget)
 {
-    return pm == 0 ? launch_coulomb_pass<LA, LB, LC, LD, 0>(variant, grid, st, bra, ket, mat_J, thr, tab, qc, cut, budget)
-                   : launch_coulomb_pass<LA, LB, LC, LD, 1>(variant, grid, st, bra, ket, mat_J, thr, tab, qc, cut, budget);
-}
-
-template <int LA, int LB, int LC, int LD>
-int launch_coulomb_grad(int pm, int grid, cudaStream_t st, const JBraRecs& bra, const JKetPairs& ket, double* out,
-                        int64_t gstride, double thr, const BoysTabs& tab, double cut)
-{
-    constexpr int GT = JGradShape<LA, LB, LC, LD>::THREADS;
-    if (pm == 0)
-        coulomb_grad_kernel<LA, LB, LC, LD, 0><<<grid, GT, 0, st>>>(bra, ket, out, gstride, thr, tab, cut);
+    if (pm == 1)
+        return launch_coulomb_pass<LA, LB, LC, LD, 1>(variant, grid, st, bra, ket, mat_J, thr, tab, qc, cut, budget);
+    if constexpr (j_rys(LA, LB, LC, LD))
+        return VLXB_EINVAL;  // launch_coulomb_rys
     else
-        coulomb_grad_kernel<LA, LB, LC, LD, 1><<<grid, GT, 0, st>>>(bra, ket, out, gstride, thr, tab, cut);
-    VLXB_CHECK_CUDA(cudaGetLastError());
-    return VLXB_OK;
+        return launch_coulomb_pass<LA, LB, LC, LD, 0>(variant, grid, st, bra, ket, mat_J, thr, tab, qc, cut, budget);
 }
 
 template <int LA, int LB, int LC, int LD>

@@ -85,9 +85,11 @@ int run_coulomb_impl(const CoulombArgs& a, cudaStream_t st, Arena& ar, const Boy
     if (rc) return rc;
     const bool batched = a.prim_mol_a && a.prim_mol_c && a.n_mol > 0;
     JKetData kd;
-    const int jvar = G ? 2 : schedule_get(0, LA, LB, LC, LD);
+    const int jvar = schedule_get(0, LA, LB, LC, LD);
+    // the Rys and McMurchie-Davidson kernels read the Hermite ket density
+    const bool hermite = G || j_rys(LA, LB, LC, LD) || jvar == 2;
     rc = jket_prepare<LC, LD>(ar, gk, a.cd_first, a.cd_second, a.cd_D, a.cd_Q, a.cd_pdata, kd,
-                              batched ? a.prim_mol_c : nullptr, batched ? a.n_mol : 0, jvar == 2);
+                              batched ? a.prim_mol_c : nullptr, batched ? a.n_mol : 0, hermite);
     if (rc) return rc;
     const double budget = (cut > 0.0 && !G) ? fp32_budget_get() : 0.0;
     if (budget > 0.0) {
@@ -108,9 +110,13 @@ int run_coulomb_impl(const CoulombArgs& a, cudaStream_t st, Arena& ar, const Boy
     if ((int64_t)grid > (int64_t)a.n_ab) grid = (int)a.n_ab;
     for (int pm = 0; pm < (cut > 0.0 ? 2 : 1); pm++) {
         if constexpr (G == 1)
-            rc = launch_coulomb_grad<LA, LB, LC, LD>(pm, grid, st, bra, ket, a.mat_J, gstride, a.thr, tab, cut);
-        else
+            rc = launch_coulomb_grad<LA, LB, LC, LD>(pm, grid, st, bra, ket, a.mat_J, gstride, a.thr, cut);
+        else if (j_rys(LA, LB, LC, LD) && pm == 0) {
+            if constexpr (j_rys(LA, LB, LC, LD))
+                rc = launch_coulomb_rys<LA, LB, LC, LD>(grid, st, bra, ket, a.mat_J, a.thr, qc, cut, budget);
+        } else {
             rc = launch_coulomb<LA, LB, LC, LD>(jvar, pm, grid, st, bra, ket, a.mat_J, a.thr, tab, qc, cut, budget);
+        }
         if (rc) return rc;
         note_launches();
     }

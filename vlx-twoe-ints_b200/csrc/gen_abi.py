@@ -178,7 +178,9 @@ def header():
          "   shell quartet, 1 warp-cooperative column kernel, 2 McMurchie-Davidson",
          "   kernel (Hermite ket densities, one quartet per warp), 3 one thread per",
          "   quartet with the sorted ket stream staged into shared memory by TMA bulk",
-         "   copies, double-buffered; kind 1 = exchange: each class has one kernel,",
+         "   copies, double-buffered; the classes with two or more units of angular",
+         "   momentum on each side and five in all run their FP64 quartets on a Rys",
+         "   quadrature kernel whatever the value; kind 1 = exchange: each class has one kernel,",
          "   whatever the value (0..12): one thread per shell quartet below a total",
          "   angular momentum of 5, Rys quadrature with one thread per root from there;",
          "   FP32 quartets of the latter run on a thread or column kernel).",
@@ -568,6 +570,12 @@ K_LAUNCH = ("const KOutBlocks&, const KPartnerRecs&, const KPartnerRecs&, const 
             "double*")
 
 
+def j_rys(cls):
+    """Classes of the Rys Coulomb kernel (j_rys of launch.cuh)."""
+    la, lb, lc, ld = (LV[x] for x in cls)
+    return la + lb >= 2 and lc + ld >= 2 and la + lb + lc + ld >= 5
+
+
 def k_rys(cls):
     """Classes of the Rys exchange kernel (k_rys of launch.cuh)."""
     return sum(LV[x] for x in cls) >= 5
@@ -603,8 +611,6 @@ def class_tu(cls, kind):
          "namespace vlxb {"]
     if kind == "j":
         L.append(f"template int launch_coulomb<{t}>(int, int, int, cudaStream_t, {J_LAUNCH});")
-        L.append(f"template int launch_coulomb_grad<{t}>(int, int, cudaStream_t, const JBraRecs&, const JKetPairs&, "
-                 "double*, int64_t, double, const BoysTabs&, double);")
     else:
         if k_rys(cls):
             L.append(f"template int launch_exchange_mixed<{t}>(int, cudaStream_t, const KOutBlocks&, "
@@ -613,6 +619,21 @@ def class_tu(cls, kind):
         else:
             L.append(f"template int launch_exchange_thread<{t}>(int, int, cudaStream_t, {K_LAUNCH}, const BoysTabs&, "
                      "unsigned long long*, double, double);")
+    L += ["}  // namespace vlxb", ""]
+    return "\n".join(L)
+
+
+def jrys_tu(ab):
+    """Rys Coulomb kernels and Coulomb gradient kernels of every class with bra pair `ab`."""
+    L = ["// Generated by gen_abi.py -- do not edit.", '#include "../jrys_kernels.cuh"', "", "namespace vlxb {"]
+    lists = "const JBraRecs&, const JKetPairs&, double*"
+    for cls in j_classes():
+        if cls[:2] == ab:
+            t = ", ".join(str(LV[x]) for x in cls)
+            if j_rys(cls):
+                L.append(f"template int launch_coulomb_rys<{t}>(int, cudaStream_t, {lists}, double, "
+                         "unsigned long long*, double, double);")
+            L.append(f"template int launch_coulomb_grad<{t}>(int, int, cudaStream_t, {lists}, int64_t, double, double);")
     L += ["}  // namespace vlxb", ""]
     return "\n".join(L)
 
@@ -662,6 +683,8 @@ def main(pkg_root, repo_root):
         write_if_changed(os.path.join(gen, f"cls_{cls}_j.cu"), class_tu(cls, "j"))
     for cls in k_classes():
         write_if_changed(os.path.join(gen, f"cls_{cls}_k.cu"), class_tu(cls, "k"))
+    for ab in sorted({cls[:2] for cls in j_classes()}):
+        write_if_changed(os.path.join(gen, f"jrys_{ab}.cu"), jrys_tu(ab))
     for ab in sorted({cls[:2] for cls in k_classes()}):
         write_if_changed(os.path.join(gen, f"kgrad_{ab}.cu"), kgrad_tu(ab))
     for old in glob.glob(os.path.join(gen, "krys_*.cu")):

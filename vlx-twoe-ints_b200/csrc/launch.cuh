@@ -16,6 +16,17 @@ namespace vlxb {
 // (L = 5); (DS|DD) 7.2 / 2.6 (L = 6).
 __host__ __device__ constexpr bool k_rys(int la, int lb, int lc, int ld) { return la + lb + lc + ld >= 5; }
 
+// FP64 kernel of a Coulomb class: Rys where the thread-per-quartet kernel's
+// registers limit it and both Hermite ranges are wide enough to repay the
+// set-up per root.  10 atoms 4s3p2d, thread / Rys, ms per class call: (SD|SD)
+// 2.0 / 2.1, (PP|PP) 0.72 / 0.78 (L = 4); (SP|DD) 1.7 / 2.5, (DD|SP) 1.18 / 1.27,
+// (PD|PP) 1.7 / 1.3, (SD|PD) 3.2 / 2.5 (L = 5); (PP|DD) 1.9 / 1.5, (PD|PD) 5.5 /
+// 2.8, (DD|PD) 6.0 / 1.7.
+__host__ __device__ constexpr bool j_rys(int la, int lb, int lc, int ld)
+{
+    return la + lb >= 2 && lc + ld >= 2 && la + lb + lc + ld >= 5;
+}
+
 // Pass pm: 0 = FP64, 1 = FP32 quartets; launch_exchange_rys evaluates the FP64
 // and launch_exchange_mixed the FP32 quartets of a class.  variant as
 // vlxb_setSchedule.
@@ -23,10 +34,14 @@ template <int LA, int LB, int LC, int LD>
 int launch_coulomb(int variant, int pm, int grid, cudaStream_t st, const JBraRecs& bra, const JKetPairs& ket,
                    double* mat_J, double thr, const BoysTabs& tab, unsigned long long* qc, double cut, double budget);
 
+template <int LA, int LB, int LC, int LD>
+int launch_coulomb_rys(int grid, cudaStream_t st, const JBraRecs& bra, const JKetPairs& ket, double* mat_J, double thr,
+                       unsigned long long* qc, double cut, double budget);
+
 // out[k * gstride + o], k = 0..5: bra-centre derivatives.
 template <int LA, int LB, int LC, int LD>
 int launch_coulomb_grad(int pm, int grid, cudaStream_t st, const JBraRecs& bra, const JKetPairs& ket, double* out,
-                        int64_t gstride, double thr, const BoysTabs& tab, double cut);
+                        int64_t gstride, double thr, double cut);
 
 // Partner groups of a contracted kernel: the records of one first primitive
 // shell whose partners belong to one contracted shell.

@@ -30,9 +30,10 @@ NVCC_FLAGS = ["-std=c++17", "-O3", "-lineinfo", "-Xcompiler", "-fPIC", "-Xptxas"
 
 HOST_HEADERS = ["common.cuh", "engine.cuh", "jk_kernels.cuh", "launch.cuh", "classes.cuh", "prep.cuh", "md.cuh"]
 CLASS_HEADERS = ["common.cuh", "engine.cuh", "jk_kernels.cuh", "launch.cuh", "class_launch.cuh", "col_kernels.cuh",
-                 "md.cuh", "md_kernels.cuh", "jgrad_kernels.cuh", "tma.cuh", "jtma_kernels.cuh"]
+                 "md.cuh", "md_kernels.cuh", "tma.cuh", "jtma_kernels.cuh"]
 RYS_HEADERS = ["common.cuh", "engine.cuh", "jk_kernels.cuh", "launch.cuh", "rys.cuh", "krys_kernels.cuh"]
 GRAD_HEADERS = RYS_HEADERS + ["kgrad_kernels.cuh"]
+JRYS_HEADERS = ["common.cuh", "engine.cuh", "jk_kernels.cuh", "launch.cuh", "rys.cuh", "md.cuh", "jrys_kernels.cuh"]
 
 
 def _run_generators():
@@ -46,12 +47,14 @@ def _sources():
             os.path.join(CSRC, "noalloc.cu"), os.path.join(CSRC, "aomap.cu"),
             os.path.join(CSRC, "listbuild.cu"), os.path.join(CSRC, "fshell.cu"), os.path.join(CSRC, "rys.cu"),
             os.path.join(GEN, "abi.cu"), os.path.join(GEN, "drivers.cu")]
-    srcs += sorted(glob.glob(os.path.join(GEN, "kgrad_*.cu"))) + sorted(glob.glob(os.path.join(GEN, "krys_*.cu"))) + sorted(glob.glob(os.path.join(GEN, "cls_*.cu")))
+    srcs += sorted(glob.glob(os.path.join(GEN, "jrys_*.cu"))) + sorted(glob.glob(os.path.join(GEN, "kgrad_*.cu"))) + sorted(glob.glob(os.path.join(GEN, "krys_*.cu"))) + sorted(glob.glob(os.path.join(GEN, "cls_*.cu")))
     return srcs
 
 
 def _deps(src):
     base = os.path.basename(src)
+    if base.startswith("jrys_"):
+        return [src] + [os.path.join(CSRC, h) for h in JRYS_HEADERS]
     if base.startswith("kgrad_"):
         return [src] + [os.path.join(CSRC, h) for h in GRAD_HEADERS]
     if base.startswith(("krys_", "rys")):

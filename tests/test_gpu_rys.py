@@ -110,3 +110,27 @@ def test_coulomb_rys_vs_oracle(atoms, degree, side, uneven, threshold):
     g = gradient.CoulombGradient(dl, wl.mol).compute().cpu().numpy()
     go, _ = helpers.oracle_coulomb_gradient(rl, wl.mol.natoms)
     assert close(g, go), float(np.abs(g - go).max())
+
+
+@pytest.mark.parametrize("atoms,omega,cut", [(1, 0.0, 0.0), (3, 0.3, 0.0), (3, 0.0, 1e-6)])
+def test_one_call_build_equals_class_calls(atoms, omega, cut):
+    """vlxb_fockBuild against the 36 + 54 class calls on the same lists: the
+    same kernels on the same preparations, so the same bits."""
+    L = lib()
+    wl, rl = system(atoms, 3, 4.0, 9, False)
+    dl = fock.to_device(rl)
+    s = torch.cuda.current_stream().cuda_stream
+    try:
+        L.set_fp32_cut(cut)
+        matJ, matK = fock.build_jk(dl, omega=omega)
+        refJ, refK = fock.alloc_outputs(dl)
+        for cls in lists.j_classes():
+            L.coulomb(cls, fock.coulomb_args(dl, cls, refJ[cls[:2]], s))
+        for cls in lists.k_classes():
+            L.exchange(cls, fock.exchange_args(dl, cls, refK[cls[0] + cls[2]], s, omega))
+        torch.cuda.synchronize()
+    finally:
+        L.set_fp32_cut(0.0)
+    for a, b in ((matJ, refJ), (matK, refK)):
+        for k in b:
+            assert torch.equal(a[k], b[k]), k

@@ -28,6 +28,7 @@ struct CoulombArgs {
     const int32_t* prim_mol_a;
     const int32_t* prim_mol_c;
     int n_mol;
+    PrepShare* share;  // preparations shared with the other classes of a build, or null
 };
 
 struct ExchangeArgs {
@@ -54,7 +55,83 @@ struct ExchangeArgs {
     uint32_t key_naos;              // bound on the AO indices in aoinds (default: naos)
     const int32_t* prim_mol_a;      // molecule of every type-a primitive
     const double* maxD_mol;         // [molecules] max |D| bound of each molecule
+    PrepShare* share;               // as for CoulombArgs
 };
+
+// The list of type pair (LA, LB) grouped by shell pair.
+template <int LA, int LB>
+int group_jlist(Arena& ar, PrepShare* sh, const CoulombArgs& a, const uint32_t* first, const uint32_t* second,
+                uint32_t n, PairGroups& g)
+{
+    constexpr int P = LA * 3 + LB;
+    if (!sh || !sh->has_jgrp[P]) {
+        const int rc = group_flat(ar, ncart(LA), ncart(LB), (int)a.count[LA], (int)a.count[LB], first, second, n,
+                                  a.info[LA], a.count[LA], a.info[LB], a.count[LB], g);
+        if (rc) return rc;
+        if (sh) {
+            sh->jgrp[P] = g;
+            sh->has_jgrp[P] = true;
+        }
+    } else {
+        g = sh->jgrp[P];
+    }
+    return VLXB_OK;
+}
+
+// Bra records of a Coulomb class (mol: molecule of every record, batched calls).
+template <int LA, int LB>
+int prepare_jbra(Arena& ar, const CoulombArgs& a, bool batched, PairGroups& g, int32_t*& mol)
+{
+    constexpr int P = LA * 3 + LB;
+    PrepShare* sh = a.share;
+    if (sh && sh->has_jbra[P]) {
+        g = sh->jbra[P];
+        mol = sh->jmol[P];
+        return VLXB_OK;
+    }
+    int rc = group_jlist<LA, LB>(ar, sh, a, a.ab_first, a.ab_second, a.n_ab, g);
+    if (rc) return rc;
+    rc = make_records(ar, ncart(LA) * ncart(LB), g, a.ab_Q, a.n_ab);
+    if (rc) return rc;
+    mol = nullptr;
+    if (batched) {
+        rc = bra_record_mol(ar, g, a.prim_mol_a, &mol);
+        if (rc) return rc;
+    }
+    if (sh) {
+        sh->jbra[P] = g;
+        sh->jmol[P] = mol;
+        sh->has_jbra[P] = true;
+    }
+    return VLXB_OK;
+}
+
+// Sorted kets of a Coulomb class.
+template <int LC, int LD>
+int prepare_jket(Arena& ar, const CoulombArgs& a, bool batched, bool hermite, bool budget, JKetData& kd)
+{
+    constexpr int P = LC * 3 + LD;
+    PrepShare* sh = a.share;
+    if (sh && sh->has_jket[P]) {
+        kd = sh->jket[P];
+        return VLXB_OK;
+    }
+    PairGroups g;
+    int rc = group_jlist<LC, LD>(ar, sh, a, a.cd_first, a.cd_second, a.n_cd, g);
+    if (rc) return rc;
+    rc = jket_prepare<LC, LD>(ar, g, a.cd_first, a.cd_second, a.cd_D, a.cd_Q, a.cd_pdata, kd,
+                              batched ? a.prim_mol_c : nullptr, batched ? a.n_mol : 0, hermite || sh != nullptr);
+    if (rc) return rc;
+    if (budget) {
+        rc = budget_prefix_kets(ar, kd, LD);
+        if (rc) return rc;
+    }
+    if (sh) {
+        sh->jket[P] = kd;
+        sh->has_jket[P] = true;
+    }
+    return VLXB_OK;
+}
 
 // Coulomb class call on a given arena (pool, static or measuring) with given
 // Boys tables and quartet counter (may be null).  G = 1: the bra-centre
@@ -73,36 +150,20 @@ int run_coulomb_impl(const CoulombArgs& a, cudaStream_t st, Arena& ar, const Boy
     if (!(a.thr >= 0.0)) return VLXB_EINVAL;
     if (G && gstride < (int64_t)a.n_ab) return VLXB_EINVAL;
     if (!tab.f64 || !tab.f32) return VLXB_ECUDA;
-    constexpr int NA = ncart(LA), NB = ncart(LB), NC = ncart(LC), ND = ncart(LD);
-    PairGroups gb, gk;
-    int rc = group_flat(ar, NA, NB, (int)a.count[LA], (int)a.count[LB], a.ab_first, a.ab_second, a.n_ab,
-                        a.info[LA], a.count[LA], a.info[LB], a.count[LB], gb);
-    if (rc) return rc;
-    rc = make_records(ar, NA * NB, gb, a.ab_Q, a.n_ab);
-    if (rc) return rc;
-    rc = group_flat(ar, NC, ND, (int)a.count[LC], (int)a.count[LD], a.cd_first, a.cd_second, a.n_cd, a.info[LC],
-                    a.count[LC], a.info[LD], a.count[LD], gk);
-    if (rc) return rc;
     const bool batched = a.prim_mol_a && a.prim_mol_c && a.n_mol > 0;
-    JKetData kd;
     const int jvar = schedule_get(0, LA, LB, LC, LD);
     // the Rys and McMurchie-Davidson kernels read the Hermite ket density
     const bool hermite = G || j_rys(LA, LB, LC, LD) || jvar == 2;
-    rc = jket_prepare<LC, LD>(ar, gk, a.cd_first, a.cd_second, a.cd_D, a.cd_Q, a.cd_pdata, kd,
-                              batched ? a.prim_mol_c : nullptr, batched ? a.n_mol : 0, hermite);
-    if (rc) return rc;
     const double budget = (cut > 0.0 && !G) ? fp32_budget_get() : 0.0;
-    if (budget > 0.0) {
-        rc = budget_prefix_kets(ar, kd, LD);
-        if (rc) return rc;
-    }
+    PairGroups gb;
+    JKetData kd;
     int32_t* bmol = nullptr;
-    if (batched) {
-        rc = bra_record_mol(ar, gb, a.prim_mol_a, &bmol);
-        if (rc) return rc;
-    }
+    int rc = prepare_jbra<LA, LB>(ar, a, batched, gb, bmol);
+    if (rc) return rc;
+    rc = prepare_jket<LC, LD>(ar, a, batched, hermite, budget > 0.0, kd);
+    if (rc) return rc;
     if (ar.failed()) return VLXB_ENOMEM;
-    if (ar.measuring()) return VLXB_OK;
+    if (ar.measuring() || (a.share && a.share->prepare_only)) return VLXB_OK;
     JBraRecs bra{gb.rec_sp, gb.rec_q, gb.rec_mask, gb.n_rec, gb.geo, gb.entry, gb.sp_stride, a.ab_pdata, bmol};
     JKetPairs ket{kd.geo, kd.tmax, kd.tmin, kd.Dpp, kd.Dm, kd.Qc, kd.Dc, kd.stride, kd.n, batched ? kd.seg : nullptr,
                   kd.Dh, kd.tpre};
@@ -131,6 +192,7 @@ int run_coulomb(const CoulombArgs& a, cudaStream_t st)
     if (rc) return rc;
     const BoysTabs tab{boys_table_device(), boys_table32_device()};
     if (!tab.f64 || !tab.f32) return VLXB_ECUDA;
+    if (a.share) return run_coulomb_impl<LA, LB, LC, LD>(a, st, a.share->ar, tab, quartet_counters_device(), fp32_cut_get());
     Arena ar(st);
     return run_coulomb_impl<LA, LB, LC, LD>(a, st, ar, tab, quartet_counters_device(), fp32_cut_get());
 }
@@ -145,8 +207,84 @@ int run_coulomb_grad(const CoulombArgs& a, int64_t gstride, cudaStream_t st)
     if (rc) return rc;
     const BoysTabs tab{boys_table_device(), boys_table32_device()};
     if (!tab.f64 || !tab.f32) return VLXB_ECUDA;
+    if (a.share) return run_coulomb_impl<LA, LB, LC, LD, 1>(a, st, a.share->ar, tab, nullptr, fp32_cut_get(), gstride);
     Arena ar(st);
     return run_coulomb_impl<LA, LB, LC, LD, 1>(a, st, ar, tab, nullptr, fp32_cut_get(), gstride);
+}
+
+// Whether a pair of types is a side of some class whose FP32 quartets run on a
+// contracted kernel.
+constexpr bool k_pair_contracted(int la, int lb)
+{
+    for (int x = 0; x < 3; x++)
+        for (int y = 0; y < 3; y++)
+            if ((la <= x && k_contracted(la, lb, x, y)) || (x <= la && k_contracted(x, y, la, lb))) return true;
+    return false;
+}
+
+// Partner records of type pair (LX, LY) from its CSR list; with FP32 on, the
+// partner groups where a class needs them and the error budget's prefix sums.
+template <int LX, int LY>
+int prepare_kpart(Arena& ar, const ExchangeArgs& a, const uint32_t* displs, const uint32_t* counts,
+                  const uint32_t* Dinds, const double* Q, const double* pdata, double cut, bool contracted,
+                  PairGroups& g)
+{
+    constexpr int P = LX * 3 + LY, NX = ncart(LX), NY = ncart(LY);
+    PrepShare* sh = a.share;
+    if (sh && sh->has_kpart[P]) {
+        g = sh->kpart[P];
+        return VLXB_OK;
+    }
+    const int npx = (int)a.count[LX], npy = (int)a.count[LY];
+    int rc = group_csr(ar, NX, NY, npx, npy, displs, counts, Dinds, (int64_t)npx * npy, a.info[LX], a.count[LX],
+                       a.info[LY], a.count[LY], g);
+    if (rc) return rc;
+    rc = make_records(ar, NX * NY, g, Q, (int64_t)npx * npy * NX * NY);
+    if (rc) return rc;
+    rc = segment_records(ar, NX * NY, npx, npy, g, pdata);
+    if (rc) return rc;
+    if (cut > 0.0 && (sh ? k_pair_contracted(LX, LY) : contracted)) {
+        rc = contract_groups(ar, npx, g, a.aoinds[LY], a.key_naos ? a.key_naos : a.naos);
+        if (rc) return rc;
+    }
+    if (cut > 0.0 && fp32_budget_get() > 0.0) {
+        // after contract_groups: groups get their amplified sums too
+        rc = budget_prefix_records(ar, g, npx, LY);
+        if (rc) return rc;
+    }
+    if (sh) {
+        sh->kpart[P] = g;
+        sh->has_kpart[P] = true;
+    }
+    return VLXB_OK;
+}
+
+// Output blocks and both sides' partner records of an exchange class.
+template <int LA, int LB, int LC, int LD>
+int prepare_exchange(Arena& ar, const ExchangeArgs& a, double cut, KOutData& ko, PairGroups& gab, PairGroups& gcd)
+{
+    constexpr int P = LA * 3 + LC;
+    constexpr bool CONTRACTED = k_rys(LA, LB, LC, LD) && k_contracted(LA, LB, LC, LD);
+    PrepShare* sh = a.share;
+    int rc;
+    if (sh && sh->has_kout[P]) {
+        ko = sh->kout[P];
+    } else {
+        rc = kout_prepare(ar, ncart(LA), ncart(LC), (int)a.count[LA], (int)a.count[LC], a.pair_i, a.pair_k, a.n_ik, ko);
+        if (rc) return rc;
+        if (sh) {
+            sh->kout[P] = ko;
+            sh->has_kout[P] = true;
+        }
+    }
+    rc = prepare_kpart<LA, LB>(ar, a, a.displs_ab, a.counts_ab, a.Dinds_ab, a.Q_ab, a.pdata_ab, cut, CONTRACTED, gab);
+    if (rc) return rc;
+    if (LA == LC && LB == LD && a.Q_ab == a.Q_cd && a.Dinds_ab == a.Dinds_cd && a.displs_ab == a.displs_cd &&
+        a.counts_ab == a.counts_cd && a.pdata_ab == a.pdata_cd) {
+        gcd = gab;
+        return VLXB_OK;
+    }
+    return prepare_kpart<LC, LD>(ar, a, a.displs_cd, a.counts_cd, a.Dinds_cd, a.Q_cd, a.pdata_cd, cut, CONTRACTED, gcd);
 }
 
 template <int LA, int LB, int LC, int LD>
@@ -165,69 +303,28 @@ int run_exchange(const ExchangeArgs& a, cudaStream_t st)
     const BoysTabs tab{boys_table_device(), boys_table32_device()};
     if (!tab.f64 || !tab.f32) return VLXB_ECUDA;
     const double cut = fp32_cut_get();
-    constexpr int NA = ncart(LA), NB = ncart(LB), NC = ncart(LC), ND = ncart(LD);
-    Arena ar(st);
+    Arena local(st);
+    Arena& ar = a.share ? a.share->ar : local;
     KOutData ko;
-    rc = kout_prepare(ar, NA, NC, (int)a.count[LA], (int)a.count[LC], a.pair_i, a.pair_k, a.n_ik, ko);
+    PairGroups gab, gcd;
+    rc = prepare_exchange<LA, LB, LC, LD>(ar, a, cut, ko, gab, gcd);
     if (rc) return rc;
-    const int npa = (int)a.count[LA], npb = (int)a.count[LB], npc = (int)a.count[LC], npd = (int)a.count[LD];
-    PairGroups gab;
-    rc = group_csr(ar, NA, NB, npa, npb, a.displs_ab, a.counts_ab, a.Dinds_ab, (int64_t)npa * npb, a.info[LA],
-                   a.count[LA], a.info[LB], a.count[LB], gab);
-    if (rc) return rc;
-    rc = make_records(ar, NA * NB, gab, a.Q_ab, (int64_t)npa * npb * NA * NB);
-    if (rc) return rc;
-    rc = segment_records(ar, NA * NB, npa, npb, gab, a.pdata_ab);
-    if (rc) return rc;
-    PairGroups gcd;
-    const bool same = (LA == LC && LB == LD && a.Q_ab == a.Q_cd && a.Dinds_ab == a.Dinds_cd &&
-                       a.displs_ab == a.displs_cd && a.counts_ab == a.counts_cd && a.pdata_ab == a.pdata_cd);
-    if (same) {
-        gcd = gab;
-    } else {
-        rc = group_csr(ar, NC, ND, npc, npd, a.displs_cd, a.counts_cd, a.Dinds_cd, (int64_t)npc * npd, a.info[LC],
-                       a.count[LC], a.info[LD], a.count[LD], gcd);
-        if (rc) return rc;
-        rc = make_records(ar, NC * ND, gcd, a.Q_cd, (int64_t)npc * npd * NC * ND);
-        if (rc) return rc;
-        rc = segment_records(ar, NC * ND, npc, npd, gcd, a.pdata_cd);
-        if (rc) return rc;
-    }
     const double budget = cut > 0.0 ? fp32_budget_get() : 0.0;
-    constexpr bool CONTRACTED = k_rys(LA, LB, LC, LD) && k_contracted(LA, LB, LC, LD);
     [[maybe_unused]] KGroups kgab{}, kgcd{};
-    if (CONTRACTED && cut > 0.0) {
-        rc = contract_groups(ar, npa, gab, a.aoinds[LB], a.key_naos ? a.key_naos : a.naos);
-        if (rc) return rc;
-        if (same) {
-            gcd = gab;
-        } else {
-            rc = contract_groups(ar, npc, gcd, a.aoinds[LD], a.key_naos ? a.key_naos : a.naos);
-            if (rc) return rc;
-        }
-    }
-    if (budget > 0.0) {
-        // after contract_groups: groups get their amplified sums too
-        rc = budget_prefix_records(ar, gab, npa, LB);
-        if (rc) return rc;
-        if (same) {
-            gcd = gab;
-        } else {
-            rc = budget_prefix_records(ar, gcd, npc, LD);
-            if (rc) return rc;
-        }
-    }
-    if (CONTRACTED && cut > 0.0) {
+    if (k_rys(LA, LB, LC, LD) && k_contracted(LA, LB, LC, LD) && cut > 0.0) {
         kgab = KGroups{gab.gseg, gab.gq, gab.gbeg, gab.gcnt, gab.msp, gab.mq, gab.msu, gab.mmask, gab.gqa, gab.gqpre,
                        gab.rec_grp};
         kgcd = KGroups{gcd.gseg, gcd.gq, gcd.gbeg, gcd.gcnt, gcd.msp, gcd.mq, gcd.msu, gcd.mmask, gcd.gqa, gcd.gqpre,
                        gcd.rec_grp};
     }
-    double* blk_maxD = nullptr;
-    if (a.prim_mol_a && a.maxD_mol) {
+    double* blk_maxD = a.share ? a.share->maxd[LA * 3 + LC][LB * 3 + LD] : nullptr;
+    if (a.prim_mol_a && a.maxD_mol && !blk_maxD) {
         rc = kout_block_maxd(ar, ko, a.prim_mol_a, a.maxD_mol, &blk_maxD);
         if (rc) return rc;
+        if (a.share) a.share->maxd[LA * 3 + LC][LB * 3 + LD] = blk_maxD;
     }
+    if (ar.failed()) return VLXB_ENOMEM;
+    if (a.share && a.share->prepare_only) return VLXB_OK;
     KOutBlocks out{ko.ish, ko.ksh, ko.idx, ko.stride, ko.n, blk_maxD};
     KPartnerRecs rab{gab.rec_sp, gab.rec_q, gab.rec_mask, gab.seg, gab.geo, gab.S, gab.sp_j, gab.sp_stride, gab.su,
                      gab.rec_qa, gab.rec_qpre};
@@ -239,7 +336,6 @@ int run_exchange(const ExchangeArgs& a, cudaStream_t st)
     unsigned long long* qk = qc ? qc + 1 : nullptr;
     const KDensity dm{a.aoinds[LB], a.count[LB], a.aoinds_col[LD] ? a.aoinds_col[LD] : a.aoinds[LD], a.count[LD],
                       a.D, a.D_stride ? a.D_stride : a.naos};
-    if (ar.failed()) return VLXB_ENOMEM;
     for (int pm = 0; pm < (cut > 0.0 ? 2 : 1); pm++) {
         if constexpr (!k_rys(LA, LB, LC, LD))
             rc = launch_exchange_thread<LA, LB, LC, LD>(pm, grid, st, out, rab, rcd, dm, a.maxD, a.omega, a.thr,
@@ -273,35 +369,14 @@ int run_exchange_grad(const ExchangeArgs& a, int64_t gstride, cudaStream_t st)
     if (gstride < (int64_t)a.n_ik) return VLXB_EINVAL;
     int rc = ensure_pool_configured();
     if (rc) return rc;
-    constexpr int NA = ncart(LA), NB = ncart(LB), NC = ncart(LC), ND = ncart(LD);
-    Arena ar(st);
+    Arena local(st);
+    Arena& ar = a.share ? a.share->ar : local;
     KOutData ko;
-    rc = kout_prepare(ar, NA, NC, (int)a.count[LA], (int)a.count[LC], a.pair_i, a.pair_k, a.n_ik, ko);
+    PairGroups gab, gcd;
+    rc = prepare_exchange<LA, LB, LC, LD>(ar, a, 0.0, ko, gab, gcd);
     if (rc) return rc;
-    const int npa = (int)a.count[LA], npb = (int)a.count[LB], npc = (int)a.count[LC], npd = (int)a.count[LD];
-    PairGroups gab;
-    rc = group_csr(ar, NA, NB, npa, npb, a.displs_ab, a.counts_ab, a.Dinds_ab, (int64_t)npa * npb, a.info[LA],
-                   a.count[LA], a.info[LB], a.count[LB], gab);
-    if (rc) return rc;
-    rc = make_records(ar, NA * NB, gab, a.Q_ab, (int64_t)npa * npb * NA * NB);
-    if (rc) return rc;
-    rc = segment_records(ar, NA * NB, npa, npb, gab, a.pdata_ab);
-    if (rc) return rc;
-    PairGroups gcd;
-    const bool same = (LA == LC && LB == LD && a.Q_ab == a.Q_cd && a.Dinds_ab == a.Dinds_cd &&
-                       a.displs_ab == a.displs_cd && a.counts_ab == a.counts_cd && a.pdata_ab == a.pdata_cd);
-    if (same) {
-        gcd = gab;
-    } else {
-        rc = group_csr(ar, NC, ND, npc, npd, a.displs_cd, a.counts_cd, a.Dinds_cd, (int64_t)npc * npd, a.info[LC],
-                       a.count[LC], a.info[LD], a.count[LD], gcd);
-        if (rc) return rc;
-        rc = make_records(ar, NC * ND, gcd, a.Q_cd, (int64_t)npc * npd * NC * ND);
-        if (rc) return rc;
-        rc = segment_records(ar, NC * ND, npc, npd, gcd, a.pdata_cd);
-        if (rc) return rc;
-    }
     if (ar.failed()) return VLXB_ENOMEM;
+    if (a.share && a.share->prepare_only) return VLXB_OK;
     KOutBlocks out{ko.ish, ko.ksh, ko.idx, ko.stride, ko.n, nullptr};
     KPartnerRecs rab{gab.rec_sp, gab.rec_q, gab.rec_mask, gab.seg, gab.geo, gab.S, gab.sp_j, gab.sp_stride, gab.su,
                      nullptr, nullptr};

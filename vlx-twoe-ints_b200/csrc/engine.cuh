@@ -68,6 +68,17 @@ class Arena {
         ptrs_.push_back(p);
         return (T*)p;
     }
+    // Hand one buffer back before the arena ends (pool mode; stream-ordered).
+    void release(void* p)
+    {
+        for (size_t k = ptrs_.size(); k-- > 0;)
+            if (ptrs_[k] == p) {
+                cudaFreeAsync(p, stream_);
+                ptrs_[k] = ptrs_.back();
+                ptrs_.pop_back();
+                return;
+            }
+    }
     bool failed() const { return failed_; }
     bool measuring() const { return measure_; }
     size_t used() const { return used_; }
@@ -216,6 +227,21 @@ int kout_block_maxd(Arena& ar, const KOutData& ko, const int32_t* prim_mol_a, co
                     double** out);
 
 int launch_grid_limit();
+
+// List preparations shared by the class calls of one build, by type pair
+// (la * 3 + lb): a build has one J list per pair, one partner list per ordered
+// pair and one (i, k) list per pair, so 27 preparations serve its 90 classes.
+struct PrepShare {
+    explicit PrepShare(cudaStream_t s) : ar(s) {}
+    Arena ar;
+    bool has_jgrp[9] = {}, has_jbra[9] = {}, has_jket[9] = {}, has_kpart[9] = {}, has_kout[9] = {};
+    PairGroups jgrp[9], jbra[9], kpart[9];
+    int32_t* jmol[9] = {};
+    JKetData jket[9];
+    KOutData kout[9];
+    double* maxd[9][9] = {};    // per-block max |D| by output pair and (b, d) (batched builds)
+    bool prepare_only = false;  // the class calls prepare their lists and launch nothing
+};
 
 // Kernel variant per class: kind 0 = Coulomb (0 thread-per-quartet, 1 column),
 // kind 1 = exchange (0 thread-per-quartet, 1 column with bra lanes, 2 column

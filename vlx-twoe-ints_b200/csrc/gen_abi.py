@@ -284,6 +284,48 @@ def header():
          "} VlxbBatchCall;",
          "int vlxb_coulombBatch(int la, int lb, int lc, int ld, const VlxbBatchCall* call, void* stream);",
          "int vlxb_exchangeBatch(int la, int lb, int lc, int ld, const VlxbBatchCall* call, void* stream);", "",
+         "/* All class calls of one build, or of its nuclear gradient, in one call: each",
+         "   list is regrouped on the device once instead of once per class that reads",
+         "   it.  Same kernels, screening and results as the class calls in the order",
+         "   of this header.  Arrays are indexed by type (s, p, d) or by type pair",
+         "   la * 3 + lb: J lists and (i, k) lists for la <= lb, partner lists and",
+         "   maxD for every ordered pair (maxD: b * 3 + d).  j_classes / k_classes: bit",
+         "   t selects the t-th Coulomb / exchange class of this header; the lists of",
+         "   selected classes must be given (a list of count 0 is empty).  gradient 0:",
+         "   mat_J / mat_K as the Fock entry points; 1: mat_J / mat_K are the grad_J /",
+         "   grad_K columns of vlxb_computeCoulombGradient / ...ExchangeGradient with",
+         "   row stride grad_stride.  n_mol > 0: a batch as for vlxb_coulombBatch /",
+         "   vlxb_exchangeBatch (prim_mol, prim_aocols, D_stride, maxD_mol), else those",
+         "   are ignored (D_stride 0 = naos).  All preparations are held until the",
+         "   call's work is done on the stream; VLXB_ENOMEM is returned before any",
+         "   output is touched, and the class calls, which hold one class's at a time,",
+         "   remain.  No reference counterpart. */",
+         "typedef struct VlxbFockBuild {",
+         "    const double* prim_info[3];",
+         "    const uint32_t* prim_aoinds[3];",
+         "    const uint32_t* prim_aocols[3];",
+         "    const int32_t* prim_mol[3];",
+         "    uint32_t prim_count[3];",
+         "    int32_t n_mol;",
+         "    double* mat_J[9];",
+         "    const uint32_t *j_first[9], *j_second[9];",
+         "    const double *j_pdata[9], *j_Q[9], *j_D[9];",
+         "    uint32_t j_count[9];",
+         "    int32_t gradient;",
+         "    double* mat_K[9];",
+         "    const uint32_t *k_i[9], *k_k[9];",
+         "    const uint32_t *kp_displs[9], *kp_counts[9], *kp_Dinds[9];",
+         "    const double *kp_Q[9], *kp_pdata[9];",
+         "    const double* maxD_mol[9];",
+         "    double maxD[9];",
+         "    uint32_t k_count[9];",
+         "    uint32_t naos;",
+         "    const double* D;",
+         "    uint64_t j_classes, k_classes, grad_stride;",
+         "    uint32_t D_stride;",
+         "    double omega, thr;",
+         "} VlxbFockBuild;",
+         "int vlxb_fockBuild(const VlxbFockBuild* build, void* stream);", "",
          "/* Allocation-free variant of vlxb_computeCoulombFockSSSS (same arguments,",
          "   same result) for callers that cannot allocate device memory, e.g. hosts",
          "   whose device memory is owned by their own allocator, or plugins that are",
@@ -594,6 +636,14 @@ def driver_tu():
         L.append(f"int exchange_{cls}(const ExchangeArgs& a, cudaStream_t s) {{ return run_exchange<{t}>(a, s); }}")
         L.append(f"int exchange_grad_{cls}(const ExchangeArgs& a, int64_t gs, cudaStream_t s) "
                  f"{{ return run_exchange_grad<{t}>(a, gs, s); }}")
+    for kind, args, classes in (("coulomb", "CoulombArgs", j_classes()), ("exchange", "ExchangeArgs", k_classes())):
+        L += [f"int dispatch_{kind}(int cls, bool grad, const {args}& a, int64_t gs, cudaStream_t s)", "{",
+              "    switch (cls) {"]
+        for cls in classes:
+            la, lb, lc, ld = (LV[x] for x in cls)
+            L.append(f"        case {la * 27 + lb * 9 + lc * 3 + ld}: "
+                     f"return grad ? {kind}_grad_{cls}(a, gs, s) : {kind}_{cls}(a, s);")
+        L += ["        default: return VLXB_EINVAL;", "    }", "}"]
     L += ["}  // namespace vlxb", ""]
     return "\n".join(L)
 

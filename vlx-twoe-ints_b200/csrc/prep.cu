@@ -268,6 +268,7 @@ int group_flat(Arena& ar, int na, int nb, int npa, int npb, const uint32_t* firs
         k_fill_pairs<<<prep_blocks(n), PREP_THREADS, 0, st>>>(first, second, n, na, nb, npb, g.spidx, g.entry, g.sp_i,
                                                               g.sp_j, g.sp_stride);
     }
+    ar.release(table);
     if (!ar.measuring()) note_launches();
     if (!ar.measuring()) {
         k_pair_geo<<<prep_blocks(g.sp_stride), PREP_THREADS, 0, st>>>(g.n_sp, g.sp_i, g.sp_j, info_a, cnt_a, info_b,
@@ -304,6 +305,7 @@ int group_csr(Arena& ar, int na, int nb, int npa, int npb, const uint32_t* displ
         k_fill_csr<<<prep_blocks(n_first), PREP_THREADS, 0, st>>>(displs, counts, Dinds, n_first, na, nb, npb, g.spidx,
                                                                   g.entry, g.sp_i, g.sp_j, g.sp_stride);
     }
+    ar.release(table);
     if (!ar.measuring()) note_launches();
     if (!ar.measuring()) {
         k_pair_geo<<<prep_blocks(g.sp_stride), PREP_THREADS, 0, st>>>(g.n_sp, g.sp_i, g.sp_j, info_a, cnt_a, info_b,

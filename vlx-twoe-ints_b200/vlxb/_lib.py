@@ -45,6 +45,20 @@ def _ctype(decl: str):
     raise ValueError(decl)
 
 
+class VlxbFockBuild(ctypes.Structure):
+    """Mirror of VlxbFockBuild in include/vlxb.h."""
+    _fields_ = [(n, ctypes.c_void_p * 3) for n in ("prim_info", "prim_aoinds", "prim_aocols", "prim_mol")] + [
+        ("prim_count", ctypes.c_uint32 * 3), ("n_mol", ctypes.c_int32)] + [
+        (n, ctypes.c_void_p * 9) for n in ("mat_J", "j_first", "j_second", "j_pdata", "j_Q", "j_D")] + [
+        ("j_count", ctypes.c_uint32 * 9), ("gradient", ctypes.c_int32)] + [
+        (n, ctypes.c_void_p * 9) for n in ("mat_K", "k_i", "k_k", "kp_displs", "kp_counts", "kp_Dinds", "kp_Q",
+                                           "kp_pdata", "maxD_mol")] + [
+        ("maxD", ctypes.c_double * 9), ("k_count", ctypes.c_uint32 * 9), ("naos", ctypes.c_uint32),
+        ("D", ctypes.c_void_p), ("j_classes", ctypes.c_uint64), ("k_classes", ctypes.c_uint64),
+        ("grad_stride", ctypes.c_uint64), ("D_stride", ctypes.c_uint32), ("omega", ctypes.c_double),
+        ("thr", ctypes.c_double)]
+
+
 class Lib:
     def __init__(self, path: str = LIB_PATH):
         if not os.path.exists(path):
@@ -61,6 +75,8 @@ class Lib:
             f.argtypes = [_ctype(p) for p in ps]
             f.restype = ctypes.c_int
             self.j_params[cls] = [ABI.pname(p) for p in ps]
+        self.j_bit = {c: t for t, c in enumerate(ABI.j_classes())}
+        self.k_bit = {c: t for t, c in enumerate(ABI.k_classes())}
         self.g_params = {}
         for cls in ABI.j_classes():
             ps = ABI.g_params(cls)
@@ -115,6 +131,8 @@ class Lib:
                                        ctypes.c_void_p, ctypes.c_int64, ctypes.c_void_p, ctypes.c_void_p]
         c.vlxb_pairGradientToAtoms.argtypes = [ctypes.c_void_p, ctypes.c_uint64, ctypes.c_void_p, ctypes.c_void_p,
                                                ctypes.c_void_p, ctypes.c_int32, ctypes.c_void_p, ctypes.c_void_p]
+        c.vlxb_fockBuild.argtypes = [ctypes.c_void_p, ctypes.c_void_p]
+        c.vlxb_fockBuild.restype = ctypes.c_int
         for fn in (c.vlxb_coulombBatch, c.vlxb_exchangeBatch):
             fn.argtypes = [ctypes.c_int] * 4 + [ctypes.c_void_p, ctypes.c_void_p]
             fn.restype = ctypes.c_int
@@ -145,6 +163,18 @@ class Lib:
         vals = [args[n] for n in self.k_params[cls]]
         rc = getattr(self.cdll, f"vlxb_computeExchangeFock{cls.upper()}")(*vals)
         self.check(rc, f"vlxb_computeExchangeFock{cls.upper()}")
+
+    def fock_build(self, build: VlxbFockBuild, j_classes, k_classes, stream: int = 0) -> bool:
+        """vlxb_fockBuild for the given classes.  False: the shared preparations
+        do not fit in device memory (no output touched); the class calls, which
+        hold one class's at a time, may."""
+        build.j_classes = sum(1 << self.j_bit[c] for c in j_classes)
+        build.k_classes = sum(1 << self.k_bit[c] for c in k_classes)
+        rc = self.cdll.vlxb_fockBuild(ctypes.addressof(build), stream)
+        if rc == 3:  # VLXB_ENOMEM
+            return False
+        self.check(rc, "vlxb_fockBuild")
+        return True
 
     def quartet_counters(self, reset: bool = True, stream: int = 0):
         out = (ctypes.c_ulonglong * 2)()

@@ -25,7 +25,7 @@ import numpy as np
 import torch
 
 from . import fock, lists
-from ._lib import lib
+from ._lib import VlxbFockBuild, lib
 from .lists import ANG, LV, NCART
 
 
@@ -200,6 +200,34 @@ class FusedBatch:
         c.omega = self.omega
         return c
 
+    def _build(self) -> VlxbFockBuild:
+        """All class calls of one iteration (vlxb_fockBuild over the union)."""
+        b, d = VlxbFockBuild(), self.d
+        t = lambda key: LV[key[0]] * 3 + LV[key[1]]  # noqa: E731
+        for l in range(3):
+            if self.count[l]:
+                b.prim_info[l], b.prim_aoinds[l] = d[f"info{l}"].data_ptr(), d[f"row{l}"].data_ptr()
+                b.prim_aocols[l], b.prim_mol[l] = d[f"col{l}"].data_ptr(), d[f"mol{l}"].data_ptr()
+                b.prim_count[l] = self.count[l]
+        for k in self.jkeys:
+            b.mat_J[t(k)] = self.matJ[k].data_ptr()
+            for n in ("first", "second", "pdata", "Q", "D"):
+                getattr(b, f"j_{n}")[t(k)] = d[f"j_{k}_{n}"].data_ptr()
+            b.j_count[t(k)] = d[f"j_{k}_first"].numel()
+        for k in self.kpkeys:
+            for n in ("displs", "counts", "Dinds", "Q", "pdata"):
+                getattr(b, f"kp_{n}")[t(k)] = d[f"kp_{k}_{n}"].data_ptr()
+        for k in self.kkeys:
+            b.mat_K[t(k)] = self.matK[k].data_ptr()
+            b.k_i[t(k)], b.k_k[t(k)] = d[f"kq_{k}_i"].data_ptr(), d[f"kq_{k}_k"].data_ptr()
+            b.k_count[t(k)] = d[f"kq_{k}_i"].numel()
+        for k in self.maxD_keys:
+            if "f" not in k:
+                b.maxD_mol[t(k)] = d[f"maxD_{k}"].data_ptr()
+        b.D, b.D_stride, b.naos = d["Dstack"].data_ptr(), self.W, self.naos
+        b.n_mol, b.thr, b.omega = self.nmol, self.threshold, self.omega
+        return b
+
     def _coulomb(self, cls, stream):
         ab, cd = cls[:2], cls[2:]
         if ab not in self.jkeys or cd not in self.jkeys:
@@ -240,10 +268,14 @@ class FusedBatch:
         with torch.cuda.stream(st):
             for t in list(self.matJ.values()) + list(self.matK.values()):
                 t.zero_()
-            for cls in lists.j_classes():
-                self._coulomb(cls, st.cuda_stream)
-            for cls in lists.k_classes():
-                self._exchange(cls, st.cuda_stream)
+            jcls = [c for c in lists.j_classes() if c[:2] in self.jkeys and c[2:] in self.jkeys]
+            kcls = [c for c in lists.k_classes()
+                    if c[0] + c[2] in self.kkeys and c[:2] in self.kpkeys and c[2:] in self.kpkeys]
+            if not self.L.fock_build(self._build(), jcls, kcls, st.cuda_stream):
+                for cls in jcls:
+                    self._coulomb(cls, st.cuda_stream)
+                for cls in kcls:
+                    self._exchange(cls, st.cuda_stream)
 
     def capture(self):
         """Capture one iteration into a CUDA graph (after an eager warm-up)."""

@@ -46,6 +46,7 @@ def _sources():
     srcs = [os.path.join(CSRC, "prep.cu"), os.path.join(CSRC, "api.cu"), os.path.join(CSRC, "schwarz.cu"),
             os.path.join(CSRC, "noalloc.cu"), os.path.join(CSRC, "aomap.cu"),
             os.path.join(CSRC, "listbuild.cu"), os.path.join(CSRC, "fshell.cu"), os.path.join(CSRC, "rys.cu"),
+            os.path.join(CSRC, "fockbuild.cu"),
             os.path.join(GEN, "abi.cu"), os.path.join(GEN, "drivers.cu")]
     srcs += sorted(glob.glob(os.path.join(GEN, "jrys_*.cu"))) + sorted(glob.glob(os.path.join(GEN, "kgrad_*.cu"))) + sorted(glob.glob(os.path.join(GEN, "krys_*.cu"))) + sorted(glob.glob(os.path.join(GEN, "cls_*.cu")))
     return srcs

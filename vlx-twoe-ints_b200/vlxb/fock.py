@@ -13,7 +13,7 @@ from dataclasses import dataclass, field
 import numpy as np
 import torch
 
-from ._lib import lib
+from ._lib import VlxbFockBuild, lib
 from .lists import ANG, LMAX, LV, ReferenceLists, j_classes_all, k_classes_all
 
 
@@ -153,26 +153,72 @@ def alloc_outputs(dl: DeviceLists):
     return matJ, matK
 
 
+def build_call(dl: DeviceLists, omega: float = 0.0) -> VlxbFockBuild:
+    """VlxbFockBuild over the s, p and d lists of `dl` (outputs not set)."""
+    b = VlxbFockBuild()
+    for l in range(3):
+        if l in dl.info:
+            b.prim_info[l], b.prim_aoinds[l] = _p(dl.info[l]), _p(dl.aoinds[l])
+            b.prim_count[l] = dl.count[l]
+    for key, jl in dl.j.items():
+        if "f" in key:
+            continue
+        t = LV[key[0]] * 3 + LV[key[1]]
+        b.j_first[t], b.j_second[t] = _p(jl["first"]), _p(jl["second"])
+        b.j_pdata[t], b.j_Q[t], b.j_D[t] = _p(jl["pdata"]), _p(jl["Q"]), _p(jl["D"])
+        b.j_count[t] = jl["first"].numel()
+    for key, kp in dl.kpart.items():
+        if "f" in key:
+            continue
+        t = LV[key[0]] * 3 + LV[key[1]]
+        b.kp_displs[t], b.kp_counts[t], b.kp_Dinds[t] = _p(kp["displs"]), _p(kp["counts"]), _p(kp["Dinds"])
+        b.kp_Q[t], b.kp_pdata[t] = _p(kp["Q"]), _p(kp["pdata"])
+    for key, kq in dl.kpair.items():
+        if "f" in key:
+            continue
+        t = LV[key[0]] * 3 + LV[key[1]]
+        b.k_i[t], b.k_k[t] = _p(kq["i"]), _p(kq["k"])
+        b.k_count[t] = kq["i"].numel()
+    for key, v in dl.maxD.items():
+        if "f" not in key:
+            b.maxD[LV[key[0]] * 3 + LV[key[1]]] = v
+    b.D = _p(dl.D_AO)
+    b.naos = dl.naos
+    b.omega = omega
+    b.thr = dl.threshold
+    return b
+
+
 def build_jk(dl: DeviceLists, stream: torch.cuda.Stream | None = None, omega: float = 0.0,
              j_only=None, k_only=None, matJ=None, matK=None, do_j=True, do_k=True):
-    """Launch every J and K class through the C ABI on `stream` (asynchronous).
-    Returns (matJ, matK): device tensors in prim-cart pair space."""
+    """Launch every J and K class through the C ABI on `stream` (asynchronous):
+    the s, p and d classes in one vlxb_fockBuild, which prepares each list once,
+    classes with f shells through their entry points.  Returns (matJ, matK):
+    device tensors in prim-cart pair space."""
     L = lib()
     if stream is None:
         stream = torch.cuda.current_stream(dl.device)
     s = stream.cuda_stream
     if matJ is None or matK is None:
         matJ, matK = alloc_outputs(dl)
+    jcls = [c for c in ((j_only or j_classes_all()) if do_j else []) if c[:2] in dl.j and c[2:] in dl.j]
+    kcls = [c for c in ((k_only or k_classes_all()) if do_k else [])
+            if c[0] + c[2] in dl.kpair and c[:2] in dl.kpart and c[2:] in dl.kpart]
     with torch.cuda.stream(stream):
-        if do_j:
-            for cls in (j_only or j_classes_all()):
-                if cls[:2] in dl.j and cls[2:] in dl.j:
-                    L.coulomb(cls, coulomb_args(dl, cls, matJ[cls[:2]], s))
-        if do_k:
-            for cls in (k_only or k_classes_all()):
-                ac = cls[0] + cls[2]
-                if ac in dl.kpair and cls[:2] in dl.kpart and cls[2:] in dl.kpart:
-                    L.exchange(cls, exchange_args(dl, cls, matK[ac], s, omega))
+        spd = [c for c in jcls if "f" not in c], [c for c in kcls if "f" not in c]
+        if len(spd[0]) == len(set(spd[0])) and len(spd[1]) == len(set(spd[1])):  # a mask holds a class once
+            b = build_call(dl, omega)
+            for key in {c[:2] for c in spd[0]}:
+                b.mat_J[LV[key[0]] * 3 + LV[key[1]]] = _p(matJ[key])
+            for key in {c[0] + c[2] for c in spd[1]}:
+                b.mat_K[LV[key[0]] * 3 + LV[key[1]]] = _p(matK[key])
+            if L.fock_build(b, spd[0], spd[1], s):
+                jcls = [c for c in jcls if "f" in c]
+                kcls = [c for c in kcls if "f" in c]
+        for cls in jcls:
+            L.coulomb(cls, coulomb_args(dl, cls, matJ[cls[:2]], s))
+        for cls in kcls:
+            L.exchange(cls, exchange_args(dl, cls, matK[cls[0] + cls[2]], s, omega))
     return matJ, matK
 
 

@@ -35,7 +35,7 @@ import numpy as np
 import torch
 
 from ._lib import lib
-from .fock import DeviceLists, exchange_args
+from .fock import DeviceLists, build_call, exchange_args
 from .lists import ANG, LV, NCART, j_classes, k_classes, prim_data
 
 
@@ -140,10 +140,17 @@ def pair_gradients(dl: DeviceLists, gmap: GradientMap, stream=None, classes=None
     L = lib()
     st = stream or torch.cuda.current_stream(dl.device)
     G = torch.zeros((6, max(gmap.total, 1)), dtype=torch.float64, device=dl.device)
+    run = [c for c in (classes or j_classes()) if c[:2] in dl.j and c[2:] in dl.j]
     with torch.cuda.stream(st):
-        for cls in (classes or j_classes()):
-            if cls[:2] in dl.j and cls[2:] in dl.j:
-                L.coulomb_grad(cls, grad_args(dl, cls, G, gmap.offsets[cls[:2]], G.shape[1], st.cuda_stream))
+        if len(run) == len(set(run)):  # a mask holds a class once
+            b = build_call(dl)
+            b.gradient, b.grad_stride = 1, G.shape[1]
+            for key in {c[:2] for c in run}:
+                b.mat_J[LV[key[0]] * 3 + LV[key[1]]] = G.data_ptr() + 8 * gmap.offsets[key]
+            if L.fock_build(b, run, [], st.cuda_stream):
+                run = []
+        for cls in run:
+            L.coulomb_grad(cls, grad_args(dl, cls, G, gmap.offsets[cls[:2]], G.shape[1], st.cuda_stream))
     return G
 
 
@@ -154,11 +161,19 @@ def exchange_pair_gradients(dl: DeviceLists, kmap: GradientMap, stream=None, ome
     L = lib()
     st = stream or torch.cuda.current_stream(dl.device)
     G = torch.zeros((6, max(kmap.total, 1)), dtype=torch.float64, device=dl.device)
+    run = [c for c in (classes or k_classes())
+           if c[0] + c[2] in dl.kpair and c[:2] in dl.kpart and c[2:] in dl.kpart]
     with torch.cuda.stream(st):
-        for cls in (classes or k_classes()):
-            ac = cls[0] + cls[2]
-            if ac in dl.kpair and cls[:2] in dl.kpart and cls[2:] in dl.kpart:
-                L.exchange_grad(cls, kgrad_args(dl, cls, G, kmap.offsets[ac], G.shape[1], st.cuda_stream, omega))
+        if len(run) == len(set(run)):
+            b = build_call(dl, omega)
+            b.gradient, b.grad_stride = 1, G.shape[1]
+            for key in {c[0] + c[2] for c in run}:
+                b.mat_K[LV[key[0]] * 3 + LV[key[1]]] = G.data_ptr() + 8 * kmap.offsets[key]
+            if L.fock_build(b, [], run, st.cuda_stream):
+                run = []
+        for cls in run:
+            L.exchange_grad(cls, kgrad_args(dl, cls, G, kmap.offsets[cls[0] + cls[2]], G.shape[1], st.cuda_stream,
+                                            omega))
     return G
 
 

@@ -134,3 +134,36 @@ def test_one_call_build_equals_class_calls(atoms, omega, cut):
     for a, b in ((matJ, refJ), (matK, refK)):
         for k in b:
             assert torch.equal(a[k], b[k]), k
+
+
+@pytest.mark.parametrize("prims", [511, 512, 513, 700])
+def test_long_partner_segments(prims):
+    """Partner segments around the length of one tile of the segment sort: an
+    s-only system of `prims` primitives on one list, a few (i, k) rows, the
+    partner lists given in reverse order (the engine sorts them)."""
+    L = lib()
+    L.init(0)
+    atoms = 7
+    wl = basis.config_custom(atoms, 9.0, {0: 1}, 100, 0.02, 1.08, 3, 1e-12, 4)
+    rl = lists.build_lists(wl.mol, wl.D, wl.threshold, fock.gpu_schwarz_fn())
+    n = rl.pd.count[0]
+    keep = np.arange(n) < prims
+    kp = rl.kpartners["ss"]
+    first = np.repeat(np.arange(n), kp.counts.astype(np.int64))
+    m = keep[first] & keep[kp.Dinds.astype(np.int64)]
+    kp.Dinds, kp.Q, kp.pdata, first = kp.Dinds[m], kp.Q[m], kp.pdata[m], first[m]
+    kp.counts = np.bincount(first, minlength=n).astype(np.uint32)
+    kp.displs = np.concatenate([[0], np.cumsum(kp.counts[:-1].astype(np.int64))]).astype(np.uint32)
+    kq = rl.kpairs["ss"]
+    rows = np.flatnonzero(keep[kq.pair_i.astype(np.int64)] & keep[kq.pair_k.astype(np.int64)])[::60000][:4]
+    kq.pair_i, kq.pair_k = kq.pair_i[rows].copy(), kq.pair_k[rows].copy()
+    exp = helpers.oracle_K(rl, "ssss")
+    for name in ("Dinds", "Q", "pdata"):
+        v = getattr(kp, name)
+        setattr(kp, name, np.concatenate([v[d:d + c][::-1] for d, c in zip(kp.displs.astype(np.int64),
+                                                                          kp.counts.astype(np.int64))]))
+    dl = fock.to_device(rl)
+    out = torch.zeros(len(rows), dtype=torch.float64, device="cuda")
+    L.exchange("ssss", fock.exchange_args(dl, "ssss", out, torch.cuda.current_stream().cuda_stream, 0.0))
+    torch.cuda.synchronize()
+    assert int(kp.counts.max()) > 256 and close(out.cpu().numpy(), exp), (out.cpu().numpy(), exp)

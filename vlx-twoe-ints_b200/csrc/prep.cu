@@ -292,7 +292,7 @@ int group_csr(Arena& ar, int na, int nb, int npa, int npb, const uint32_t* displ
         VLXB_CHECK_CUDA(cudaMemsetAsync(table, 0, sizeof(int) * ntab, st));
     }
     if (!ar.measuring()) {
-        k_mark_csr<<<prep_blocks(n_first), PREP_THREADS, 0, st>>>(displs, counts, Dinds, n_first, na, nb, npb, table);
+        k_mark_csr<<<prep_blocks((int64_t)n_first * 32), PREP_THREADS, 0, st>>>(displs, counts, Dinds, n_first, na, nb, npb, table);
     }
     if (!ar.measuring()) note_launches();
     VLXB_CHECK_CUDA(cudaGetLastError());
@@ -302,7 +302,7 @@ int group_csr(Arena& ar, int na, int nb, int npa, int npb, const uint32_t* displ
     rc = alloc_sp(ar, na * nb, g);
     if (rc) return rc;
     if (!ar.measuring()) {
-        k_fill_csr<<<prep_blocks(n_first), PREP_THREADS, 0, st>>>(displs, counts, Dinds, n_first, na, nb, npb, g.spidx,
+        k_fill_csr<<<prep_blocks((int64_t)n_first * 32), PREP_THREADS, 0, st>>>(displs, counts, Dinds, n_first, na, nb, npb, g.spidx,
                                                                   g.entry, g.sp_i, g.sp_j, g.sp_stride);
     }
     ar.release(table);
@@ -393,14 +393,18 @@ int make_records(Arena& ar, int nxy, PairGroups& g, const double* Q, int64_t n_e
     return VLXB_OK;
 }
 
+// Longest segment (records of one first primitive) that k_sort_segments takes:
+// its time grows with the square, 512 x 512 comparisons being about what the
+// thirteen launches of the library sort cost (60 us); at the bound a segment
+// takes 5 ms, of which 148 run at once.
+constexpr int64_t SORT_SEGMENT_MAX = 16384;
+
 int segment_records(Arena& ar, int nxy, int npa, int npb, PairGroups& g, const double* pdata)
 {
     cudaStream_t st = ar.stream();
     const int* recoff = g.seg;
     int* seg = ar.alloc<int>(npa + 1);
     double* q_sorted = ar.alloc<double>(g.rec_stride);
-    int* perm_in = ar.alloc<int>(g.rec_stride);
-    int* perm = ar.alloc<int>(g.rec_stride);
     int32_t* sp_sorted = ar.alloc<int32_t>(g.rec_stride);
     uint64_t* mask_sorted = ar.alloc<uint64_t>(g.rec_stride);
     g.S = ar.alloc<double>(g.sp_stride * nxy);
@@ -410,25 +414,30 @@ int segment_records(Arena& ar, int nxy, int npa, int npb, PairGroups& g, const d
         k_rec_segments<<<prep_blocks(npa + 1), PREP_THREADS, 0, st>>>(g.spidx, recoff, npa, npb, g.n_rec, seg);
     }
     if (!ar.measuring()) note_launches();
-    if (!ar.measuring()) {
-        k_iota<<<prep_blocks(g.rec_stride), PREP_THREADS, 0, st>>>(perm_in, g.rec_stride);
-    }
-    if (!ar.measuring()) note_launches();
-    VLXB_CHECK_CUDA(cudaGetLastError());
-    size_t bytes = 0;
-    VLXB_CHECK_CUDA(cub::DeviceSegmentedRadixSort::SortPairsDescending(
-        nullptr, bytes, g.rec_q, q_sorted, perm_in, perm, (int)g.rec_stride, npa, seg, seg + 1, 0, 64, st));
-    void* tmp = ar.alloc<char>((int64_t)bytes);
-    if (!tmp) return VLXB_ENOMEM;
-    if (!ar.measuring()) {
+    if ((int64_t)npb * nxy <= SORT_SEGMENT_MAX) {
+        if (!ar.measuring()) {
+            k_sort_segments<<<npa, 128, 0, st>>>(seg, npa, g.rec_q, g.rec_sp, g.rec_mask, q_sorted, sp_sorted,
+                                                 mask_sorted);
+            note_launches();
+        }
+    } else {
+        int* perm_in = ar.alloc<int>(g.rec_stride);
+        int* perm = ar.alloc<int>(g.rec_stride);
+        if (ar.failed()) return VLXB_ENOMEM;
+        size_t bytes = 0;
         VLXB_CHECK_CUDA(cub::DeviceSegmentedRadixSort::SortPairsDescending(
-            tmp, bytes, g.rec_q, q_sorted, perm_in, perm, (int)g.rec_stride, npa, seg, seg + 1, 0, 64, st));
+            nullptr, bytes, g.rec_q, q_sorted, perm_in, perm, (int)g.rec_stride, npa, seg, seg + 1, 0, 64, st));
+        void* tmp = ar.alloc<char>((int64_t)bytes);
+        if (!tmp) return VLXB_ENOMEM;
+        if (!ar.measuring()) {
+            k_iota<<<prep_blocks(g.rec_stride), PREP_THREADS, 0, st>>>(perm_in, g.rec_stride);
+            VLXB_CHECK_CUDA(cub::DeviceSegmentedRadixSort::SortPairsDescending(
+                tmp, bytes, g.rec_q, q_sorted, perm_in, perm, (int)g.rec_stride, npa, seg, seg + 1, 0, 64, st));
+            k_gather_recs<<<prep_blocks(g.rec_stride), PREP_THREADS, 0, st>>>(g.n_rec, perm, g.rec_sp, g.rec_mask,
+                                                                               sp_sorted, mask_sorted);
+            note_launches(2);
+        }
     }
-    if (!ar.measuring()) {
-        k_gather_recs<<<prep_blocks(g.rec_stride), PREP_THREADS, 0, st>>>(g.n_rec, perm, g.rec_sp, g.rec_mask,
-                                                                           sp_sorted, mask_sorted);
-    }
-    if (!ar.measuring()) note_launches();
     VLXB_CHECK_CUDA(cudaGetLastError());
     g.rec_q = q_sorted;
     g.rec_sp = sp_sorted;

@@ -12,15 +12,11 @@
 // the same for 170 f classes would multiply the library's size and build
 // time.  The f classes run one generic kernel per kind instead, with the
 // angular momenta as runtime arguments, at the reference's granularity: one
-// Cartesian component quartet per work item, evaluated in
-// McMurchie-Davidson form,
-//   (ab|cd) = S_ab S_cd 2 sqrt(rho'/pi) sum_{tuv} E^ab_t E^ab_u E^ab_v
-//             sum_{t'u'v'} (-1)^{t'+u'+v'} E^cd_t' E^cd_u' E^cd_v' R_{t+t',u+u',v+v'}
-// with the 1-D Hermite coefficients of each pair and the Hermite Coulomb
-// integrals R_{tuv} of the quartet (R^{(n)}_{000} = (-2 rho')^n F_n(rho'|PQ|^2),
-// rho' = rho for the Coulomb operator and rho w^2 / (rho + w^2) for the
-// attenuated one), built inside the component's own box t <= a_x+b_x+c_x+d_x,
-// u <= .., v <= .. .  Screening is the reference's per-component predicate
+// Cartesian component quartet per work item, evaluated by Rys quadrature in
+// registers (eri_component), rho' = rho for the Coulomb operator and
+// rho w^2 / (rho + w^2) for the attenuated one.  Two atoms 1s1p1d1f (170 f class
+// calls): 189 ms with a Hermite box per component in local memory, 39 ms so.
+// Screening is the reference's per-component predicate
 // (|Q_ij Q_kl D_kl| > thr for J, |Q_ij Q_kl max_D| > thr for K), the J ket
 // weights gen_coulomb.py:276-281, the K density gather gen_exchange.py:323.
 // A CTA owns one output entry (J bra entry, K (i, k) entry); its threads
@@ -29,58 +25,14 @@
 // by vlxb_quartetCounters.
 #include "classes.cuh"
 #include "md.cuh"
+#include "rys.cuh"
 
 namespace vlxb {
 
 constexpr int FS_THREADS = 128;
 constexpr int FS_LMAX = 3;                  // f
-constexpr int FS_EMAX = 2 * FS_LMAX + 1;    // 1-D Hermite coefficients per pair and direction
-constexpr int FS_BOX = 125;                 // max (tx+1)(ty+1)(tz+1) for tx+ty+tz <= 12
-
-// F_m(T), m = 0..L (runtime L <= 12), from the FP64 table as boys_f64.
-__device__ void boys_rt(int L, double T, const double* __restrict__ tab, double* F)
-{
-    if (T < BOYS_TMAX) {
-        const int k = __double2int_rn(T * BOYS_INV_H);
-        const double md = (double)k * BOYS_H - T;
-        const double* row = tab + k * BOYS_NCOL + L;
-        double acc = __ldg(row + BOYS_NT - 1);
-        for (int j = BOYS_NT - 1; j >= 1; j--) acc = fma(acc, md * (1.0 / j), __ldg(row + j - 1));
-        F[L] = acc;
-        const double ex = exp(-T);
-        for (int m = L - 1; m >= 0; m--) F[m] = fma(2.0 * T, F[m + 1], ex) / (2.0 * m + 1.0);
-    } else {
-        F[0] = SQRT_PI_4 * sqrt(1.0 / T);
-        const double ex = exp(-T);
-        for (int m = 0; m < L; m++) F[m + 1] = fma(2.0 * m + 1.0, F[m], -ex) * (0.5 / T);
-    }
-}
-
-// 1-D Hermite coefficients E^{ij}_t, t = 0..i+j, of one pair and direction
-// (md.cuh's recurrence with runtime i, j <= 3).
-__device__ void herm1(int i, int j, double PA, double PB, double i2p, double* E)
-{
-    double e[FS_LMAX + 1][FS_LMAX + 1][FS_EMAX];
-    for (int a = 0; a <= i; a++)
-        for (int b = 0; b <= j; b++)
-            for (int t = 0; t < FS_EMAX; t++) e[a][b][t] = 0.0;
-    e[0][0][0] = 1.0;
-    for (int a = 0; a < i; a++)
-        for (int t = 0; t <= a + 1; t++) {
-            double v = (t <= a) ? PA * e[a][0][t] : 0.0;
-            if (t > 0) v = fma(i2p, e[a][0][t - 1], v);
-            if (t + 1 <= a) v = fma((double)(t + 1), e[a][0][t + 1], v);
-            e[a + 1][0][t] = v;
-        }
-    for (int b = 0; b < j; b++)
-        for (int t = 0; t <= i + b + 1; t++) {
-            double v = (t <= i + b) ? PB * e[i][b][t] : 0.0;
-            if (t > 0) v = fma(i2p, e[i][b][t - 1], v);
-            if (t + 1 <= i + b) v = fma((double)(t + 1), e[i][b][t + 1], v);
-            e[i][b + 1][t] = v;
-        }
-    for (int t = 0; t <= i + j; t++) E[t] = e[i][j][t];
-}
+constexpr int FS_N = 2 * FS_LMAX + 1;     // rows and columns of a 1-D table: exponents 0..6 per pair
+constexpr int FS_NR = RYS_MAX;            // roots of an (FF|FF) quartet
 
 struct FPrim {
     double alpha, r[3];
@@ -99,88 +51,114 @@ __device__ __forceinline__ FPrim fprim(const double* __restrict__ info, uint32_t
     f.r[0] = __ldg(info + p + 2 * (int64_t)count);
     f.r[1] = __ldg(info + p + 3 * (int64_t)count);
     f.r[2] = __ldg(info + p + 4 * (int64_t)count);
-    f.c[0] = cart_x(l, comp);
-    f.c[1] = cart_y(l, comp);
-    f.c[2] = l - f.c[0] - f.c[1];
+    const int yz = comp < 1 ? 0 : (comp < 3 ? 1 : (comp < 6 ? 2 : 3));  // y + z exponents (x^l first)
+    f.c[2] = comp - yz * (yz + 1) / 2;
+    f.c[1] = yz - f.c[2];
+    f.c[0] = l - yz;
     return f;
 }
 
-// (ab|cd) / (S_ab S_cd) of one Cartesian component quartet.
-__device__ double eri_component(const FPrim& A, const FPrim& B, const FPrim& C, const FPrim& D, double omega,
-                                const double* __restrict__ tab)
+// Coefficients of the 1-D shift (x, y) = sum_n cf[n] (n, 0):
+// binomial(y, n - x) R^(y - n + x), 0 outside n = x .. x + y (y <= 3).
+__device__ __forceinline__ void fs_shift(int x, int y, double R, double* cf)
+{
+    const double R2 = R * R, R3 = R2 * R;
+#pragma unroll
+    for (int n = 0; n < FS_N; n++) {
+        const int k = n - x, j = y - k;
+        double c = j == 0 ? 1.0 : (j == 1 ? R : (j == 2 ? R2 : R3));
+        if ((y == 3 && (k == 1 || k == 2))) c *= 3.0;
+        else if (y == 2 && k == 1) c *= 2.0;
+        cf[n] = k >= 0 && j >= 0 ? c : 0.0;
+    }
+}
+
+// (ab|cd) / (S_ab S_cd) of one Cartesian component quartet by Rys quadrature:
+// per direction the 2-D integrals (a b; c d) at every root, as the shifts of
+// the recurrence table V(n, m), built column by column in registers (indices of
+// arrays are constants throughout; nab, ncd = la + lb, lc + ld bound the rows,
+// and columns stop at c + d).  About a quarter of the operations of the Hermite
+// box it replaces and no local memory.
+__device__ double eri_component(const FPrim& A, const FPrim& B, const FPrim& C, const FPrim& D, int nab, int ncd,
+                                double omega, const double* __restrict__ rtab)
 {
     const double p = A.alpha + B.alpha, q = C.alpha + D.alpha;
-    double Eab[3][FS_EMAX], Ecd[3][FS_EMAX], PQ[3];
-    int tb[3];
-    for (int x = 0; x < 3; x++) {
-        const double P = (A.alpha * A.r[x] + B.alpha * B.r[x]) / p;
-        const double Q = (C.alpha * C.r[x] + D.alpha * D.r[x]) / q;
-        herm1(A.c[x], B.c[x], P - A.r[x], P - B.r[x], 0.5 / p, Eab[x]);
-        herm1(C.c[x], D.c[x], Q - C.r[x], Q - D.r[x], 0.5 / q, Ecd[x]);
-        PQ[x] = P - Q;
-        tb[x] = A.c[x] + B.c[x] + C.c[x] + D.c[x];
-    }
-    const int L = tb[0] + tb[1] + tb[2];
-    const double rho = p * q / (p + q);
+    const double ip = 1.0 / p, iq = 1.0 / q, inv = 1.0 / (p + q);
+    const double rho = p * q * inv;
     const double d2 = omega != 0.0 ? omega * omega / (rho + omega * omega) : 1.0;
     const double rp = rho * d2;
-    double F[4 * FS_LMAX + 1];
-    boys_rt(L, rp * (PQ[0] * PQ[0] + PQ[1] * PQ[1] + PQ[2] * PQ[2]), tab, F);
-    // R^{(n)}_{tuv} inside the box, levels n = L .. 0 (two buffers)
-    const int nx = tb[0] + 1, ny = tb[1] + 1, nz = tb[2] + 1;
-    double Ra[FS_BOX], Rb[FS_BOX];
-    double* src = Ra;
-    double* dst = Rb;
-    double s = 2.0 * sqrt(rp * INV_PI_D);
-    double base[4 * FS_LMAX + 1];
-    for (int n = 0; n <= L; n++) {
-        base[n] = F[n] * s;
-        s *= -2.0 * rp;
+    double PA[3], QC[3], PQ[3], r2 = 0.0;
+#pragma unroll
+    for (int x = 0; x < 3; x++) {
+        PA[x] = -B.alpha * ip * (A.r[x] - B.r[x]);
+        QC[x] = -D.alpha * iq * (C.r[x] - D.r[x]);
+        PQ[x] = (QC[x] + C.r[x]) - (PA[x] + A.r[x]);
+        r2 = fma(PQ[x], PQ[x], r2);
     }
-    src[0] = base[L];
-    for (int n = L - 1; n >= 0; n--) {
-        const int lev = L - n;  // t + u + v <= lev
-        for (int t = 0; t < nx; t++)
-            for (int u = 0; u < ny; u++)
-                for (int v = 0; v < nz; v++) {
-                    if (t + u + v > lev) continue;
-                    const int o = (t * ny + u) * nz + v;
-                    double val;
-                    if (t > 0) {
-                        val = PQ[0] * src[((t - 1) * ny + u) * nz + v];
-                        if (t > 1) val = fma((double)(t - 1), src[((t - 2) * ny + u) * nz + v], val);
-                    } else if (u > 0) {
-                        val = PQ[1] * src[(u - 1) * nz + v];
-                        if (u > 1) val = fma((double)(u - 1), src[(u - 2) * nz + v], val);
-                    } else if (v > 0) {
-                        val = PQ[2] * src[v - 1];
-                        if (v > 1) val = fma((double)(v - 1), src[v - 2], val);
-                    } else {
-                        val = base[n];
-                    }
-                    dst[o] = val;
+    const int nr = (nab + ncd) / 2 + 1;
+    double x2[FS_NR], prod[FS_NR];
+#pragma unroll
+    for (int r = 0; r < FS_NR; r++) {
+        if (r < nr) {
+            double xr, wr;
+            rys_root_rt(nr, rp * r2, rtab, r, xr, wr);
+            x2[r] = xr * d2;
+            prod[r] = wr;
+        } else {
+            x2[r] = prod[r] = 0.0;
+        }
+    }
+#pragma unroll
+    for (int x = 0; x < 3; x++) {
+        const int mc = C.c[x] + D.c[x];
+        double cb[FS_N], cd[FS_N];
+        fs_shift(A.c[x], B.c[x], A.r[x] - B.r[x], cb);
+        fs_shift(C.c[x], D.c[x], C.r[x] - D.r[x], cd);
+#pragma unroll
+        for (int r = 0; r < FS_NR; r++) {
+            if (r >= nr) break;
+            const double zx = q * inv * x2[r], ex = p * inv * x2[r];
+            const double B10 = 0.5 * ip * (1.0 - zx), B01 = 0.5 * iq * (1.0 - ex), B00 = 0.5 * inv * x2[r];
+            const double Cx = fma(zx, PQ[x], PA[x]), Dx = fma(-ex, PQ[x], QC[x]);
+            double v[FS_N], w[FS_N];  // columns m and m - 1
+            v[0] = 1.0;
+            v[1] = Cx;
+            double s = fma(cb[1], v[1], cb[0]);
+#pragma unroll
+            for (int n = 2; n < FS_N; n++) {
+                v[n] = 0.0;
+                if (n <= nab) {
+                    v[n] = fma(Cx, v[n - 1], (n - 1) * B10 * v[n - 2]);
+                    s = fma(cb[n], v[n], s);
                 }
-        double* tmp = src;
-        src = dst;
-        dst = tmp;
-    }
-    // src holds R^{(0)}; contract with the bra and (signed) ket coefficients
-    double sum = 0.0;
-    for (int t = 0; t <= A.c[0] + B.c[0]; t++)
-        for (int u = 0; u <= A.c[1] + B.c[1]; u++)
-            for (int v = 0; v <= A.c[2] + B.c[2]; v++) {
-                const double eb = Eab[0][t] * Eab[1][u] * Eab[2][v];
-                double k = 0.0;
-                for (int t2 = 0; t2 <= C.c[0] + D.c[0]; t2++)
-                    for (int u2 = 0; u2 <= C.c[1] + D.c[1]; u2++)
-                        for (int v2 = 0; v2 <= C.c[2] + D.c[2]; v2++) {
-                            const double ek = Ecd[0][t2] * Ecd[1][u2] * Ecd[2][v2];
-                            const double r = src[((t + t2) * ny + (u + u2)) * nz + (v + v2)];
-                            k = fma(((t2 + u2 + v2) & 1) ? -ek : ek, r, k);
-                        }
-                sum = fma(eb, k, sum);
             }
-    return sum;
+#pragma unroll
+            for (int n = 0; n < FS_N; n++) w[n] = 0.0;
+            double sum = cd[0] * s;
+#pragma unroll
+            for (int m = 1; m < FS_N; m++) {
+                if (m > mc) break;
+                double prev = 0.0;  // v[n - 1] of the column before this one
+                s = 0.0;
+#pragma unroll
+                for (int n = 0; n < FS_N; n++) {
+                    if (n > nab) break;
+                    const double t = fma(Dx, v[n], fma((m - 1) * B01, w[n], n * B00 * prev));
+                    prev = v[n];
+                    w[n] = v[n];
+                    v[n] = t;
+                    s = fma(cb[n], t, s);
+                }
+                sum = fma(cd[m], s, sum);
+            }
+            prod[r] *= sum;
+        }
+    }
+    double sum = 0.0;
+#pragma unroll
+    for (int r = 0; r < FS_NR; r++)
+        if (r < nr) sum += prod[r];
+    return 2.0 * sqrt(rp * INV_PI_D) * sum;
 }
 
 __device__ __forceinline__ double fs_block_sum(double v, double* red)
@@ -226,7 +204,7 @@ coulomb_fshell_kernel(FShellJ a, double* __restrict__ mat_J, const double* __res
             const FPrim C = fprim(a.info[a.lc], a.count[a.lc], a.lc, k);
             const FPrim D = fprim(a.info[a.ld], a.count[a.ld], a.ld, l);
             const double w = (a.lc != a.ld || k != l) ? 2.0 : 1.0;
-            acc = fma(__ldg(a.cd_pdata + kl) * eri_component(A, B, C, D, 0.0, tab), dkl * w, acc);
+            acc = fma(__ldg(a.cd_pdata + kl) * eri_component(A, B, C, D, a.la + a.lb, a.lc + a.ld, 0.0, tab), dkl * w, acc);
         }
         const double s = fs_block_sum(acc, red);
         if (threadIdx.x == 0) mat_J[ij] += __ldg(a.ab_pdata + ij) * s;
@@ -270,7 +248,7 @@ exchange_fshell_kernel(FShellK a, double* __restrict__ mat_K, const double* __re
             const FPrim D = fprim(a.info[a.ld], a.count[a.ld], a.ld, lp);
             const uint32_t jao = __ldg(a.aoinds[a.lb] + jp / (uint32_t)ncb + (int64_t)a.count[a.lb] * (jp % ncb));
             const uint32_t lao = __ldg(a.aoinds[a.ld] + lp / (uint32_t)ncd + (int64_t)a.count[a.ld] * (lp % ncd));
-            const double eri = __ldg(a.pdata_ab + pj) * __ldg(a.pdata_cd + pl) * eri_component(A, B, C, D, a.omega, tab);
+            const double eri = __ldg(a.pdata_ab + pj) * __ldg(a.pdata_cd + pl) * eri_component(A, B, C, D, a.la + a.lb, a.lc + a.ld, a.omega, tab);
             acc = fma(eri, __ldg(a.D + (int64_t)jao * a.naos + lao), acc);
         }
         const double s = fs_block_sum(acc, red);
@@ -293,7 +271,7 @@ schwarz_fshell_kernel(int la, int lb, const double* __restrict__ info_a, uint32_
             for (int cb = 0; cb < nb; cb++) {
                 const FPrim A = fprim(info_a, cnt_a, la, P[t] * (uint32_t)na + ca);
                 const FPrim B = fprim(info_b, cnt_b, lb, Q[t] * (uint32_t)nb + cb);
-                m = fmax(m, fabs(eri_component(A, B, A, B, 0.0, tab)));
+                m = fmax(m, fabs(eri_component(A, B, A, B, la + lb, la + lb, 0.0, tab)));
             }
         out[t] = sqrt(m);
     }
@@ -324,7 +302,7 @@ shell_pair_fshell_kernel(int la, int lb, const double* __restrict__ info_a, uint
             for (int cb = 0; cb < nb; cb++) {
                 const FPrim A = fprim(info_a, cnt_a, la, i * (uint32_t)na + ca);
                 const FPrim B = fprim(info_b, cnt_b, lb, j * (uint32_t)nb + cb);
-                m = fmax(m, fabs(eri_component(A, B, A, B, 0.0, tab)));
+                m = fmax(m, fabs(eri_component(A, B, A, B, la + lb, la + lb, 0.0, tab)));
             }
         S_out[t] = S;
         q_out[t] = fabs(S) * sqrt(m);
@@ -335,7 +313,7 @@ int run_shell_pair_f(int la, int lb, const double* info_a, uint32_t cnt_a, const
                      const uint32_t* P, const uint32_t* Q, uint32_t n, double* S_out, double* q_out,
                      cudaStream_t st)
 {
-    const double* tab = boys_table_device();
+    const double* tab = rys_table_device();
     if (!tab) return VLXB_ECUDA;
     const uint32_t want = (n + FS_THREADS - 1) / FS_THREADS;
     const int grid = (int)(want < 148u * 64u ? want : 148u * 64u);
@@ -349,7 +327,7 @@ int run_shell_pair_f(int la, int lb, const double* info_a, uint32_t cnt_a, const
 int run_schwarz_f(int la, int lb, const double* info_a, uint32_t cnt_a, const double* info_b, uint32_t cnt_b,
                   const uint32_t* P, const uint32_t* Q, uint32_t n, double* out, cudaStream_t st)
 {
-    const double* tab = boys_table_device();
+    const double* tab = rys_table_device();
     if (!tab) return VLXB_ECUDA;
     const uint32_t want = (n + FS_THREADS - 1) / FS_THREADS;
     const int grid = (int)(want < 148u * 64u ? want : 148u * 64u);
@@ -369,7 +347,7 @@ int run_coulomb_f(int la, int lb, int lc, int ld, const CoulombArgs& a, cudaStre
     for (int t = 0; t < 4; t++)
         if (L4[t] < 0 || L4[t] > FS_LMAX || !a.info[L4[t]] || a.count[L4[t]] == 0) return VLXB_EINVAL;
     if (!(a.thr >= 0.0)) return VLXB_EINVAL;
-    const double* tab = boys_table_device();
+    const double* tab = rys_table_device();
     if (!tab) return VLXB_ECUDA;
     FShellJ f{la, lb, lc, ld, {a.info[0], a.info[1], a.info[2], a.info[3]},
               {a.count[0], a.count[1], a.count[2], a.count[3]}, a.cd_D, a.ab_Q, a.cd_Q, a.ab_first, a.ab_second,
@@ -393,7 +371,7 @@ int run_exchange_f(int la, int lb, int lc, int ld, const ExchangeArgs& a, cudaSt
         if (L4[t] < 0 || L4[t] > FS_LMAX || !a.info[L4[t]] || !a.aoinds[L4[t]] || a.count[L4[t]] == 0)
             return VLXB_EINVAL;
     if (!(a.thr >= 0.0) || !(a.omega >= 0.0)) return VLXB_EINVAL;
-    const double* tab = boys_table_device();
+    const double* tab = rys_table_device();
     if (!tab) return VLXB_ECUDA;
     FShellK f{la, lb, lc, ld, a.pair_i, a.pair_k, a.n_ik, {a.info[0], a.info[1], a.info[2], a.info[3]},
               {a.aoinds[0], a.aoinds[1], a.aoinds[2], a.aoinds[3]}, {a.count[0], a.count[1], a.count[2], a.count[3]},

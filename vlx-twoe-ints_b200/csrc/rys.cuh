@@ -60,4 +60,19 @@ __device__ __forceinline__ void rys_root(double T, const double* __restrict__ ta
     }
 }
 
+// The same for an order known at run time; tab = rys_table_device().
+__device__ __forceinline__ void rys_root_rt(int nr, double T, const double* __restrict__ tab, int r, double& x,
+                                            double& w)
+{
+    switch (nr) {
+        case 1: rys_root<1>(T, tab + rys_offset(1), r, x, w); break;
+        case 2: rys_root<2>(T, tab + rys_offset(2), r, x, w); break;
+        case 3: rys_root<3>(T, tab + rys_offset(3), r, x, w); break;
+        case 4: rys_root<4>(T, tab + rys_offset(4), r, x, w); break;
+        case 5: rys_root<5>(T, tab + rys_offset(5), r, x, w); break;
+        case 6: rys_root<6>(T, tab + rys_offset(6), r, x, w); break;
+        default: rys_root<7>(T, tab + rys_offset(7), r, x, w); break;
+    }
+}
+
 }  // namespace vlxb

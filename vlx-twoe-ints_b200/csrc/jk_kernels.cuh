@@ -355,12 +355,31 @@ __device__ __forceinline__ void k_chunk_scan(const double* __restrict__ aq, cons
         k_prefixes(__ldg(aq + jb + t), aqa ? __ldg(aqa + jb + t) : 0.0, cq, aqa ? cqpre : nullptr, c0, c1, maxD, thr,
                    fp32_cut, njtot, budget, s.nl[t], s.n64[t]);
     __syncthreads();
-    if (threadIdx.x == 0) {
-        s.c64[0] = 0;
-        s.c32[0] = 0;
-        for (int t = 0; t < nj; t++) {
-            s.c64[t + 1] = s.c64[t] + s.n64[t];
-            s.c32[t + 1] = s.c32[t] + (s.nl[t] - s.n64[t]);
+    // both exclusive scans by one warp (a single thread took 3k cycles of a
+    // block's 20k for 96 s primitives)
+    if (threadIdx.x < 32) {
+        int b64 = 0, b32 = 0;
+        for (int t0 = 0; t0 < nj; t0 += 32) {
+            const int t = t0 + threadIdx.x;
+            int v64 = t < nj ? s.n64[t] : 0, v32 = t < nj ? s.nl[t] - s.n64[t] : 0;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int u64 = __shfl_up_sync(0xffffffffu, v64, o), u32 = __shfl_up_sync(0xffffffffu, v32, o);
+                if (threadIdx.x >= o) {
+                    v64 += u64;
+                    v32 += u32;
+                }
+            }
+            if (t < nj) {
+                s.c64[t + 1] = b64 + v64;
+                s.c32[t + 1] = b32 + v32;
+            }
+            b64 += __shfl_sync(0xffffffffu, v64, 31);
+            b32 += __shfl_sync(0xffffffffu, v32, 31);
+        }
+        if (threadIdx.x == 0) {
+            s.c64[0] = 0;
+            s.c32[0] = 0;
         }
     }
     __syncthreads();
@@ -484,13 +503,15 @@ exchange_kernel(KOutBlocks out, KPartnerRecs ab, KPartnerRecs cd, KDensity dm, d
             const int t64 = s_c64[nj], t32 = s_c32[nj];
             if (qcount && PM == 0 && threadIdx.x == 0) atomicAdd(qcount, (unsigned long long)(t64 + t32));
             if (PM == 0) {
+                int jj = 0;
                 for (int w = threadIdx.x; w < t64; w += K_THREADS) {
-                    const int jj = k_find(s_c64, nj, w);
+                    while (s_c64[jj + 1] <= w) jj++;  // w ascends; s_c64[nj] = t64 > w
                     k_quartet<LA, LB, LC, LD, double>(ab, cd, jb + jj, c0 + (w - s_c64[jj]), dm, omega, tabs, Kacc);
                 }
             } else {
+                int jj = 0;
                 for (int w = threadIdx.x; w < t32; w += K_THREADS) {
-                    const int jj = k_find(s_c32, nj, w);
+                    while (s_c32[jj + 1] <= w) jj++;
                     k_quartet<LA, LB, LC, LD, float>(ab, cd, jb + jj, c0 + s_n64[jj] + (w - s_c32[jj]), dm, omega,
                                                      tabs, Kacc);
                 }

@@ -23,10 +23,11 @@ enum Status : int {
         if (_e != cudaSuccess) return (_e == cudaErrorMemoryAllocation) ? VLXB_ENOMEM : VLXB_ECUDA; \
     } while (0)
 
-// Scratch arena of one call.  Pool mode (default): every buffer is taken
-// from the device's default memory pool with cudaMallocAsync on the call's
-// stream and handed back with cudaFreeAsync when the arena goes out of scope,
-// so scratch is reused across calls without synchronisation.  Static mode:
+// Scratch arena of one call.  Pool mode (default): buffers, or slabs that hold
+// the small ones, are taken from the device's default memory pool with
+// cudaMallocAsync on the call's stream and handed back with cudaFreeAsync when
+// the arena goes out of scope, so scratch is reused across calls without
+// synchronisation.  Static mode:
 // buffers are carved (256-byte aligned) out of a fixed device buffer given by
 // the caller, nothing is allocated.  Measure mode: nothing is allocated or
 // launched; alloc only adds up the bytes a static-mode call would need (the
@@ -40,6 +41,7 @@ class Arena {
     ~Arena()
     {
         for (void* p : ptrs_) cudaFreeAsync(p, stream_);
+        for (void* p : slabs_) cudaFreeAsync(p, stream_);
     }
     Arena(const Arena&) = delete;
     Arena& operator=(const Arena&) = delete;
@@ -59,19 +61,26 @@ class Arena {
             }
             return (T*)(base_ + off);
         }
-        void* p = nullptr;
-        if (cudaMallocAsync(&p, bytes, stream_) != cudaSuccess) {
-            failed_ = true;
-            cudaGetLastError();
-            return nullptr;
+        // small buffers are cut from slabs: an allocation call costs the host
+        // about a microsecond and a build needs some six hundred of them
+        if (bytes <= SLAB / 8) {
+            const size_t off = (slab_used_ + 255) & ~(size_t)255;
+            if (!slab_ || off + bytes > SLAB) {
+                slab_ = (char*)take(SLAB, slabs_);
+                if (!slab_) return nullptr;
+                slab_used_ = bytes;
+                return (T*)slab_;
+            }
+            slab_used_ = off + bytes;
+            return (T*)(slab_ + off);
         }
-        ptrs_.push_back(p);
-        return (T*)p;
+        return (T*)take(bytes, ptrs_);
     }
-    // Hand one buffer back before the arena ends (pool mode; stream-ordered).
+    // Hand one buffer back before the arena ends (pool mode, stream-ordered; a
+    // buffer cut from a slab stays until then).
     void release(void* p)
     {
-        for (size_t k = ptrs_.size(); k-- > 0;)
+        for (size_t k = ptrs_.size(); k-- > 0;)  // never a slab, whose first buffer has its address
             if (ptrs_[k] == p) {
                 cudaFreeAsync(p, stream_);
                 ptrs_[k] = ptrs_.back();
@@ -85,8 +94,22 @@ class Arena {
     cudaStream_t stream() const { return stream_; }
 
   private:
+    static constexpr size_t SLAB = 4u << 20;
+    void* take(size_t bytes, std::vector<void*>& owner)
+    {
+        void* p = nullptr;
+        if (cudaMallocAsync(&p, bytes, stream_) != cudaSuccess) {
+            failed_ = true;
+            cudaGetLastError();
+            return nullptr;
+        }
+        owner.push_back(p);
+        return p;
+    }
     cudaStream_t stream_;
-    std::vector<void*> ptrs_;
+    std::vector<void*> ptrs_, slabs_;  // own buffers, slabs
+    char* slab_ = nullptr;
+    size_t slab_used_ = 0;
     char* base_ = nullptr;
     size_t cap_ = 0, used_ = 0;
     bool static_ = false, measure_ = false;

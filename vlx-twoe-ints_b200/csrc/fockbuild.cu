@@ -3,6 +3,8 @@
 // integral kernel; the 90 classes of a build do that 225 times for only 27
 // distinct lists.  Here every list is prepared once: two atoms 4s3p2d, 4735
 // device operations and 25.5 ms per build become about 700 and 4.0 ms.
+#include <mutex>
+
 #include "classes.cuh"
 #include "../../include/vlxb.h"
 
@@ -11,7 +13,91 @@ namespace vlxb {
 int dispatch_coulomb(int cls, bool grad, const CoulombArgs& a, int64_t gstride, cudaStream_t st);
 int dispatch_exchange(int cls, bool grad, const ExchangeArgs& a, int64_t gstride, cudaStream_t st);
 
-static int run_build(const VlxbFockBuild& b, PrepShare& share, cudaStream_t st)
+// Class kernels of a small build leave most of the device idle, so those of
+// different output lists (which share no output) run on four streams between
+// a fork and a join on the caller's stream; the classes of one list keep their
+// order and their stream, so results do not depend on it.
+constexpr int FORK_STREAMS = 4;
+// Builds of at most this many output entries fork.  Larger ones fill the
+// device with single kernels.
+constexpr uint64_t FORK_ENTRIES = 400000;
+
+// Streams of the current device (never captured: a capturing call does not
+// fork, so that calls of other threads may use them meanwhile).
+static cudaStream_t* fork_streams()
+{
+    static std::mutex mu;
+    static cudaStream_t pool[64][FORK_STREAMS];
+    static bool made[64] = {false};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
+    std::lock_guard<std::mutex> lk(mu);
+    if (!made[dev]) {
+        for (int k = 0; k < FORK_STREAMS; k++)
+            if (cudaStreamCreateWithFlags(&pool[dev][k], cudaStreamNonBlocking) != cudaSuccess) return nullptr;
+        made[dev] = true;
+    }
+    return pool[dev];
+}
+
+// Streams of the output lists of one build: group g runs on at(g).
+class Fork {
+  public:
+    Fork(const VlxbFockBuild& b, cudaStream_t st) : st_(st)
+    {
+        uint64_t entries = 0;
+        for (int p = 0; p < 9; p++) entries += (uint64_t)b.j_count[p] + b.k_count[p];
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        if (entries > FORK_ENTRIES || cudaStreamIsCapturing(st, &cap) != cudaSuccess ||
+            cap != cudaStreamCaptureStatusNone)
+            return;
+        pool_ = fork_streams();
+        if (!pool_ || cudaEventCreateWithFlags(&start_, cudaEventDisableTiming) != cudaSuccess ||
+            cudaEventRecord(start_, st) != cudaSuccess)
+            pool_ = nullptr;
+    }
+    cudaStream_t at(int g)
+    {
+        if (!pool_) return st_;
+        const int k = g % FORK_STREAMS;
+        if (!used_[k]) {
+            if (cudaStreamWaitEvent(pool_[k], start_, 0) != cudaSuccess) return st_;
+            used_[k] = true;
+        }
+        return pool_[k];
+    }
+    // The caller's stream continues after every forked kernel.
+    int join()
+    {
+        int rc = VLXB_OK;
+        for (int k = 0; k < FORK_STREAMS; k++)
+            if (used_[k]) {
+                cudaEvent_t e = nullptr;
+                if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess ||
+                    cudaEventRecord(e, pool_[k]) != cudaSuccess || cudaStreamWaitEvent(st_, e, 0) != cudaSuccess) {
+                    // never leave work behind that the caller's stream does not wait for
+                    cudaStreamSynchronize(pool_[k]);
+                    rc = VLXB_ECUDA;
+                }
+                if (e) cudaEventDestroy(e);
+                used_[k] = false;
+            }
+        return rc;
+    }
+    ~Fork()
+    {
+        join();
+        if (start_) cudaEventDestroy(start_);
+    }
+
+  private:
+    cudaStream_t st_;
+    cudaStream_t* pool_ = nullptr;
+    cudaEvent_t start_ = nullptr;
+    bool used_[FORK_STREAMS] = {};
+};
+
+static int run_build(const VlxbFockBuild& b, PrepShare& share, Fork* fork, cudaStream_t stream)
 {
     static const int pair_ab[6][2] = {{0, 0}, {0, 1}, {0, 2}, {1, 1}, {1, 2}, {2, 2}};
     const bool batched = b.n_mol > 0;
@@ -19,6 +105,7 @@ static int run_build(const VlxbFockBuild& b, PrepShare& share, cudaStream_t st)
     for (int x = 0; x < 6; x++)
         for (int y = 0; y < 6; y++, bit++) {
             if (!((b.j_classes >> bit) & 1ull)) continue;
+            const cudaStream_t st = fork ? fork->at(x) : stream;
             const int la = pair_ab[x][0], lb = pair_ab[x][1], lc = pair_ab[y][0], ld = pair_ab[y][1];
             const int p = la * 3 + lb, q = lc * 3 + ld;
             CoulombArgs A{};
@@ -46,6 +133,7 @@ static int run_build(const VlxbFockBuild& b, PrepShare& share, cudaStream_t st)
     for (int x = 0; x < 6; x++)
         for (int bd = 0; bd < 9; bd++, bit++) {
             if (!((b.k_classes >> bit) & 1ull)) continue;
+            const cudaStream_t st = fork ? fork->at(x + 2) : stream;
             const int la = pair_ab[x][0], lc = pair_ab[x][1], lb = bd / 3, ld = bd % 3;
             const int o = la * 3 + lc, p = la * 3 + lb, q = lc * 3 + ld;
             ExchangeArgs A{};
@@ -86,10 +174,14 @@ static int run_build(const VlxbFockBuild& b, PrepShare& share, cudaStream_t st)
 extern "C" int vlxb_fockBuild(const VlxbFockBuild* b, void* stream)
 {
     if (!b || b->n_mol < 0 || b->grad_stride > (uint64_t)INT64_MAX || (b->gradient && b->n_mol > 0)) return VLXB_EINVAL;
-    vlxb::PrepShare share((cudaStream_t)stream);
+    const cudaStream_t st = (cudaStream_t)stream;
+    vlxb::PrepShare share(st);
     share.prepare_only = true;  // every list first: a call short of memory then leaves the outputs as they were
-    int rc = vlxb::run_build(*b, share, (cudaStream_t)stream);
+    int rc = vlxb::run_build(*b, share, nullptr, st);
     if (rc) return rc;
     share.prepare_only = false;
-    return vlxb::run_build(*b, share, (cudaStream_t)stream);
+    vlxb::Fork fork(*b, st);  // joined before the preparations are handed back on `st`
+    rc = vlxb::run_build(*b, share, &fork, st);
+    const int jc = fork.join();
+    return rc ? rc : jc;
 }

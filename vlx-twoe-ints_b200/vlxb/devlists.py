@@ -49,6 +49,13 @@ def _shell_pairs(L, dl, la, lb, s):
     return P, Q, S, q
 
 
+def _take(mask, *arrays):
+    """The masked entries of each array: the positions are found once (each
+    boolean index would look for them again and wait for the device)."""
+    idx = mask.nonzero().squeeze(1)
+    return tuple(a[idx] for a in arrays)
+
+
 def _expand(P, Q, S, q, la, lb, upper):
     """Shell pairs -> prim-cart pairs (lists._expand on the device)."""
     na, nb = NCART[la], NCART[lb]
@@ -60,8 +67,7 @@ def _expand(P, Q, S, q, la, lb, upper):
     Sx = S.repeat_interleave(na * nb)
     qx = q.repeat_interleave(na * nb)
     if upper:
-        m = i <= j
-        i, j, Sx, qx = i[m], j[m], Sx[m], qx[m]
+        return _take(i <= j, i, j, Sx, qx)
     return i, j, Sx, qx
 
 
@@ -98,17 +104,18 @@ def build_device_lists(mol, D_AO, threshold: float, device="cuda") -> DeviceList
         for lb in ls:
             if la <= lb:
                 sp[(la, lb)] = _shell_pairs(L, dl, la, lb, s)
-    qmax = max(float(v[3].max()) for v in sp.values() if v[3].numel())
-    dmax = float(dl.D_AO.abs().max())
     bmax = {b + d: _block_max(L, dl, dl.D_AO, LV[b], LV[d], s) for b in ANG for d in ANG
             if LV[b] in ls and LV[d] in ls}
-    dl.maxD = {k: float(v) for k, v in bmax.items()}
+    bounds = torch.cat([torch.stack([v[3].max() for v in sp.values() if v[3].numel()]).max().reshape(1),
+                        dl.D_AO.abs().max().reshape(1)] + list(bmax.values())).tolist()  # one read-back
+    qmax, dmax = bounds[:2]
+    dl.maxD = dict(zip(bmax, bounds[2:]))
 
     # J lists: pairs that can pass with the largest partner, prim-cart pairs
     # (i <= j for same-type lists), sorted by descending |Q D| (stable)
     for (la, lb), (P, Q, S, q) in sp.items():
         keep = q * qmax * dmax > threshold
-        i, j, Sx, qx = _expand(P[keep], Q[keep], S[keep], q[keep], la, lb, upper=(la == lb))
+        i, j, Sx, qx = _expand(*_take(keep, P, Q, S, q), la, lb, upper=(la == lb))
         i32, j32 = _u32(i), _u32(j)
         Dv = torch.empty(i.numel(), dtype=torch.float64, device=dev)
         _gather_D(L, dl, dl.D_AO, la, lb, i32, j32, Dv, s)
@@ -123,13 +130,13 @@ def build_device_lists(mol, D_AO, threshold: float, device="cuda") -> DeviceList
             if la <= lb:
                 P, Q, S, q = sp[(la, lb)]
                 if la == lb:  # add the mirrored pairs P > Q
-                    off = P != Q
-                    P, Q = torch.cat([P, Q[off]]), torch.cat([Q, P[off]])
-                    S, q = torch.cat([S, S[off]]), torch.cat([q, q[off]])
+                    P1, Q1, S1, q1 = _take(P != Q, P, Q, S, q)
+                    P, Q = torch.cat([P, Q1]), torch.cat([Q, P1])
+                    S, q = torch.cat([S, S1]), torch.cat([q, q1])
             else:
                 Q, P, S, q = sp[(lb, la)]
             keep = q * qmax * dmax > threshold
-            i, j, Sx, qx = _expand(P[keep], Q[keep], S[keep], q[keep], la, lb, upper=False)
+            i, j, Sx, qx = _expand(*_take(keep, P, Q, S, q), la, lb, upper=False)
             o1 = torch.sort(qx, descending=True, stable=True).indices
             o2 = torch.sort(i[o1], stable=True).indices
             order = o1[o2]
@@ -148,20 +155,18 @@ def build_device_lists(mol, D_AO, threshold: float, device="cuda") -> DeviceList
         best = torch.zeros(dl.count[la] * NCART[la], dtype=torch.float64, device=dev)
         for lb in ls:
             kp = dl.kpart[ANG[la] + ANG[lb]]
-            has = kp["counts"] > 0
-            first_q = torch.zeros_like(best)
             if kp["Q"].numel():
-                first_q[has] = kp["Q"][kp["displs"][has].long()]
-            best = torch.maximum(best, first_q)
+                first_q = kp["Q"][kp["displs"].long().clamp(max=kp["Q"].numel() - 1)]
+                best = torch.maximum(best, torch.where(kp["counts"] > 0, first_q, 0.0))
         qpart[la] = best
     for la in ls:
         for lc in ls:
             if la > lc:
                 continue
-            ii, kk = torch.nonzero(qpart[la][:, None] * qpart[lc][None, :] * dmax > threshold, as_tuple=True)
+            passing = qpart[la][:, None] * qpart[lc][None, :] * dmax > threshold
             if la == lc:
-                m = ii <= kk
-                ii, kk = ii[m], kk[m]
+                passing = passing.triu()
+            ii, kk = torch.nonzero(passing, as_tuple=True)
             dl.kpair[ANG[la] + ANG[lc]] = {"i": _u32(ii), "k": _u32(kk)}
     return dl
 

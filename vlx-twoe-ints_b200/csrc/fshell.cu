@@ -30,6 +30,7 @@
 namespace vlxb {
 
 constexpr int FS_THREADS = 128;
+constexpr int FS_WIDE = 512;                // threads per entry of lists too short to fill the device
 constexpr int FS_LMAX = 3;                  // f
 constexpr int FS_N = 2 * FS_LMAX + 1;     // rows and columns of a 1-D table: exponents 0..6 per pair
 constexpr int FS_NR = RYS_MAX;            // roots of an (FF|FF) quartet
@@ -169,7 +170,7 @@ __device__ __forceinline__ double fs_block_sum(double v, double* red)
     __syncthreads();
     double s = 0.0;
     if (threadIdx.x == 0)
-        for (int w = 0; w < FS_THREADS / 32; w++) s += red[w];
+        for (int w = 0; w < (int)(blockDim.x >> 5); w++) s += red[w];
     __syncthreads();
     return s;
 }
@@ -188,16 +189,19 @@ struct FShellJ {
     double thr;
 };
 
-__global__ void __launch_bounds__(FS_THREADS)
+// 128 registers: four blocks of 128 threads per SM or one of 512.  The spills
+// they cost (300 bytes) are repaid by the warps: 170 f class calls of two atoms
+// 1s1p1d1f, 239 registers 43.5 ms, 168 35.5, 128 31.2.
+__global__ void __launch_bounds__(FS_WIDE, 1)
 coulomb_fshell_kernel(FShellJ a, double* __restrict__ mat_J, const double* __restrict__ tab)
 {
-    __shared__ double red[FS_THREADS / 32];
+    __shared__ double red[FS_WIDE / 32];
     for (uint32_t ij = blockIdx.x; ij < a.n_ab; ij += gridDim.x) {
         const FPrim A = fprim(a.info[a.la], a.count[a.la], a.la, __ldg(a.ab_first + ij));
         const FPrim B = fprim(a.info[a.lb], a.count[a.lb], a.lb, __ldg(a.ab_second + ij));
         const double qij = __ldg(a.ab_Q + ij);
         double acc = 0.0;
-        for (uint32_t kl = threadIdx.x; kl < a.n_cd; kl += FS_THREADS) {
+        for (uint32_t kl = threadIdx.x; kl < a.n_cd; kl += blockDim.x) {
             const double dkl = __ldg(a.cd_D + kl);
             if (fabs(qij * __ldg(a.cd_Q + kl) * dkl) <= a.thr) continue;
             const uint32_t k = __ldg(a.cd_first + kl), l = __ldg(a.cd_second + kl);
@@ -227,10 +231,10 @@ struct FShellK {
     double omega, thr;
 };
 
-__global__ void __launch_bounds__(FS_THREADS)
+__global__ void __launch_bounds__(FS_WIDE, 1)
 exchange_fshell_kernel(FShellK a, double* __restrict__ mat_K, const double* __restrict__ tab)
 {
-    __shared__ double red[FS_THREADS / 32];
+    __shared__ double red[FS_WIDE / 32];
     const int ncb = ncart(a.lb), ncd = ncart(a.ld);
     for (uint32_t ik = blockIdx.x; ik < a.n_ik; ik += gridDim.x) {
         const uint32_t i = __ldg(a.pair_i + ik), k = __ldg(a.pair_k + ik);
@@ -240,7 +244,7 @@ exchange_fshell_kernel(FShellK a, double* __restrict__ mat_K, const double* __re
         const uint32_t l0 = __ldg(a.displs_cd + k), nl = __ldg(a.counts_cd + k);
         const uint64_t npair = (uint64_t)nj * nl;
         double acc = 0.0;
-        for (uint64_t w = threadIdx.x; w < npair; w += FS_THREADS) {
+        for (uint64_t w = threadIdx.x; w < npair; w += blockDim.x) {
             const uint32_t pj = j0 + (uint32_t)(w / nl), pl = l0 + (uint32_t)(w % nl);
             if (fabs(__ldg(a.Q_ab + pj) * __ldg(a.Q_cd + pl) * a.maxD) <= a.thr) continue;
             const uint32_t jp = __ldg(a.Dinds_ab + pj), lp = __ldg(a.Dinds_cd + pl);
@@ -337,6 +341,10 @@ int run_schwarz_f(int la, int lb, const double* info_a, uint32_t cnt_a, const do
     return VLXB_OK;
 }
 
+// Threads per output entry: with fewer entries than four blocks per SM the
+// entry's partners are spread wider instead.
+static int fs_threads(uint32_t entries) { return entries < 148u * 4u ? FS_WIDE : FS_THREADS; }
+
 int run_coulomb_f(int la, int lb, int lc, int ld, const CoulombArgs& a, cudaStream_t st)
 {
     if (a.n_ab == 0 || a.n_cd == 0) return VLXB_OK;
@@ -354,7 +362,7 @@ int run_coulomb_f(int la, int lb, int lc, int ld, const CoulombArgs& a, cudaStre
               a.ab_pdata, a.n_ab, a.cd_first, a.cd_second, a.cd_pdata, a.n_cd, a.thr};
     int grid = launch_grid_limit();
     if ((int64_t)grid > (int64_t)a.n_ab) grid = (int)a.n_ab;
-    coulomb_fshell_kernel<<<grid, FS_THREADS, 0, st>>>(f, a.mat_J, tab);
+    coulomb_fshell_kernel<<<grid, fs_threads(a.n_ab), 0, st>>>(f, a.mat_J, tab);
     note_launches();
     VLXB_CHECK_CUDA(cudaGetLastError());
     return VLXB_OK;
@@ -379,7 +387,7 @@ int run_exchange_f(int la, int lb, int lc, int ld, const ExchangeArgs& a, cudaSt
               a.counts_cd, a.pdata_ab, a.pdata_cd, a.omega, a.thr};
     int grid = launch_grid_limit();
     if ((int64_t)grid > (int64_t)a.n_ik) grid = (int)a.n_ik;
-    exchange_fshell_kernel<<<grid, FS_THREADS, 0, st>>>(f, a.mat_K, tab);
+    exchange_fshell_kernel<<<grid, fs_threads(a.n_ik), 0, st>>>(f, a.mat_K, tab);
     note_launches();
     VLXB_CHECK_CUDA(cudaGetLastError());
     return VLXB_OK;

@@ -215,11 +215,40 @@ def build_jk(dl: DeviceLists, stream: torch.cuda.Stream | None = None, omega: fl
             if L.fock_build(b, spd[0], spd[1], s):
                 jcls = [c for c in jcls if "f" in c]
                 kcls = [c for c in kcls if "f" in c]
+        at, join = _fork(dl, stream, len(jcls) + len(kcls))
         for cls in jcls:
-            L.coulomb(cls, coulomb_args(dl, cls, matJ[cls[:2]], s))
+            L.coulomb(cls, coulomb_args(dl, cls, matJ[cls[:2]], at("J" + cls[:2])))
         for cls in kcls:
-            L.exchange(cls, exchange_args(dl, cls, matK[cls[0] + cls[2]], s, omega))
+            L.exchange(cls, exchange_args(dl, cls, matK[cls[0] + cls[2]], at("K" + cls[0] + cls[2]), omega))
+        join()
     return matJ, matK
+
+
+FORK_ENTRIES = 400000  # vlxb_fockBuild's bound: larger builds fill the device with single kernels
+
+
+def _fork(dl: DeviceLists, stream: torch.cuda.Stream, calls: int):
+    """(at, join): at(list) is the stream (handle) for the class calls that
+    write one output list, four side streams in turn for small builds, else
+    `stream`; join() makes `stream` wait for them.  The calls of one list keep
+    their order; nothing is forked while a graph is captured."""
+    entries = sum(v["first"].numel() for v in dl.j.values()) + sum(v["i"].numel() for v in dl.kpair.values())
+    if calls < 2 or entries > FORK_ENTRIES or torch.cuda.is_current_stream_capturing():
+        return (lambda key: stream.cuda_stream), (lambda: None)
+    side, keys, start = {}, {}, stream.record_event()
+
+    def at(key):
+        k = keys.setdefault(key, len(keys)) % 4
+        if k not in side:
+            side[k] = torch.cuda.Stream(device=dl.device)
+            side[k].wait_event(start)
+        return side[k].cuda_stream
+
+    def join():
+        for st in side.values():
+            stream.wait_stream(st)
+
+    return at, join
 
 
 def gpu_schwarz_fn(device="cuda"):

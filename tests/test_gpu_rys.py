@@ -167,3 +167,21 @@ def test_long_partner_segments(prims):
     L.exchange("ssss", fock.exchange_args(dl, "ssss", out, torch.cuda.current_stream().cuda_stream, 0.0))
     torch.cuda.synchronize()
     assert int(kp.counts.max()) > 256 and close(out.cpu().numpy(), exp), (out.cpu().numpy(), exp)
+
+
+def test_quartet_counts_do_not_depend_on_precision():
+    """Every screened-in quartet is evaluated once, in FP64 or in FP32."""
+    L = lib()
+    wl, rl = system(3, 3, 4.0, 9, False)
+    dl = fock.to_device(rl)
+    counts = []
+    try:
+        for cut in (0.0, 1e-6, 1e30):
+            L.set_fp32_cut(cut)
+            L.reset_counters()
+            fock.build_jk(dl)
+            torch.cuda.synchronize()
+            counts.append(L.quartet_counters())
+    finally:
+        L.set_fp32_cut(0.0)
+    assert counts[0] == counts[1] == counts[2], counts

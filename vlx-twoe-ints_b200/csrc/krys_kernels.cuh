@@ -18,8 +18,9 @@
 // quartet by one lane for up to 32 quartets at a time and read back from
 // shared memory by the lanes of the roots.
 //
-// Bound: FP64 issue.  (SD|DD) on 10 atoms 4s3p2d runs the FP64 pipe at 66 %
-// with two CTAs of 128 threads per SM (registers); with the tables in shared
+// Bound: FP64 issue.  (SD|DD) on 10 atoms 4s3p2d runs the FP64 pipe at 57 %
+// ((PD|DP) 65 %), the rest being arithmetic latency that two warps per scheduler do not
+// cover, with two CTAs of 128 threads per SM (registers); with the tables in shared
 // memory the shared-memory pipe limits it (80 % busy, FP64 at 45 %).  Against
 // the column kernels it replaces, ms per class call on that case: (DD|DD) 37.0
 // -> 10.3, (PD|DD) 33.2 -> 9.6, (PD|DP) 31.8 -> 6.7, (DP|DD) 18.6 -> 5.8,
@@ -467,7 +468,8 @@ exchange_rys_kernel(KOutBlocks out, KPartnerRecs ab, KPartnerRecs cd, KGroups ga
             const int nj = min(K_JCHUNK, a1 - jb);
             k_chunk_scan(ab, cd, jb, nj, c0, c1, mD, thr, grouped ? 0.0 : fp32_cut, ch, a1 - a0, fp32_budget);
             const int total = s_c64[nj];
-            if (qcount && threadIdx.x == 0) atomicAdd(qcount, (unsigned long long)(total + s_c32[nj]));
+            // the contracted kernels count their own FP32 quartets
+            if (qcount && !grouped && threadIdx.x == 0) atomicAdd(qcount, (unsigned long long)(total + s_c32[nj]));
             if (grouped) {
                 // first FP32 group of l for every j record (the split of exchange_colc_kernel)
                 for (int t = threadIdx.x; t < nj; t += KR_THREADS) {
@@ -492,6 +494,7 @@ exchange_rys_kernel(KOutBlocks out, KPartnerRecs ab, KPartnerRecs cd, KGroups ga
                 }
                 const unsigned taken = __ballot_sync(0xffffffffu, mine);
                 const int n = __popc(taken);
+                if (grouped && qcount && lane == 0) atomicAdd(qcount, (unsigned long long)n);
                 if (mine)
                     krys_setup<false>(ab, cd, jb + jj, l, omega, set, __popc(taken & ((1u << lane) - 1)));
                 __syncwarp();

@@ -1,4 +1,6 @@
 // Warp-cooperative ("column") J and K kernels for the heavy classes (sm_100a).
+// The exchange kernels evaluate the FP32 quartets of mixed-precision calls
+// (k_mixed in launch.cuh); FP64 exchange runs on krys_kernels.cuh.
 //
 // A group of ColTab::NL lanes evaluates one primitive shell quartet: lane x
 // holds the column [x|y]^(m) of its lane-side Cartesian component x in

@@ -15,7 +15,9 @@
 // Cartesian component quartet per work item, evaluated by Rys quadrature in
 // registers (eri_component), rho' = rho for the Coulomb operator and
 // rho w^2 / (rho + w^2) for the attenuated one.  Two atoms 1s1p1d1f (170 f class
-// calls): 189 ms with a Hermite box per component in local memory, 39 ms so.
+// calls and the s/p/d ones): 209 ms with a Hermite box per component in local
+// memory, 45 ms so, 27 ms with four blocks per SM and wide blocks for short
+// lists, 21 ms with the class calls on side streams.
 // Screening is the reference's per-component predicate
 // (|Q_ij Q_kl D_kl| > thr for J, |Q_ij Q_kl max_D| > thr for K), the J ket
 // weights gen_coulomb.py:276-281, the K density gather gen_exchange.py:323.

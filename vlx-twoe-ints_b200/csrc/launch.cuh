@@ -10,10 +10,10 @@ namespace vlxb {
 // Exchange kernel of a class.  The thread-per-quartet kernel shares a quartet's
 // set-up and recurrences among all its components and wins while its
 // straight-line code fits in registers; the Rys kernel repeats part of them per
-// root.  10 atoms 4s3p2d, thread / Rys, ms per class call: (PP|PP) 1.6 / 3.3,
-// (SD|DS) 2.7 / 6.1 (L = 4, tables in shared memory); (DP|DS) 2.10 / 2.15,
-// (PD|DS) 3.8 / 3.7, (SP|DD) 4.8 / 3.4, (PP|DP) 9.2 / 4.4, (SD|PD) 11.3 / 4.5
-// (L = 5); (DS|DD) 7.2 / 2.6 (L = 6).
+// root.  10 atoms 4s3p2d, thread / Rys, ms per class call: (PP|PP) 1.3 / 1.8,
+// (SD|DS) 2.2 / 2.9, (SP|PD) 2.5 / 3.3 (L = 4); (DP|DS) 2.10 / 2.15, (PD|DS)
+// 3.8 / 3.7, (SP|DD) 4.8 / 3.4, (PP|DP) 9.2 / 4.4, (SD|PD) 11.3 / 4.5 (L = 5);
+// (DS|DD) 7.2 / 2.6 (L = 6).
 __host__ __device__ constexpr bool k_rys(int la, int lb, int lc, int ld) { return la + lb + lc + ld >= 5; }
 
 // FP64 kernel of a Coulomb class: Rys where the thread-per-quartet kernel's
@@ -94,8 +94,9 @@ int launch_exchange_mixed(int grid, cudaStream_t st, const KOutBlocks& out, cons
 
 template <int LA, int LB, int LC, int LD>
 int launch_exchange_rys(int grid, cudaStream_t st, const KOutBlocks& out, const KPartnerRecs& ab,
-                        const KPartnerRecs& cd, const KGroups& gab, const KGroups& gcd, const KDensity& dm, double maxD, double omega, double thr,
-                        double* mat_K, unsigned long long* qk, double cut, double budget);
+                        const KPartnerRecs& cd, const KGroups& gab, const KGroups& gcd, const KDensity& dm,
+                        double maxD, double omega, double thr, double* mat_K, unsigned long long* qk, double cut,
+                        double budget);
 
 // D_ik per (i, k) block of the exchange gradient: rows / columns of the (i, k)
 // components in the AO density (single-molecule calls).

@@ -13,8 +13,8 @@
 // same counters, same FP32/FP64 passes as coulomb_kernel; no atomics on J.
 //
 // The nuclear-gradient form of the same mathematics (bra Hermite range one
-// level higher, derivative epilogue) is coulomb_grad_kernel in
-// jgrad_kernels.cuh.
+// level higher, derivative epilogue) is in jrys_kernels.cuh, which evaluates
+// R by Rys quadrature.
 #pragma once
 #include <type_traits>
 

@@ -3,6 +3,7 @@
 // integral kernel; the 90 classes of a build do that 225 times for only 27
 // distinct lists.  Here every list is prepared once: two atoms 4s3p2d, 4735
 // device operations and 25.5 ms per build become about 700 and 4.0 ms.
+#include <algorithm>
 #include <mutex>
 
 #include "classes.cuh"
@@ -169,11 +170,47 @@ static int run_build(const VlxbFockBuild& b, PrepShare& share, Fork* fork, cudaS
     return VLXB_OK;
 }
 
+// Scratch of the shared preparations, from the sizes of the lists' dense bounds:
+// a partner list reserves its whole (shell, shell, component) table.  A class
+// call holds two such lists at a time, a shared build nine, which grows with
+// the square of the primitive count: 14 atoms 4s3p2d 0.1 GB, but a union of 64
+// molecules of 3 to 8 atoms 53 GB in FP64 and 157 GB in mixed precision.
+static uint64_t share_bytes(const VlxbFockBuild& b)
+{
+    static const int pair_ab[6][2] = {{0, 0}, {0, 1}, {0, 2}, {1, 1}, {1, 2}, {2, 2}};
+    bool kp[9] = {}, j[9] = {};
+    for (int x = 0; x < 6; x++) {
+        for (int y = 0; y < 6; y++)
+            if ((b.j_classes >> (x * 6 + y)) & 1ull)
+                j[pair_ab[x][0] * 3 + pair_ab[x][1]] = j[pair_ab[y][0] * 3 + pair_ab[y][1]] = true;
+        for (int bd = 0; bd < 9; bd++)
+            if ((b.k_classes >> (x * 9 + bd)) & 1ull)
+                kp[pair_ab[x][0] * 3 + bd / 3] = kp[pair_ab[x][1] * 3 + bd % 3] = true;
+    }
+    uint64_t bytes = 0;
+    for (int p = 0; p < 9; p++) {
+        const int la = p / 3, lb = p % 3;
+        const uint64_t nxy = (uint64_t)ncart(la) * ncart(lb), ntab = (uint64_t)b.prim_count[la] * b.prim_count[lb];
+        if (kp[p]) {
+            uint64_t rec = 60;  // records before and after the sort, S, list positions
+            if (fp32_cut_get() > 0.0) rec += (k_pair_contracted(la, lb) ? 150 : 0) + (fp32_budget_get() > 0.0 ? 32 : 0);
+            bytes += ntab * (130 + rec * nxy);
+        }
+        if (j[p]) bytes += ntab * 8 + std::min<uint64_t>(b.j_count[p], ntab) * (250 + 16 * (4 * nxy + 35));
+    }
+    return bytes;
+}
+
+// Above this (of 180 GB) a build goes class by class: its integral kernels take
+// minutes, beside which the repeated preparations are nothing.
+constexpr uint64_t SHARE_MAX_BYTES = 40ull << 30;
+
 }  // namespace vlxb
 
 extern "C" int vlxb_fockBuild(const VlxbFockBuild* b, void* stream)
 {
     if (!b || b->n_mol < 0 || b->grad_stride > (uint64_t)INT64_MAX || (b->gradient && b->n_mol > 0)) return VLXB_EINVAL;
+    if (vlxb::share_bytes(*b) > vlxb::SHARE_MAX_BYTES) return VLXB_ENOMEM;
     const cudaStream_t st = (cudaStream_t)stream;
     vlxb::PrepShare share(st);
     share.prepare_only = true;  // every list first: a call short of memory then leaves the outputs as they were

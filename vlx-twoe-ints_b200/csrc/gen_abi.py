@@ -297,9 +297,10 @@ def header():
          "   row stride grad_stride.  n_mol > 0: a batch as for vlxb_coulombBatch /",
          "   vlxb_exchangeBatch (prim_mol, prim_aocols, D_stride, maxD_mol), else those",
          "   are ignored (D_stride 0 = naos).  All preparations are held until the",
-         "   call's work is done on the stream; VLXB_ENOMEM is returned before any",
-         "   output is touched, and the class calls, which hold one class's at a time,",
-         "   remain.  No reference counterpart. */",
+         "   call's work is done on the stream; VLXB_ENOMEM (they do not fit, or their",
+         "   bound is above 40 GB) is returned before any output is touched, and the",
+         "   class calls, which hold one class's at a time, remain.  No reference",
+         "   counterpart. */",
          "typedef struct VlxbFockBuild {",
          "    const double* prim_info[3];",
          "    const uint32_t* prim_aoinds[3];",

@@ -216,11 +216,13 @@ def build_jk(dl: DeviceLists, stream: torch.cuda.Stream | None = None, omega: fl
                 jcls = [c for c in jcls if "f" in c]
                 kcls = [c for c in kcls if "f" in c]
         at, join = _fork(dl, stream, len(jcls) + len(kcls))
-        for cls in jcls:
-            L.coulomb(cls, coulomb_args(dl, cls, matJ[cls[:2]], at("J" + cls[:2])))
-        for cls in kcls:
-            L.exchange(cls, exchange_args(dl, cls, matK[cls[0] + cls[2]], at("K" + cls[0] + cls[2]), omega))
-        join()
+        try:
+            for cls in jcls:
+                L.coulomb(cls, coulomb_args(dl, cls, matJ[cls[:2]], at("J" + cls[:2])))
+            for cls in kcls:
+                L.exchange(cls, exchange_args(dl, cls, matK[cls[0] + cls[2]], at("K" + cls[0] + cls[2]), omega))
+        finally:
+            join()  # also after an error: nothing runs on that `stream` does not wait for
     return matJ, matK
 
 

@@ -185,3 +185,57 @@ def test_quartet_counts_do_not_depend_on_precision():
     finally:
         L.set_fp32_cut(0.0)
     assert counts[0] == counts[1] == counts[2], counts
+
+
+@pytest.mark.parametrize("prims", [63, 64, 65, 181, 182])
+def test_short_scans(prims):
+    """Occupancy tables around one round (64 x 64 entries) and around the bound
+    (182 x 182 is above it) of the one-block scan: s primitives on one centre,
+    sparse J and (i, k) lists that hold the first and the last pair."""
+    L = lib()
+    L.init(0)
+    wl = basis.config_custom(1, 3.0, {0: 1}, prims, 0.02, 1.08, 1, 1e-12, 4)
+    rl = lists.build_lists(wl.mol, wl.D, 0.0, fock.gpu_schwarz_fn())
+    last = prims - 1
+    jl, kq = rl.jlists["ss"], rl.kpairs["ss"]
+    f, g = jl.first.astype(np.int64), jl.second.astype(np.int64)
+    pick = np.flatnonzero((f * 7 + g) % 61 == 3)
+    pick = np.unique(np.concatenate([pick, np.flatnonzero((f == 0) & (g == 0)), np.flatnonzero((f == last) & (g == last))]))
+    for n in ("first", "second", "pdata", "Q", "D"):
+        setattr(jl, n, np.ascontiguousarray(getattr(jl, n)[pick]))
+    i, k = kq.pair_i.astype(np.int64), kq.pair_k.astype(np.int64)
+    rows = np.flatnonzero(((i == 0) & (k == 0)) | ((i == last) & (k == last)) | ((i == 1) & (k == last)))
+    kq.pair_i, kq.pair_k = kq.pair_i[rows].copy(), kq.pair_k[rows].copy()
+    expJ, expK = helpers.oracle_J(rl, "ssss"), helpers.oracle_K(rl, "ssss")
+    dl = fock.to_device(rl)
+    matJ, matK = fock.build_jk(dl)
+    torch.cuda.synchronize()
+    assert len(rows) == 3 and len(pick) > 30
+    assert close(matJ["ss"].cpu().numpy(), expJ), (matJ["ss"], expJ)
+    assert close(matK["ss"].cpu().numpy(), expK), (matK["ss"], expK)
+
+
+@pytest.mark.parametrize("kets", [1, 33, 511, 513, 4096, 4097])
+def test_short_ket_sorts(kets):
+    """Ket lists around the tile and the bound of the rank sort, in a shuffled
+    order (the engine sorts them): seeded bra rows of (ss|ss)."""
+    L = lib()
+    L.init(0)
+    wl = basis.config_custom(1, 3.0, {0: 1}, 100, 0.02, 1.08, 1, 1e-12, 4)
+    rl = lists.build_lists(wl.mol, wl.D, 0.0, fock.gpu_schwarz_fn())
+    rng = np.random.default_rng(kets)
+    jl = rl.jlists["ss"]  # by descending |Q D|
+    names = ("first", "second", "pdata", "Q", "D")
+    pick = np.sort(rng.permutation(len(jl.first))[:kets])
+    for n in names:
+        setattr(jl, n, np.ascontiguousarray(getattr(jl, n)[pick]))
+    rl.threshold = 0.5 * float(np.median(np.abs(jl.Q * jl.D)) * np.median(jl.Q))  # screens out some of the kets
+    rows = rng.permutation(kets)[:5]
+    exp = helpers.oracle_J(rl, "ssss", rows=rows)[rows]
+    order = rng.permutation(kets)
+    for n in names:
+        setattr(jl, n, np.ascontiguousarray(getattr(jl, n)[order]))
+    matJ, _ = fock.build_jk(fock.to_device(rl), do_k=False)
+    got = np.empty(kets)
+    got[order] = matJ["ss"].cpu().numpy()
+    assert np.abs(exp).max() > 0.0 and close(got[rows], exp), (got[rows], exp)

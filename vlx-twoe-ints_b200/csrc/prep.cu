@@ -202,6 +202,29 @@ static int scan_int(Arena& ar, const int* in, int* out, int64_t n)
     return VLXB_OK;
 }
 
+// Exclusive scan with its total.  One block takes short arrays: three launches
+// of some 2 us each become one of 2 to 5 us.  At the bound it makes eight rounds.
+constexpr int64_t SCAN_BLOCK_MAX = 32768;
+
+static int scan_total(Arena& ar, const int* in, int* out, int64_t n, const int* valid, int* total)
+{
+    if (n <= SCAN_BLOCK_MAX) {
+        if (!ar.measuring()) {
+            k_scan_block<<<1, SCAN_THREADS, 0, ar.stream()>>>(in, out, (int)n, valid, total);
+            note_launches();
+        }
+    } else {
+        const int rc = scan_int(ar, in, out, n);
+        if (rc) return rc;
+        if (!ar.measuring()) {
+            k_scan_total<<<1, 1, 0, ar.stream()>>>(out, in, n, total);
+            note_launches();
+        }
+    }
+    VLXB_CHECK_CUDA(cudaGetLastError());
+    return VLXB_OK;
+}
+
 static int inclusive_sum_f64(Arena& ar, const double* in, double* out, int64_t n)
 {
     size_t bytes = 0;
@@ -216,18 +239,10 @@ static int inclusive_sum_f64(Arena& ar, const double* in, double* out, int64_t n
 
 static int finish_grouping(Arena& ar, int64_t ntab, int* table, PairGroups& g)
 {
-    cudaStream_t st = ar.stream();
     g.spidx = ar.alloc<int>(ntab);
     g.n_sp = ar.alloc<int>(1);
     if (!g.spidx || !g.n_sp) return VLXB_ENOMEM;
-    int rc = scan_int(ar, table, g.spidx, ntab);
-    if (rc) return rc;
-    if (!ar.measuring()) {
-        k_scan_total<<<1, 1, 0, st>>>(g.spidx, table, ntab, g.n_sp);
-    }
-    if (!ar.measuring()) note_launches();
-    VLXB_CHECK_CUDA(cudaGetLastError());
-    return VLXB_OK;
+    return scan_total(ar, table, g.spidx, ntab, nullptr, g.n_sp);
 }
 
 static int alloc_sp(Arena& ar, int nxy, PairGroups& g)
@@ -237,9 +252,6 @@ static int alloc_sp(Arena& ar, int nxy, PairGroups& g)
     g.entry = ar.alloc<int32_t>(g.sp_stride * nxy);
     g.geo = ar.alloc<double>(g.sp_stride * GEO_N);
     if (ar.failed()) return VLXB_ENOMEM;
-    if (!ar.measuring()) {
-        VLXB_CHECK_CUDA(cudaMemsetAsync(g.entry, 0xFF, sizeof(int32_t) * g.sp_stride * nxy, ar.stream()));
-    }
     return VLXB_OK;
 }
 
@@ -254,15 +266,16 @@ int group_flat(Arena& ar, int na, int nb, int npa, int npb, const uint32_t* firs
     if (!ar.measuring()) {
         VLXB_CHECK_CUDA(cudaMemsetAsync(table, 0, sizeof(int) * ntab, st));
     }
+    g.sp_stride = n < ntab ? n : ntab;
+    int rc = alloc_sp(ar, na * nb, g);
+    if (rc) return rc;
     if (!ar.measuring()) {
-        k_mark_pairs<<<prep_blocks(n), PREP_THREADS, 0, st>>>(first, second, n, na, nb, npb, table);
+        k_mark_pairs<<<prep_blocks(n), PREP_THREADS, 0, st>>>(first, second, n, na, nb, npb, table, g.entry,
+                                                              g.sp_stride * na * nb);
     }
     if (!ar.measuring()) note_launches();
     VLXB_CHECK_CUDA(cudaGetLastError());
-    int rc = finish_grouping(ar, ntab, table, g);
-    if (rc) return rc;
-    g.sp_stride = n < ntab ? n : ntab;
-    rc = alloc_sp(ar, na * nb, g);
+    rc = finish_grouping(ar, ntab, table, g);
     if (rc) return rc;
     if (!ar.measuring()) {
         k_fill_pairs<<<prep_blocks(n), PREP_THREADS, 0, st>>>(first, second, n, na, nb, npb, g.spidx, g.entry, g.sp_i,
@@ -291,15 +304,16 @@ int group_csr(Arena& ar, int na, int nb, int npa, int npb, const uint32_t* displ
     if (!ar.measuring()) {
         VLXB_CHECK_CUDA(cudaMemsetAsync(table, 0, sizeof(int) * ntab, st));
     }
+    g.sp_stride = n_entries_bound < ntab ? n_entries_bound : ntab;
+    int rc = alloc_sp(ar, na * nb, g);
+    if (rc) return rc;
     if (!ar.measuring()) {
-        k_mark_csr<<<prep_blocks((int64_t)n_first * 32), PREP_THREADS, 0, st>>>(displs, counts, Dinds, n_first, na, nb, npb, table);
+        k_mark_csr<<<prep_blocks((int64_t)n_first * 32), PREP_THREADS, 0, st>>>(
+            displs, counts, Dinds, n_first, na, nb, npb, table, g.entry, g.sp_stride * na * nb);
     }
     if (!ar.measuring()) note_launches();
     VLXB_CHECK_CUDA(cudaGetLastError());
-    int rc = finish_grouping(ar, ntab, table, g);
-    if (rc) return rc;
-    g.sp_stride = n_entries_bound < ntab ? n_entries_bound : ntab;
-    rc = alloc_sp(ar, na * nb, g);
+    rc = finish_grouping(ar, ntab, table, g);
     if (rc) return rc;
     if (!ar.measuring()) {
         k_fill_csr<<<prep_blocks((int64_t)n_first * 32), PREP_THREADS, 0, st>>>(displs, counts, Dinds, n_first, na, nb, npb, g.spidx,
@@ -337,12 +351,8 @@ template <int NXY>
 static void launch_sp_S(const PairGroups& g, const double* pdata, cudaStream_t st)
 {
     {
-        k_sp_S<NXY><<<prep_blocks(g.sp_stride), PREP_THREADS, 0, st>>>(g.n_sp, g.entry, g.sp_stride, pdata, g.S);
-    }
-    note_launches();
-    {
-        k_rec_uniform_s<NXY><<<prep_blocks(g.rec_stride), PREP_THREADS, 0, st>>>(g.n_rec, g.rec_sp, g.rec_mask, g.S,
-                                                                                 g.sp_stride, g.su);
+        k_sp_S<NXY><<<prep_blocks(g.rec_stride), PREP_THREADS, 0, st>>>(g.n_sp, g.entry, g.sp_stride, pdata, g.S,
+                                                                        g.n_rec, g.rec_sp, g.rec_mask, g.su);
     }
     note_launches();
 }
@@ -371,19 +381,15 @@ int make_records(Arena& ar, int nxy, PairGroups& g, const double* Q, int64_t n_e
     g.rec_q = ar.alloc<double>(g.rec_stride);
     g.rec_mask = ar.alloc<uint64_t>(g.rec_stride);
     if (ar.failed()) return VLXB_ENOMEM;
-    if (!ar.measuring()) {
+    if (!ar.measuring() && g.sp_stride + 1 > SCAN_BLOCK_MAX) {  // the short scan leaves out what is not counted
         VLXB_CHECK_CUDA(cudaMemsetAsync(nrec, 0, sizeof(int) * (g.sp_stride + 1), st));
     }
     if (!ar.measuring()) {
         VLXB_NXY_DISPATCH(nxy, launch_rec_count, g, Q, nrec, st);
     }
     VLXB_CHECK_CUDA(cudaGetLastError());
-    int rc = scan_int(ar, nrec, recoff, g.sp_stride + 1);
+    int rc = scan_total(ar, nrec, recoff, g.sp_stride + 1, g.n_sp, g.n_rec);
     if (rc) return rc;
-    if (!ar.measuring()) {
-        k_scan_total<<<1, 1, 0, st>>>(recoff, nrec, g.sp_stride + 1, g.n_rec);
-    }
-    if (!ar.measuring()) note_launches();
     if (!ar.measuring()) {
         VLXB_NXY_DISPATCH(nxy, launch_rec_fill, g, Q, recoff, st);
     }
@@ -410,17 +416,17 @@ int segment_records(Arena& ar, int nxy, int npa, int npb, PairGroups& g, const d
     g.S = ar.alloc<double>(g.sp_stride * nxy);
     g.su = ar.alloc<double>(g.rec_stride);
     if (ar.failed()) return VLXB_ENOMEM;
-    if (!ar.measuring()) {
-        k_rec_segments<<<prep_blocks(npa + 1), PREP_THREADS, 0, st>>>(g.spidx, recoff, npa, npb, g.n_rec, seg);
-    }
-    if (!ar.measuring()) note_launches();
     if ((int64_t)npb * nxy <= SORT_SEGMENT_MAX) {
         if (!ar.measuring()) {
-            k_sort_segments<<<npa, 128, 0, st>>>(seg, npa, g.rec_q, g.rec_sp, g.rec_mask, q_sorted, sp_sorted,
-                                                 mask_sorted);
+            k_sort_segments<<<npa, 128, 0, st>>>(g.spidx, recoff, npa, npb, g.n_rec, seg, g.rec_q, g.rec_sp,
+                                                 g.rec_mask, q_sorted, sp_sorted, mask_sorted);
             note_launches();
         }
     } else {
+        if (!ar.measuring()) {
+            k_rec_segments<<<prep_blocks(npa + 1), PREP_THREADS, 0, st>>>(g.spidx, recoff, npa, npb, g.n_rec, seg);
+            note_launches();
+        }
         int* perm_in = ar.alloc<int>(g.rec_stride);
         int* perm = ar.alloc<int>(g.rec_stride);
         if (ar.failed()) return VLXB_ENOMEM;
@@ -541,6 +547,10 @@ int contract_groups(Arena& ar, int npa, PairGroups& g, const uint32_t* part_aoin
     return VLXB_OK;
 }
 
+// Longest key array that k_rank_sort takes: up to it one launch of 3 to 6 us, the
+// library sort 14 us in one block and more than twice that above its tile.
+constexpr int64_t RANK_SORT_MAX = 4096;
+
 template <int LC, int LD>
 int jket_prepare(Arena& ar, const PairGroups& g, const uint32_t* first, const uint32_t* second,
                  const double* D, const double* Q, const double* pdata, JKetData& out,
@@ -576,19 +586,28 @@ int jket_prepare(Arena& ar, const PairGroups& g, const uint32_t* first, const ui
                                                                      g.geo, keys, tmin_u, Dpp_u, Dm_u, Qc_u, Dc_u, S);
     }
     if (!ar.measuring()) note_launches();
-    if (!ar.measuring()) {
+    if (!ar.measuring() && (S > RANK_SORT_MAX || prim_mol_c)) {
         k_iota<<<prep_blocks(S), PREP_THREADS, 0, st>>>(perm_in, S);
+        note_launches();
     }
-    if (!ar.measuring()) note_launches();
     VLXB_CHECK_CUDA(cudaGetLastError());
-    size_t bytes = 0;
-    VLXB_CHECK_CUDA(cub::DeviceRadixSort::SortPairsDescending(nullptr, bytes, keys, keys_sorted, perm_in, perm,
-                                                              (int)S, 0, 64, st));
-    void* tmp = ar.alloc<char>((int64_t)bytes);
-    if (!tmp) return VLXB_ENOMEM;
-    if (!ar.measuring()) {
-        VLXB_CHECK_CUDA(cub::DeviceRadixSort::SortPairsDescending(tmp, bytes, keys, keys_sorted, perm_in, perm, (int)S,
-                                                                  0, 64, st));
+    if (S <= RANK_SORT_MAX) {
+        if (!ar.measuring()) {
+            constexpr int per_block = RANK_THREADS / RANK_SPLIT;
+            k_rank_sort<<<((int)S + per_block - 1) / per_block, RANK_THREADS, 0, st>>>(keys, (int)S, keys_sorted, perm);
+            note_launches();
+        }
+        VLXB_CHECK_CUDA(cudaGetLastError());
+    } else {
+        size_t bytes = 0;
+        VLXB_CHECK_CUDA(cub::DeviceRadixSort::SortPairsDescending(nullptr, bytes, keys, keys_sorted, perm_in, perm,
+                                                                  (int)S, 0, 64, st));
+        void* tmp = ar.alloc<char>((int64_t)bytes);
+        if (!tmp) return VLXB_ENOMEM;
+        if (!ar.measuring()) {
+            VLXB_CHECK_CUDA(cub::DeviceRadixSort::SortPairsDescending(tmp, bytes, keys, keys_sorted, perm_in, perm,
+                                                                      (int)S, 0, 64, st));
+        }
     }
     if (prim_mol_c) {
         // stable second sort by molecule: per molecule, descending bound
@@ -698,23 +717,21 @@ int kout_prepare(Arena& ar, int na, int nc, int npa, int npc, const uint32_t* pi
     if (!ar.measuring()) {
         VLXB_CHECK_CUDA(cudaMemsetAsync(table, 0, sizeof(int) * ntab, st));
     }
-    if (!ar.measuring()) {
-        k_mark_pairs<<<prep_blocks(n), PREP_THREADS, 0, st>>>(pi, pk, n, na, nc, npc, table);
-    }
-    if (!ar.measuring()) note_launches();
-    VLXB_CHECK_CUDA(cudaGetLastError());
-    PairGroups g;
-    int rc = finish_grouping(ar, ntab, table, g);
-    if (rc) return rc;
     out.stride = n < ntab ? n : ntab;
-    out.n = g.n_sp;
     out.ish = ar.alloc<int32_t>(out.stride);
     out.ksh = ar.alloc<int32_t>(out.stride);
     out.idx = ar.alloc<int32_t>(out.stride * na * nc);
     if (ar.failed()) return VLXB_ENOMEM;
     if (!ar.measuring()) {
-        VLXB_CHECK_CUDA(cudaMemsetAsync(out.idx, 0xFF, sizeof(int32_t) * out.stride * na * nc, st));
+        k_mark_pairs<<<prep_blocks(n), PREP_THREADS, 0, st>>>(pi, pk, n, na, nc, npc, table, out.idx,
+                                                              out.stride * na * nc);
+        note_launches();
     }
+    VLXB_CHECK_CUDA(cudaGetLastError());
+    PairGroups g;
+    int rc = finish_grouping(ar, ntab, table, g);
+    if (rc) return rc;
+    out.n = g.n_sp;
     if (!ar.measuring()) {
         VLXB_NXY_DISPATCH(na * nc, launch_kout, pi, pk, n, na, nc, npc, g.spidx, out, st);
     }

@@ -37,9 +37,19 @@ __global__ void k_iota(int* __restrict__ p, int64_t n)
 
 // ------------------------------------------------------------ flat lists
 
-__global__ void k_mark_pairs(const uint32_t* __restrict__ first, const uint32_t* __restrict__ second,
-                             int64_t n, int na, int nb, int npb, int* __restrict__ table)
+// Both marking kernels also set the list positions that the next launch fills
+// (entry, n_entry values) to -1, which saves a memset per list.
+__device__ __forceinline__ void clear_entries(int32_t* __restrict__ entry, int64_t n_entry)
 {
+    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n_entry; e += (int64_t)gridDim.x * blockDim.x)
+        entry[e] = -1;
+}
+
+__global__ void k_mark_pairs(const uint32_t* __restrict__ first, const uint32_t* __restrict__ second,
+                             int64_t n, int na, int nb, int npb, int* __restrict__ table,
+                             int32_t* __restrict__ entry, int64_t n_entry)
+{
+    clear_entries(entry, n_entry);
     for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x) {
         const int64_t key = (int64_t)(first[e] / na) * npb + second[e] / nb;
         table[key] = 1;
@@ -68,8 +78,9 @@ __global__ void k_fill_pairs(const uint32_t* __restrict__ first, const uint32_t*
 // list; one thread per first index took 9.4 + 4.0 ms of a 14-atom build).
 __global__ void k_mark_csr(const uint32_t* __restrict__ displs, const uint32_t* __restrict__ counts,
                            const uint32_t* __restrict__ Dinds, int n_first, int na, int nb, int npb,
-                           int* __restrict__ table)
+                           int* __restrict__ table, int32_t* __restrict__ entry, int64_t n_entry)
 {
+    clear_entries(entry, n_entry);
     const int lane = threadIdx.x & 31, warps = gridDim.x * (blockDim.x >> 5);
     for (int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < n_first; i += warps) {
         const uint32_t d0 = displs[i], c = counts[i];
@@ -100,6 +111,54 @@ __global__ void k_fill_csr(const uint32_t* __restrict__ displs, const uint32_t* 
 __global__ void k_scan_total(const int* __restrict__ scan, const int* __restrict__ flag, int64_t n, int* __restrict__ out)
 {
     if (blockIdx.x == 0 && threadIdx.x == 0) out[0] = (n > 0) ? scan[n - 1] + flag[n - 1] : 0;
+}
+
+// Exclusive scan of short arrays and its total in one launch: one block, four
+// values per thread and round.  valid: values from position *valid on count as
+// zero (n values are written all the same).
+constexpr int SCAN_THREADS = 1024;
+
+__global__ void __launch_bounds__(SCAN_THREADS)
+k_scan_block(const int* __restrict__ in, int* __restrict__ out, int n, const int* __restrict__ valid,
+             int* __restrict__ total)
+{
+    __shared__ int wsum[SCAN_THREADS / 32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int m = valid ? min(n, *valid) : n;
+    int carry = 0;
+    for (int t0 = 0; t0 < n; t0 += 4 * SCAN_THREADS) {
+        const int i0 = t0 + 4 * (int)threadIdx.x;
+        int v[4], sum = 0;
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            v[u] = i0 + u < m ? in[i0 + u] : 0;
+            sum += v[u];
+        }
+        int x = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (lane == 31) wsum[w] = x;
+        __syncthreads();
+        int z = wsum[lane];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, z, o);
+            if (lane >= o) z += y;
+        }
+        const int before = __shfl_sync(0xffffffffu, z, w > 0 ? w - 1 : 0);
+        int run = carry + (w > 0 ? before : 0) + x - sum;
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            if (i0 + u < n) out[i0 + u] = run;
+            run += v[u];
+        }
+        carry += __shfl_sync(0xffffffffu, z, 31);
+        __syncthreads();  // wsum is written again
+    }
+    if (threadIdx.x == 0) *total = carry;
 }
 
 // Pair geometry (see PairGeo): z, 0.5/z, P, P - A, A - B, and the first
@@ -135,12 +194,45 @@ __global__ void k_pair_geo(const int* __restrict__ n_sp, const int32_t* __restri
 // (shell pair, q, component bitmask).  Records of a shell pair follow the
 // first appearance of each distinct q in component order.
 
+// Loads every component's Q of shell pair s at once (the loops over distinct
+// values would wait for them one by one: 2 us of a 5 us launch on short lists);
+// true: the components present share one value, q (their mask in m).
+template <int NXY>
+__device__ __forceinline__ bool rec_one_q(const int32_t* __restrict__ entry, int64_t stride,
+                                          const double* __restrict__ Q, int s, double& q, uint64_t& m)
+{
+    int32_t e[NXY];
+    double v[NXY];
+#pragma unroll
+    for (int c = 0; c < NXY; c++) e[c] = entry[c * stride + s];
+#pragma unroll
+    for (int c = 0; c < NXY; c++) v[c] = e[c] >= 0 ? Q[e[c]] : 0.0;
+    bool same = true;
+    m = 0;
+#pragma unroll
+    for (int c = 0; c < NXY; c++) {
+        if (e[c] < 0) continue;
+        if (m == 0)
+            q = v[c];
+        else
+            same &= v[c] == q;
+        m |= 1ull << c;
+    }
+    return same;
+}
+
 template <int NXY>
 __global__ void k_rec_count(const int* __restrict__ n_sp, const int32_t* __restrict__ entry, int64_t stride,
                             const double* __restrict__ Q, int* __restrict__ nrec)
 {
     const int n = *n_sp;
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x) {
+        double q = 0.0;
+        uint64_t m;
+        if (rec_one_q<NXY>(entry, stride, Q, s, q, m)) {
+            nrec[s] = m != 0;
+            continue;
+        }
         double qs[NXY];
         int nd = 0;
         for (int c = 0; c < NXY; c++) {
@@ -162,6 +254,17 @@ __global__ void k_rec_fill(const int* __restrict__ n_sp, const int32_t* __restri
 {
     const int n = *n_sp;
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x) {
+        const int r0 = recoff[s];
+        double q = 0.0;
+        uint64_t m;
+        if (rec_one_q<NXY>(entry, stride, Q, s, q, m)) {
+            if (m) {
+                rec_sp[r0] = s;
+                rec_q[r0] = q;
+                rec_mask[r0] = m;
+            }
+            continue;
+        }
         double qs[NXY];
         uint64_t ms[NXY];
         int nd = 0;
@@ -174,7 +277,6 @@ __global__ void k_rec_fill(const int* __restrict__ n_sp, const int32_t* __restri
             if (t == nd) { qs[nd] = v; ms[nd] = 0; nd++; }
             ms[t] |= (1ull << c);
         }
-        const int r0 = recoff[s];
         for (int t = 0; t < nd; t++) {
             rec_sp[r0 + t] = s;
             rec_q[r0 + t] = qs[t];
@@ -183,37 +285,36 @@ __global__ void k_rec_fill(const int* __restrict__ n_sp, const int32_t* __restri
     }
 }
 
-// S per shell pair and component (0 where the caller has no entry).
+// S per shell pair and component (0 where the caller has no entry), and su[r]
+// = the S shared by all components of record r when the record covers every
+// component of its shell pair and they share one S value, else NaN (the
+// kernels then digest with per-component S).
 template <int NXY>
 __global__ void k_sp_S(const int* __restrict__ n_sp, const int32_t* __restrict__ entry, int64_t stride,
-                       const double* __restrict__ pdata, double* __restrict__ S)
+                       const double* __restrict__ pdata, double* __restrict__ S, const int* __restrict__ n_rec,
+                       const int32_t* __restrict__ rec_sp, const uint64_t* __restrict__ rec_mask,
+                       double* __restrict__ su)
 {
-    const int n = *n_sp;
-    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x)
+    const int n = *n_sp, nr = *n_rec;
+    const int t0 = blockIdx.x * blockDim.x + threadIdx.x, dt = gridDim.x * blockDim.x;
+    for (int s = t0; s < n; s += dt)
+#pragma unroll
         for (int c = 0; c < NXY; c++) {
             const int32_t e = entry[c * stride + s];
             S[c * stride + s] = (e >= 0) ? pdata[e] : 0.0;
         }
-}
-
-// su[r] = the S shared by all components of record r when the record covers
-// every component of its shell pair and they share one S value, else NaN
-// (the kernels then digest with per-component S).
-template <int NXY>
-__global__ void k_rec_uniform_s(const int* __restrict__ n_rec, const int32_t* __restrict__ rec_sp,
-                                const uint64_t* __restrict__ rec_mask, const double* __restrict__ S, int64_t stride,
-                                double* __restrict__ su)
-{
-    const int n = *n_rec;
     const uint64_t full = (NXY >= 64) ? ~0ull : ((1ull << NXY) - 1ull);
-    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
+    for (int r = t0; r < nr; r += dt) {
         const int sp = rec_sp[r];
         double v = __longlong_as_double(0x7ff8000000000000ll);
-        if (rec_mask[r] == full) {
-            const double s0 = S[sp];
+        if (rec_mask[r] == full) {  // every entry is present; S may not be written yet
+            double x[NXY];
+#pragma unroll
+            for (int c = 0; c < NXY; c++) x[c] = pdata[entry[c * stride + sp]];
             bool same = true;
-            for (int c = 1; c < NXY; c++) same &= (S[c * stride + sp] == s0);
-            if (same) v = s0;
+#pragma unroll
+            for (int c = 1; c < NXY; c++) same &= x[c] == x[0];
+            if (same) v = x[0];
         }
         su[r] = v;
     }
@@ -232,7 +333,7 @@ __global__ void k_rec_segments(const int* __restrict__ spidx, const int* __restr
 // order: one block per segment, the position of a record is the number of
 // records before it (a segment holds the partners of one primitive, tens to a
 // few hundred).  q is compared as an order-preserving integer, so that every
-// bit pattern has a place.
+// bit pattern has a place.  Writes the segment offsets (as k_rec_segments).
 __device__ __forceinline__ uint64_t sort_key(double q)
 {
     const uint64_t u = (uint64_t)__double_as_longlong(q == 0.0 ? 0.0 : q);
@@ -241,14 +342,20 @@ __device__ __forceinline__ uint64_t sort_key(double q)
 
 constexpr int SORT_TILE = 512;
 
-__global__ void k_sort_segments(const int* __restrict__ seg, int nseg, const double* __restrict__ q,
-                                const int32_t* __restrict__ sp, const uint64_t* __restrict__ mask,
+__global__ void k_sort_segments(const int* __restrict__ spidx, const int* __restrict__ recoff, int nseg, int npb,
+                                const int* __restrict__ n_rec, int* __restrict__ seg,
+                                const double* __restrict__ q, const int32_t* __restrict__ sp, const uint64_t* __restrict__ mask,
                                 double* __restrict__ q_out, int32_t* __restrict__ sp_out,
                                 uint64_t* __restrict__ mask_out)
 {
     __shared__ uint64_t tile[SORT_TILE];
     for (int i = blockIdx.x; i < nseg; i += gridDim.x) {
-        const int b = seg[i], n = seg[i + 1] - b;
+        const int b = recoff[spidx[(int64_t)i * npb]];
+        const int end = i + 1 < nseg ? recoff[spidx[(int64_t)(i + 1) * npb]] : *n_rec, n = end - b;
+        if (threadIdx.x == 0) {
+            seg[i] = b;
+            if (i + 1 == nseg) seg[nseg] = end;
+        }
         for (int e0 = 0; e0 < n; e0 += blockDim.x) {  // every thread walks the tiles of each round
             const int e = e0 + threadIdx.x;
             const uint64_t key = e < n ? sort_key(q[b + e]) : 0;
@@ -266,6 +373,33 @@ __global__ void k_sort_segments(const int* __restrict__ seg, int nseg, const dou
                 mask_out[b + rank] = mask[b + e];
             }
         }
+    }
+}
+
+// Positions and keys of a short array in descending order, equal keys in their
+// order (the same permutation as a stable radix sort): the position is the
+// number of keys before it, counted by RANK_SPLIT lanes.
+constexpr int RANK_THREADS = 128, RANK_SPLIT = 4;
+
+__global__ void __launch_bounds__(RANK_THREADS)
+k_rank_sort(const double* __restrict__ key, int n, double* __restrict__ key_out, int* __restrict__ perm)
+{
+    __shared__ uint64_t tile[SORT_TILE];
+    const int sub = threadIdx.x % RANK_SPLIT, e = blockIdx.x * (RANK_THREADS / RANK_SPLIT) + threadIdx.x / RANK_SPLIT;
+    const uint64_t k = e < n ? sort_key(key[e]) : 0;
+    int rank = 0;
+    for (int t0 = 0; t0 < n; t0 += SORT_TILE) {
+        const int m = min(SORT_TILE, n - t0);
+        __syncthreads();
+        for (int t = threadIdx.x; t < m; t += RANK_THREADS) tile[t] = sort_key(key[t0 + t]);
+        __syncthreads();
+        for (int t = sub; t < m; t += RANK_SPLIT) rank += tile[t] > k || (tile[t] == k && t0 + t < e);
+    }
+    rank += __shfl_xor_sync(0xffffffffu, rank, 1);
+    rank += __shfl_xor_sync(0xffffffffu, rank, 2);
+    if (e < n && sub == 0) {
+        key_out[rank] = key[e];
+        perm[rank] = e;
     }
 }
 

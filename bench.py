@@ -136,7 +136,7 @@ def workload_desc(name, wl, rl):
     nk = sum(len(v.pair_i) for v in rl.kpairs.values())
     return {"workload": ("40 atoms 14-bohr cube 4s3p2d deg 3 Cartesian (1000 AOs), nocc 80, thr 1e-12"
                          if name == "medium" else "5 atoms 6-bohr cube 3s2p deg 3 (45 AOs), nocc 10, thr 1e-12"),
-            "precision": "fp64", "path": "C ABI: 36 Coulomb + 54 exchange entry points per build",
+            "precision": "fp64", "path": "C ABI: one vlxb_fockBuild over the 36 Coulomb + 54 exchange classes per build",
             "j_pairs": nj, "k_ik_pairs": nk, "naos": rl.naos}
 
 

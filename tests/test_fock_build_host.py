@@ -1,0 +1,36 @@
+"""Host side of vlxb_fockBuild against fakes of the list preparations and the
+kernel launchers (fock_build_host.cu); no GPU."""
+import os
+import shutil
+import subprocess
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+NVCC = os.environ.get("NVCC", "nvcc")
+
+
+@pytest.fixture(scope="module")
+def harness(tmp_path_factory):
+    if not shutil.which(NVCC):
+        pytest.skip("no nvcc")
+    exe = str(tmp_path_factory.mktemp("fockbuild") / "harness")
+    subprocess.run([NVCC, "-std=c++17", "-O0", "-gencode", "arch=compute_100a,code=sm_100a", "-o", exe,
+                    os.path.join(HERE, "fock_build_host.cu")], check=True, capture_output=True, text=True)
+
+    def run(scenario, number=0):
+        r = subprocess.run([exe, scenario, str(number)], check=True, capture_output=True, text=True, timeout=60)
+        return {k: int(v) for k, v in (ln.split() for ln in r.stdout.splitlines())}
+
+    return run
+
+
+@pytest.mark.parametrize("scenario", ["cutoff set", "cutoff reset", "budget set"])
+@pytest.mark.parametrize("reads", [1, 2, 3, 4, 5, 6, 8])
+def test_fp32_settings_are_read_once_per_build(harness, scenario, reads):
+    """Settings that another thread changes during a build (after `reads` reads):
+    every preparation and every launch goes by one value of each.  A launch with
+    a cutoff on lists prepared without one has no partner groups to read."""
+    r = harness(scenario, reads)
+    assert r["rc"] == 0 and r["launches"] in (2, 4), r  # one pass per kind, or two
+    assert r["null_groups"] == r["null_sums"] == r["cut_differs"] == 0, r

@@ -138,7 +138,7 @@ int prepare_jket(Arena& ar, const CoulombArgs& a, bool batched, bool hermite, bo
 // derivatives of J instead, written to a.mat_J[k * gstride + o], k = 0..5.
 template <int LA, int LB, int LC, int LD, int G = 0>
 int run_coulomb_impl(const CoulombArgs& a, cudaStream_t st, Arena& ar, const BoysTabs& tab,
-                     unsigned long long* qc, double cut, int64_t gstride = 0)
+                     unsigned long long* qc, const Fp32Settings& fp32, int64_t gstride = 0)
 {
     if (a.n_ab == 0 || a.n_cd == 0) return VLXB_OK;
     if (!a.mat_J || !a.cd_D || !a.ab_Q || !a.cd_Q || !a.ab_first || !a.ab_second || !a.ab_pdata || !a.cd_first ||
@@ -154,7 +154,7 @@ int run_coulomb_impl(const CoulombArgs& a, cudaStream_t st, Arena& ar, const Boy
     const int jvar = schedule_get(0, LA, LB, LC, LD);
     // the Rys and McMurchie-Davidson kernels read the Hermite ket density
     const bool hermite = G || j_rys(LA, LB, LC, LD) || jvar == 2;
-    const double budget = (cut > 0.0 && !G) ? fp32_budget_get() : 0.0;
+    const double cut = fp32.cut, budget = G ? 0.0 : fp32.budget;
     PairGroups gb;
     JKetData kd;
     int32_t* bmol = nullptr;
@@ -192,9 +192,10 @@ int run_coulomb(const CoulombArgs& a, cudaStream_t st)
     if (rc) return rc;
     const BoysTabs tab{boys_table_device(), boys_table32_device()};
     if (!tab.f64 || !tab.f32) return VLXB_ECUDA;
-    if (a.share) return run_coulomb_impl<LA, LB, LC, LD>(a, st, a.share->ar, tab, quartet_counters_device(), fp32_cut_get());
+    if (a.share)
+        return run_coulomb_impl<LA, LB, LC, LD>(a, st, a.share->ar, tab, quartet_counters_device(), a.share->fp32);
     Arena ar(st);
-    return run_coulomb_impl<LA, LB, LC, LD>(a, st, ar, tab, quartet_counters_device(), fp32_cut_get());
+    return run_coulomb_impl<LA, LB, LC, LD>(a, st, ar, tab, quartet_counters_device(), fp32_settings());
 }
 
 // Bra-centre derivatives of one Coulomb class: grad[k * gstride + o] +=
@@ -207,9 +208,10 @@ int run_coulomb_grad(const CoulombArgs& a, int64_t gstride, cudaStream_t st)
     if (rc) return rc;
     const BoysTabs tab{boys_table_device(), boys_table32_device()};
     if (!tab.f64 || !tab.f32) return VLXB_ECUDA;
-    if (a.share) return run_coulomb_impl<LA, LB, LC, LD, 1>(a, st, a.share->ar, tab, nullptr, fp32_cut_get(), gstride);
+    if (a.share)
+        return run_coulomb_impl<LA, LB, LC, LD, 1>(a, st, a.share->ar, tab, nullptr, a.share->fp32, gstride);
     Arena ar(st);
-    return run_coulomb_impl<LA, LB, LC, LD, 1>(a, st, ar, tab, nullptr, fp32_cut_get(), gstride);
+    return run_coulomb_impl<LA, LB, LC, LD, 1>(a, st, ar, tab, nullptr, fp32_settings(), gstride);
 }
 
 // Whether a pair of types is a side of some class whose FP32 quartets run on a
@@ -226,8 +228,8 @@ constexpr bool k_pair_contracted(int la, int lb)
 // partner groups where a class needs them and the error budget's prefix sums.
 template <int LX, int LY>
 int prepare_kpart(Arena& ar, const ExchangeArgs& a, const uint32_t* displs, const uint32_t* counts,
-                  const uint32_t* Dinds, const double* Q, const double* pdata, double cut, bool contracted,
-                  PairGroups& g)
+                  const uint32_t* Dinds, const double* Q, const double* pdata, const Fp32Settings& fp32,
+                  bool contracted, PairGroups& g)
 {
     constexpr int P = LX * 3 + LY, NX = ncart(LX), NY = ncart(LY);
     PrepShare* sh = a.share;
@@ -243,11 +245,11 @@ int prepare_kpart(Arena& ar, const ExchangeArgs& a, const uint32_t* displs, cons
     if (rc) return rc;
     rc = segment_records(ar, NX * NY, npx, npy, g, pdata);
     if (rc) return rc;
-    if (cut > 0.0 && (sh ? k_pair_contracted(LX, LY) : contracted)) {
+    if (fp32.cut > 0.0 && (sh ? k_pair_contracted(LX, LY) : contracted)) {
         rc = contract_groups(ar, npx, g, a.aoinds[LY], a.key_naos ? a.key_naos : a.naos);
         if (rc) return rc;
     }
-    if (cut > 0.0 && fp32_budget_get() > 0.0) {
+    if (fp32.budget > 0.0) {
         // after contract_groups: groups get their amplified sums too
         rc = budget_prefix_records(ar, g, npx, LY);
         if (rc) return rc;
@@ -261,7 +263,8 @@ int prepare_kpart(Arena& ar, const ExchangeArgs& a, const uint32_t* displs, cons
 
 // Output blocks and both sides' partner records of an exchange class.
 template <int LA, int LB, int LC, int LD>
-int prepare_exchange(Arena& ar, const ExchangeArgs& a, double cut, KOutData& ko, PairGroups& gab, PairGroups& gcd)
+int prepare_exchange(Arena& ar, const ExchangeArgs& a, const Fp32Settings& fp32, KOutData& ko, PairGroups& gab,
+                     PairGroups& gcd)
 {
     constexpr int P = LA * 3 + LC;
     constexpr bool CONTRACTED = k_rys(LA, LB, LC, LD) && k_contracted(LA, LB, LC, LD);
@@ -277,14 +280,14 @@ int prepare_exchange(Arena& ar, const ExchangeArgs& a, double cut, KOutData& ko,
             sh->has_kout[P] = true;
         }
     }
-    rc = prepare_kpart<LA, LB>(ar, a, a.displs_ab, a.counts_ab, a.Dinds_ab, a.Q_ab, a.pdata_ab, cut, CONTRACTED, gab);
+    rc = prepare_kpart<LA, LB>(ar, a, a.displs_ab, a.counts_ab, a.Dinds_ab, a.Q_ab, a.pdata_ab, fp32, CONTRACTED, gab);
     if (rc) return rc;
     if (LA == LC && LB == LD && a.Q_ab == a.Q_cd && a.Dinds_ab == a.Dinds_cd && a.displs_ab == a.displs_cd &&
         a.counts_ab == a.counts_cd && a.pdata_ab == a.pdata_cd) {
         gcd = gab;
         return VLXB_OK;
     }
-    return prepare_kpart<LC, LD>(ar, a, a.displs_cd, a.counts_cd, a.Dinds_cd, a.Q_cd, a.pdata_cd, cut, CONTRACTED, gcd);
+    return prepare_kpart<LC, LD>(ar, a, a.displs_cd, a.counts_cd, a.Dinds_cd, a.Q_cd, a.pdata_cd, fp32, CONTRACTED, gcd);
 }
 
 template <int LA, int LB, int LC, int LD>
@@ -302,14 +305,14 @@ int run_exchange(const ExchangeArgs& a, cudaStream_t st)
     if (rc) return rc;
     const BoysTabs tab{boys_table_device(), boys_table32_device()};
     if (!tab.f64 || !tab.f32) return VLXB_ECUDA;
-    const double cut = fp32_cut_get();
+    const Fp32Settings fp32 = a.share ? a.share->fp32 : fp32_settings();
+    const double cut = fp32.cut, budget = fp32.budget;
     Arena local(st);
     Arena& ar = a.share ? a.share->ar : local;
     KOutData ko;
     PairGroups gab, gcd;
-    rc = prepare_exchange<LA, LB, LC, LD>(ar, a, cut, ko, gab, gcd);
+    rc = prepare_exchange<LA, LB, LC, LD>(ar, a, fp32, ko, gab, gcd);
     if (rc) return rc;
-    const double budget = cut > 0.0 ? fp32_budget_get() : 0.0;
     [[maybe_unused]] KGroups kgab{}, kgcd{};
     if (k_rys(LA, LB, LC, LD) && k_contracted(LA, LB, LC, LD) && cut > 0.0) {
         kgab = KGroups{gab.gseg, gab.gq, gab.gbeg, gab.gcnt, gab.msp, gab.mq, gab.msu, gab.mmask, gab.gqa, gab.gqpre,
@@ -373,7 +376,7 @@ int run_exchange_grad(const ExchangeArgs& a, int64_t gstride, cudaStream_t st)
     Arena& ar = a.share ? a.share->ar : local;
     KOutData ko;
     PairGroups gab, gcd;
-    rc = prepare_exchange<LA, LB, LC, LD>(ar, a, 0.0, ko, gab, gcd);
+    rc = prepare_exchange<LA, LB, LC, LD>(ar, a, Fp32Settings{}, ko, gab, gcd);
     if (rc) return rc;
     if (ar.failed()) return VLXB_ENOMEM;
     if (a.share && a.share->prepare_only) return VLXB_OK;

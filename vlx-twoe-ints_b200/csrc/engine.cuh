@@ -146,6 +146,18 @@ int fp32_cut_set(double cut);
 // times hrr_amp on both pairs) stays within the budget runs in FP32.
 double fp32_budget_get();
 int fp32_budget_set(double budget);
+// Both settings as one call sees them: a call reads them once, so that lists
+// and kernels agree when another thread sets them meanwhile.
+struct Fp32Settings {
+    double cut = 0.0, budget = 0.0;
+};
+inline Fp32Settings fp32_settings()
+{
+    Fp32Settings f;
+    f.cut = fp32_cut_get();
+    if (f.cut > 0.0) f.budget = fp32_budget_get();
+    return f;
+}
 
 // Per-device counters of screened-in primitive shell quartets processed by
 // the J ([0]) and K ([1]) kernels (device memory, allocated with the table).
@@ -255,8 +267,9 @@ int launch_grid_limit();
 // (la * 3 + lb): a build has one J list per pair, one partner list per ordered
 // pair and one (i, k) list per pair, so 27 preparations serve its 90 classes.
 struct PrepShare {
-    explicit PrepShare(cudaStream_t s) : ar(s) {}
+    PrepShare(cudaStream_t s, const Fp32Settings& f) : ar(s), fp32(f) {}
     Arena ar;
+    Fp32Settings fp32;  // of the whole build
     bool has_jgrp[9] = {}, has_jbra[9] = {}, has_jket[9] = {}, has_kpart[9] = {}, has_kout[9] = {};
     PairGroups jgrp[9], jbra[9], kpart[9];
     int32_t* jmol[9] = {};

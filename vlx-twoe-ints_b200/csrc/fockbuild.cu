@@ -175,7 +175,7 @@ static int run_build(const VlxbFockBuild& b, PrepShare& share, Fork* fork, cudaS
 // call holds two such lists at a time, a shared build nine, which grows with
 // the square of the primitive count: 14 atoms 4s3p2d 0.1 GB, but a union of 64
 // molecules of 3 to 8 atoms 53 GB in FP64 and 157 GB in mixed precision.
-static uint64_t share_bytes(const VlxbFockBuild& b)
+static uint64_t share_bytes(const VlxbFockBuild& b, const Fp32Settings& fp32)
 {
     static const int pair_ab[6][2] = {{0, 0}, {0, 1}, {0, 2}, {1, 1}, {1, 2}, {2, 2}};
     bool kp[9] = {}, j[9] = {};
@@ -193,7 +193,7 @@ static uint64_t share_bytes(const VlxbFockBuild& b)
         const uint64_t nxy = (uint64_t)ncart(la) * ncart(lb), ntab = (uint64_t)b.prim_count[la] * b.prim_count[lb];
         if (kp[p]) {
             uint64_t rec = 60;  // records before and after the sort, S, list positions
-            if (fp32_cut_get() > 0.0) rec += (k_pair_contracted(la, lb) ? 150 : 0) + (fp32_budget_get() > 0.0 ? 32 : 0);
+            if (fp32.cut > 0.0) rec += (k_pair_contracted(la, lb) ? 150 : 0) + (fp32.budget > 0.0 ? 32 : 0);
             bytes += ntab * (130 + rec * nxy);
         }
         if (j[p]) bytes += ntab * 8 + std::min<uint64_t>(b.j_count[p], ntab) * (250 + 16 * (4 * nxy + 35));
@@ -210,9 +210,10 @@ constexpr uint64_t SHARE_MAX_BYTES = 40ull << 30;
 extern "C" int vlxb_fockBuild(const VlxbFockBuild* b, void* stream)
 {
     if (!b || b->n_mol < 0 || b->grad_stride > (uint64_t)INT64_MAX || (b->gradient && b->n_mol > 0)) return VLXB_EINVAL;
-    if (vlxb::share_bytes(*b) > vlxb::SHARE_MAX_BYTES) return VLXB_ENOMEM;
+    const vlxb::Fp32Settings fp32 = vlxb::fp32_settings();
+    if (vlxb::share_bytes(*b, fp32) > vlxb::SHARE_MAX_BYTES) return VLXB_ENOMEM;
     const cudaStream_t st = (cudaStream_t)stream;
-    vlxb::PrepShare share(st);
+    vlxb::PrepShare share(st, fp32);
     share.prepare_only = true;  // every list first: a call short of memory then leaves the outputs as they were
     int rc = vlxb::run_build(*b, share, nullptr, st);
     if (rc) return rc;

@@ -106,14 +106,14 @@ extern "C" int vlxb_computeCoulombFockSSSS_noalloc(
     if (rc) return rc;
     cudaStream_t st = (cudaStream_t)stream;
     const BoysTabs tab{d.boys64, d.boys32};
-    const double cut = fp32_cut_get();
+    const Fp32Settings fp32 = fp32_settings();
     {
         // size the call first: nothing is launched or allocated
         Arena probe(st, nullptr, NOALLOC_SCRATCH_BYTES, true);
-        rc = run_coulomb_impl<0, 0, 0, 0>(A, st, probe, tab, nullptr, cut);
+        rc = run_coulomb_impl<0, 0, 0, 0>(A, st, probe, tab, nullptr, fp32);
         if (rc) return rc;
         if (probe.used() > NOALLOC_SCRATCH_BYTES) return VLXB_ETOOBIG;
     }
     Arena ar(st, d.scratch, NOALLOC_SCRATCH_BYTES, false);
-    return run_coulomb_impl<0, 0, 0, 0>(A, st, ar, tab, nullptr, cut);
+    return run_coulomb_impl<0, 0, 0, 0>(A, st, ar, tab, nullptr, fp32);
 }

@@ -33,7 +33,11 @@ int group_flat(Arena&, int, int, int, int, const uint32_t*, const uint32_t*, int
                const double*, uint32_t, PairGroups&) { return VLXB_OK; }
 int group_csr(Arena&, int, int, int, int, const uint32_t*, const uint32_t*, const uint32_t*, int64_t, const double*,
               uint32_t, const double*, uint32_t, PairGroups&) { return VLXB_OK; }
-int make_records(Arena&, int, PairGroups&, const double*, int64_t) { return VLXB_OK; }
+static int g_prepared, g_short_at = -1;  // the preparation that runs out of memory
+int make_records(Arena&, int, PairGroups&, const double*, int64_t)
+{
+    return g_prepared++ == g_short_at ? VLXB_ENOMEM : VLXB_OK;
+}
 int segment_records(Arena&, int, int, int, PairGroups&, const double*) { return VLXB_OK; }
 int bra_record_mol(Arena&, const PairGroups&, const int32_t*, int32_t** mol)
 {
@@ -149,6 +153,12 @@ int main(int argc, char** argv)
         g_change_at = number;
         g_cut[0] = g_cut[1] = 1e-6;
         g_budget[1] = 0.2;
+    } else if (!strcmp(what, "launch fails")) {
+        g_cut[0] = g_cut[1] = 1e-6;
+        g_fail_at = number;
+        g_fail_rc = VLXB_ENOMEM;
+    } else if (!strcmp(what, "preparation fails")) {
+        g_short_at = number;
     }
     const int rc = vlxb_fockBuild(&b, nullptr);
     printf("rc %d\nlaunches %d\nnull_groups %d\nnull_sums %d\ncut_differs %d\n", rc, g_launches, g_null_groups,

@@ -34,3 +34,15 @@ def test_fp32_settings_are_read_once_per_build(harness, scenario, reads):
     r = harness(scenario, reads)
     assert r["rc"] == 0 and r["launches"] in (2, 4), r  # one pass per kind, or two
     assert r["null_groups"] == r["null_sums"] == r["cut_differs"] == 0, r
+
+
+@pytest.mark.parametrize("number", [0, 1, 2, 3])
+def test_memory_runs_out_before_or_after_the_first_launch(harness, number):
+    """VLXB_ENOMEM (3) tells the caller that no output was touched and that the
+    class calls may go on: so it comes from a preparation.  An allocation error
+    of a launch (of a kernel's first load, say) is VLXB_ECUDA (2), as other
+    classes have added to the outputs by then."""
+    r = harness("preparation fails", min(number, 2))  # three record lists, four launches
+    assert r["launches"] == 0 and r["rc"] == 3, r
+    r = harness("launch fails", number)
+    assert r["launches"] == number + 1 and r["rc"] == 2, r

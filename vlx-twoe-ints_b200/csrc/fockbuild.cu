@@ -221,5 +221,8 @@ extern "C" int vlxb_fockBuild(const VlxbFockBuild* b, void* stream)
     vlxb::Fork fork(*b, st);  // joined before the preparations are handed back on `st`
     rc = vlxb::run_build(*b, share, &fork, st);
     const int jc = fork.join();
-    return rc ? rc : jc;
+    if (!rc) rc = jc;
+    // a launch may fail for memory too (a kernel's code or stack): outputs have
+    // been added to by then, so it must not read as "nothing done"
+    return rc == VLXB_ENOMEM ? VLXB_ECUDA : rc;
 }

@@ -159,8 +159,16 @@ int main(int argc, char** argv)
         g_fail_rc = VLXB_ENOMEM;
     } else if (!strcmp(what, "preparation fails")) {
         g_short_at = number;
+    } else if (!strcmp(what, "batch")) {  // number: bits of what is missing
+        b.n_mol = 2;
+        if (!(number & 1)) b.prim_mol[1] = (const int32_t*)p;
+        if (!(number & 2)) b.prim_mol[2] = (const int32_t*)p;
+        if (!(number & 4)) b.maxD_mol[8] = (const double*)p;
+        if (number & 8) b.k_classes = 0;
+        if (number & 16) b.j_count[4] = 0;
     }
     const int rc = vlxb_fockBuild(&b, nullptr);
+    printf("prepared %d\n", g_prepared);
     printf("rc %d\nlaunches %d\nnull_groups %d\nnull_sums %d\ncut_differs %d\n", rc, g_launches, g_null_groups,
            g_null_sums, g_launch_cut_differs);
     printf("col_index %d\nstride %d\n", g_col_index, g_stride);

@@ -46,3 +46,17 @@ def test_memory_runs_out_before_or_after_the_first_launch(harness, number):
     assert r["launches"] == 0 and r["rc"] == 3, r
     r = harness("launch fails", number)
     assert r["launches"] == number + 1 and r["rc"] == 2, r
+
+
+@pytest.mark.parametrize("missing,rc", [
+    (0, 0), (1, 1), (2, 1), (4, 1),
+    (8, 0), (8 + 1, 1), (8 + 2, 1), (8 + 4, 0),  # Coulomb class alone: molecules of p and d primitives
+    (16 + 2, 0), (16 + 8 + 3, 0),                # an empty Coulomb list needs none
+])
+def test_batch_without_molecules_is_refused(harness, missing, rc):
+    """A batch (n_mol > 0) whose Coulomb classes have no molecule of their
+    primitives is refused as by vlxb_coulombBatch, before anything is queued:
+    without them every molecule would meet the kets of all others."""
+    r = harness("batch", missing)
+    assert r["rc"] == rc, r
+    assert rc == 0 or r["prepared"] == r["launches"] == 0, r

@@ -98,9 +98,28 @@ class Fork {
     bool used_[FORK_STREAMS] = {};
 };
 
+constexpr int pair_ab[6][2] = {{0, 0}, {0, 1}, {0, 2}, {1, 1}, {1, 2}, {2, 2}};
+
+// Whether a batch names the molecules that its classes ask for (as
+// vlxb_coulombBatch and vlxb_exchangeBatch; an empty Coulomb list asks for none).
+static bool batch_complete(const VlxbFockBuild& b)
+{
+    for (int x = 0; x < 6; x++) {
+        const int la = pair_ab[x][0], lb = pair_ab[x][1];
+        for (int y = 0; y < 6; y++) {
+            const int lc = pair_ab[y][0], ld = pair_ab[y][1];
+            if (((b.j_classes >> (x * 6 + y)) & 1ull) && b.j_count[la * 3 + lb] && b.j_count[lc * 3 + ld] &&
+                (!b.prim_mol[la] || !b.prim_mol[lc]))
+                return false;
+        }
+        for (int bd = 0; bd < 9; bd++)
+            if (((b.k_classes >> (x * 9 + bd)) & 1ull) && (!b.prim_mol[la] || !b.maxD_mol[bd])) return false;
+    }
+    return true;
+}
+
 static int run_build(const VlxbFockBuild& b, PrepShare& share, Fork* fork, cudaStream_t stream)
 {
-    static const int pair_ab[6][2] = {{0, 0}, {0, 1}, {0, 2}, {1, 1}, {1, 2}, {2, 2}};
     const bool batched = b.n_mol > 0;
     int bit = 0;
     for (int x = 0; x < 6; x++)
@@ -161,7 +180,6 @@ static int run_build(const VlxbFockBuild& b, PrepShare& share, Fork* fork, cudaS
             if (batched) {
                 A.prim_mol_a = b.prim_mol[la];
                 A.maxD_mol = b.maxD_mol[bd];
-                if (!A.prim_mol_a || !A.maxD_mol) return VLXB_EINVAL;
             }
             A.share = &share;
             const int rc = dispatch_exchange(la * 27 + lb * 9 + lc * 3 + ld, b.gradient != 0, A, (int64_t)b.grad_stride, st);
@@ -177,7 +195,6 @@ static int run_build(const VlxbFockBuild& b, PrepShare& share, Fork* fork, cudaS
 // molecules of 3 to 8 atoms 53 GB in FP64 and 157 GB in mixed precision.
 static uint64_t share_bytes(const VlxbFockBuild& b, const Fp32Settings& fp32)
 {
-    static const int pair_ab[6][2] = {{0, 0}, {0, 1}, {0, 2}, {1, 1}, {1, 2}, {2, 2}};
     bool kp[9] = {}, j[9] = {};
     for (int x = 0; x < 6; x++) {
         for (int y = 0; y < 6; y++)
@@ -210,6 +227,7 @@ constexpr uint64_t SHARE_MAX_BYTES = 40ull << 30;
 extern "C" int vlxb_fockBuild(const VlxbFockBuild* b, void* stream)
 {
     if (!b || b->n_mol < 0 || b->grad_stride > (uint64_t)INT64_MAX || (b->gradient && b->n_mol > 0)) return VLXB_EINVAL;
+    if (b->n_mol > 0 && !vlxb::batch_complete(*b)) return VLXB_EINVAL;
     const vlxb::Fp32Settings fp32 = vlxb::fp32_settings();
     if (vlxb::share_bytes(*b, fp32) > vlxb::SHARE_MAX_BYTES) return VLXB_ENOMEM;
     const cudaStream_t st = (cudaStream_t)stream;

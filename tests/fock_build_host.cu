@@ -165,7 +165,7 @@ int main(int argc, char** argv)
         if (!(number & 2)) b.prim_mol[2] = (const int32_t*)p;
         if (!(number & 4)) b.maxD_mol[8] = (const double*)p;
         if (number & 8) b.k_classes = 0;
-        if (number & 16) b.j_count[4] = 0;
+        if (number & 16) b.j_count[1 * 3 + 2] = 0;
     }
     const int rc = vlxb_fockBuild(&b, nullptr);
     printf("prepared %d\n", g_prepared);

@@ -166,6 +166,14 @@ int main(int argc, char** argv)
         if (!(number & 4)) b.maxD_mol[8] = (const double*)p;
         if (number & 8) b.k_classes = 0;
         if (number & 16) b.j_count[1 * 3 + 2] = 0;
+    } else if (!strcmp(what, "columns")) {  // number: n_mol
+        b.n_mol = number;
+        for (int l = 0; l < 3; l++) {
+            b.prim_mol[l] = (const int32_t*)p;
+            b.prim_aocols[l] = (const uint32_t*)(g_buffer + 8);
+        }
+        b.maxD_mol[8] = (const double*)p;
+        b.D_stride = 3;
     }
     const int rc = vlxb_fockBuild(&b, nullptr);
     printf("prepared %d\n", g_prepared);

@@ -60,3 +60,12 @@ def test_batch_without_molecules_is_refused(harness, missing, rc):
     r = harness("batch", missing)
     assert r["rc"] == rc, r
     assert rc == 0 or r["prepared"] == r["launches"] == 0, r
+
+
+def test_density_columns_and_stride_belong_to_a_batch(harness):
+    """prim_aocols and D_stride are read for n_mol > 0 alone (vlxb.h): one
+    molecule's density has the rows' indices and naos columns."""
+    r = harness("columns", 0)
+    assert (r["rc"], r["col_index"], r["stride"]) == (0, 0, 5), r
+    r = harness("columns", 2)
+    assert (r["rc"], r["col_index"], r["stride"]) == (0, 8, 3), r

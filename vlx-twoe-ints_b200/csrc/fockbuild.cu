@@ -164,13 +164,13 @@ static int run_build(const VlxbFockBuild& b, PrepShare& share, Fork* fork, cudaS
             for (int l = 0; l < 3; l++) {
                 A.info[l] = b.prim_info[l];
                 A.aoinds[l] = b.prim_aoinds[l];
-                A.aoinds_col[l] = b.prim_aocols[l];
+                if (batched) A.aoinds_col[l] = b.prim_aocols[l];
                 A.count[l] = b.prim_count[l];
             }
             A.maxD = b.maxD[bd];
             A.D = b.D;
             A.naos = b.naos;
-            A.D_stride = b.D_stride;
+            if (batched) A.D_stride = b.D_stride;
             A.Q_ab = b.kp_Q[p]; A.pdata_ab = b.kp_pdata[p]; A.Dinds_ab = b.kp_Dinds[p];
             A.displs_ab = b.kp_displs[p]; A.counts_ab = b.kp_counts[p];
             A.Q_cd = b.kp_Q[q]; A.pdata_cd = b.kp_pdata[q]; A.Dinds_cd = b.kp_Dinds[q];

@@ -1,0 +1,57 @@
+"""The build call and the class entry points beside stream capture and beside
+other streams' work."""
+import os
+import subprocess
+import sys
+
+import pytest
+
+torch = pytest.importorskip("torch")
+
+import helpers
+from vlxb import basis, fock, gradient, lists
+from vlxb._lib import lib
+
+pytestmark = pytest.mark.gpu
+HERE = os.path.dirname(os.path.abspath(__file__))
+
+# class calls of the kernels that read the root tables, each with its output
+CALLS = {
+    "exchange": lambda L, dl, out, s: L.exchange("dddd", fock.exchange_args(dl, "dddd", out, s, 0.0)),
+    "coulomb": lambda L, dl, out, s: L.coulomb("dddd", fock.coulomb_args(dl, "dddd", out, s)),
+    "gradient": lambda L, dl, out, s: L.coulomb_grad("dddd", gradient.grad_args(dl, "dddd", out, 0, out.shape[1], s)),
+    "fshell": lambda L, dl, out, s: L.coulomb("ffff", fock.coulomb_args(dl, "ffff", out, s)),
+}
+
+
+def capture_first_call(name):
+    """In a process of its own: vlxb_init, then the library's first launch under
+    capture; its replay has the bits of an eager call."""
+    L = lib()
+    L.init(0)
+    shells = {0: 1, 1: 1, 3: 1} if name == "fshell" else {0: 1, 1: 1, 2: 1}
+    wl = basis.config_custom(2, 3.0, shells, 1, 0.4, 3.0, 2, 1e-12, 3)
+    dl = fock.to_device(lists.build_lists(wl.mol, wl.D, wl.threshold, helpers.oracle_schwarz_fn))
+    key = "ff" if name == "fshell" else "dd"
+    n = (dl.kpair[key]["i"] if name == "exchange" else dl.j[key]["first"]).numel()
+    shape = (6, n) if name == "gradient" else (n,)
+    out = torch.zeros(shape, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        CALLS[name](L, dl, out, torch.cuda.current_stream().cuda_stream)
+    g.replay()
+    torch.cuda.synchronize()
+    ref = torch.zeros_like(out)
+    CALLS[name](L, dl, ref, torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    assert float(ref.abs().max()) > 0.0 and torch.equal(out, ref)
+
+
+@pytest.mark.parametrize("name", sorted(CALLS))
+def test_first_call_after_init_can_be_captured(name):
+    code = (f"import sys; sys.path[:0] = [{HERE!r}, {os.path.dirname(HERE)!r}, "
+            f"{os.path.join(os.path.dirname(HERE), 'vlx-twoe-ints_b200')!r}]; "
+            f"import test_gpu_fock_build as t; t.capture_first_call({name!r})")
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]

@@ -2,6 +2,7 @@
 #include <cuda_runtime.h>
 
 #include "engine.cuh"
+#include "rys.cuh"
 #include "../../include/vlxb.h"
 
 namespace vlxb {
@@ -38,7 +39,7 @@ int vlxb_init(int device)
     int rc = vlxb::ensure_pool_configured();
     if (rc) return rc;
     if (!vlxb::quartet_counters_device()) return VLXB_ECUDA;
-    return (vlxb::boys_table_device() && vlxb::boys_table32_device()) ? VLXB_OK : VLXB_ECUDA;
+    return (vlxb::boys_table_device() && vlxb::boys_table32_device() && vlxb::rys_table_device()) ? VLXB_OK : VLXB_ECUDA;
 }
 
 int vlxb_setFp32Cutoff(double cutoff) { return vlxb::fp32_cut_set(cutoff); }

@@ -125,6 +125,25 @@ class Arena {
         }                            \
     } while (0)
 
+// Device copy of a host table, complete when the call returns: cudaMemcpy may
+// return before its transfer from pageable memory ends, and kernels on
+// non-blocking streams would not wait for it.  Null on failure (no error left).
+inline void* upload_table(const void* host, size_t bytes)
+{
+    void* d = nullptr;
+    if (cudaMalloc(&d, bytes) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    if (cudaMemcpy(d, host, bytes, cudaMemcpyHostToDevice) != cudaSuccess ||
+        cudaStreamSynchronize(nullptr) != cudaSuccess) {
+        cudaGetLastError();
+        cudaFree(d);
+        return nullptr;
+    }
+    return d;
+}
+
 // Per-device FP64 Boys table (BOYS_NGRID x BOYS_NCOL), built on first use.
 // Returns nullptr on failure.  The first call on a device synchronises it
 // (table upload); call vlxb_init() before any stream capture.

@@ -7,6 +7,7 @@
 #include <mutex>
 
 #include "classes.cuh"
+#include "rys.cuh"
 #include "../../include/vlxb.h"
 
 namespace vlxb {
@@ -230,6 +231,7 @@ extern "C" int vlxb_fockBuild(const VlxbFockBuild* b, void* stream)
     if (b->n_mol > 0 && !vlxb::batch_complete(*b)) return VLXB_EINVAL;
     const vlxb::Fp32Settings fp32 = vlxb::fp32_settings();
     if (vlxb::share_bytes(*b, fp32) > vlxb::SHARE_MAX_BYTES) return VLXB_ENOMEM;
+    if (!vlxb::rys_table_device()) return VLXB_ECUDA;  // uploaded before any kernel of the build is queued
     const cudaStream_t st = (cudaStream_t)stream;
     vlxb::PrepShare share(st, fp32);
     share.prepare_only = true;  // every list first: a call short of memory then leaves the outputs as they were

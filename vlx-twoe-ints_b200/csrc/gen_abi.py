@@ -137,7 +137,7 @@ def header():
          "#ifdef __cplusplus", 'extern "C" {', "#endif", "",
          "#define VLXB_OK 0", "#define VLXB_EINVAL 1", "#define VLXB_ECUDA 2", "#define VLXB_ENOMEM 3",
          "#define VLXB_ETOOBIG 4", "",
-         "/* Select `device`, configure its memory pool and upload the Boys table.",
+         "/* Select `device`, configure its memory pool and upload the Boys and Rys tables.",
          "   Call once per device before any stream capture.  No reference",
          "   counterpart (the reference's caller owns its Boys table). */",
          "int vlxb_init(int device);", "",

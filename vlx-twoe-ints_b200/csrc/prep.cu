@@ -74,12 +74,8 @@ const float* boys_table32_device()
     std::vector<double> host;
     build_boys_host(host);
     std::vector<float> h32(host.begin(), host.end());
-    float* d = nullptr;
-    if (cudaMalloc(&d, h32.size() * sizeof(float)) != cudaSuccess) return nullptr;
-    if (cudaMemcpy(d, h32.data(), h32.size() * sizeof(float), cudaMemcpyHostToDevice) != cudaSuccess) {
-        cudaFree(d);
-        return nullptr;
-    }
+    float* d = (float*)upload_table(h32.data(), h32.size() * sizeof(float));
+    if (!d) return nullptr;
     std::lock_guard<std::mutex> lk(g_mu);
     if (g_boys32_dev[dev]) {
         cudaFree(d);
@@ -119,14 +115,8 @@ const double* boys_table_device()
     if (g_boys_dev[dev]) return g_boys_dev[dev];
     static std::vector<double> host;
     if (host.empty()) build_boys_host(host);
-    double* d = nullptr;
-    if (cudaMalloc(&d, host.size() * sizeof(double)) != cudaSuccess) return nullptr;
-    if (cudaMemcpy(d, host.data(), host.size() * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess) {
-        cudaFree(d);
-        return nullptr;
-    }
-    g_boys_dev[dev] = d;
-    return d;
+    g_boys_dev[dev] = (const double*)upload_table(host.data(), host.size() * sizeof(double));
+    return g_boys_dev[dev];
 }
 
 int ensure_pool_configured()

@@ -181,14 +181,8 @@ const double* rys_table_device()
     if (g_rys_dev[dev]) return g_rys_dev[dev];
     static std::vector<double> host;
     if (host.empty()) rys_host_table(host);
-    double* d = nullptr;
-    if (cudaMalloc(&d, host.size() * sizeof(double)) != cudaSuccess) return nullptr;
-    if (cudaMemcpy(d, host.data(), host.size() * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess) {
-        cudaFree(d);
-        return nullptr;
-    }
-    g_rys_dev[dev] = d;
-    return d;
+    g_rys_dev[dev] = (const double*)upload_table(host.data(), host.size() * sizeof(double));
+    return g_rys_dev[dev];
 }
 
 }  // namespace vlxb

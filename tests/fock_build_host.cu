@@ -8,6 +8,7 @@
 #include <string.h>
 
 #include "../vlx-twoe-ints_b200/csrc/fockbuild.cu"
+#include "../vlx-twoe-ints_b200/csrc/fork.cu"
 
 namespace vlxb {
 

@@ -24,6 +24,12 @@ CALLS = {
 }
 
 
+def system(atoms, shells, degree=1):
+    lib().init(0)
+    wl = basis.config_custom(atoms, 3.0, shells, degree, 0.4, 3.0, atoms, 1e-12, 3)
+    return wl, fock.to_device(lists.build_lists(wl.mol, wl.D, wl.threshold, fock.gpu_schwarz_fn()))
+
+
 def capture_first_call(name):
     """In a process of its own: vlxb_init, then the library's first launch under
     capture; its replay has the bits of an eager call."""
@@ -55,3 +61,28 @@ def test_first_call_after_init_can_be_captured(name):
             f"import test_gpu_fock_build as t; t.capture_first_call({name!r})")
     r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stderr[-2000:]
+
+
+def test_calls_on_two_streams_do_not_wait_for_each_other():
+    """A small build whose stream still has a long kernel before it holds up no
+    build of another stream (both run their classes on side streams)."""
+    _, dl = system(2, {0: 1, 1: 1, 2: 1})
+    busy, other = torch.cuda.Stream(), torch.cuda.Stream()
+    for s in (busy, other):  # first calls load kernels, which may wait for the device
+        with torch.cuda.stream(s):
+            ref = fock.build_jk(dl)
+    torch.cuda.synchronize()
+    end = torch.cuda.Event()
+    with torch.cuda.stream(busy):
+        torch.cuda._sleep(2_000_000_000)  # a second, ends by itself
+        end.record()
+        late = fock.build_jk(dl)
+    with torch.cuda.stream(other):
+        first = fock.build_jk(dl)
+    other.synchronize()
+    waited = end.query()
+    torch.cuda.synchronize()
+    assert not waited
+    for out in (late, first):
+        for part, r in zip(out, ref):
+            assert all(torch.equal(part[k], r[k]) for k in r)

@@ -4,9 +4,9 @@
 // distinct lists.  Here every list is prepared once: two atoms 1s1p1d, 4735
 // device operations and 22 ms per build become 284 and 1.1 ms.
 #include <algorithm>
-#include <mutex>
 
 #include "classes.cuh"
+#include "fork.cuh"
 #include "rys.cuh"
 #include "../../include/vlxb.h"
 
@@ -14,90 +14,6 @@ namespace vlxb {
 
 int dispatch_coulomb(int cls, bool grad, const CoulombArgs& a, int64_t gstride, cudaStream_t st);
 int dispatch_exchange(int cls, bool grad, const ExchangeArgs& a, int64_t gstride, cudaStream_t st);
-
-// Class kernels of a small build leave most of the device idle, so those of
-// different output lists (which share no output) run on four streams between
-// a fork and a join on the caller's stream; the classes of one list keep their
-// order and their stream, so results do not depend on it.
-constexpr int FORK_STREAMS = 4;
-// Builds of at most this many output entries fork.  Larger ones fill the
-// device with single kernels.
-constexpr uint64_t FORK_ENTRIES = 400000;
-
-// Streams of the current device (never captured: a capturing call does not
-// fork, so that calls of other threads may use them meanwhile).
-static cudaStream_t* fork_streams()
-{
-    static std::mutex mu;
-    static cudaStream_t pool[64][FORK_STREAMS];
-    static bool made[64] = {false};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
-    std::lock_guard<std::mutex> lk(mu);
-    if (!made[dev]) {
-        for (int k = 0; k < FORK_STREAMS; k++)
-            if (cudaStreamCreateWithFlags(&pool[dev][k], cudaStreamNonBlocking) != cudaSuccess) return nullptr;
-        made[dev] = true;
-    }
-    return pool[dev];
-}
-
-// Streams of the output lists of one build: group g runs on at(g).
-class Fork {
-  public:
-    Fork(const VlxbFockBuild& b, cudaStream_t st) : st_(st)
-    {
-        uint64_t entries = 0;
-        for (int p = 0; p < 9; p++) entries += (uint64_t)b.j_count[p] + b.k_count[p];
-        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-        if (entries > FORK_ENTRIES || cudaStreamIsCapturing(st, &cap) != cudaSuccess ||
-            cap != cudaStreamCaptureStatusNone)
-            return;
-        pool_ = fork_streams();
-        if (!pool_ || cudaEventCreateWithFlags(&start_, cudaEventDisableTiming) != cudaSuccess ||
-            cudaEventRecord(start_, st) != cudaSuccess)
-            pool_ = nullptr;
-    }
-    cudaStream_t at(int g)
-    {
-        if (!pool_) return st_;
-        const int k = g % FORK_STREAMS;
-        if (!used_[k]) {
-            if (cudaStreamWaitEvent(pool_[k], start_, 0) != cudaSuccess) return st_;
-            used_[k] = true;
-        }
-        return pool_[k];
-    }
-    // The caller's stream continues after every forked kernel.
-    int join()
-    {
-        int rc = VLXB_OK;
-        for (int k = 0; k < FORK_STREAMS; k++)
-            if (used_[k]) {
-                cudaEvent_t e = nullptr;
-                if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess ||
-                    cudaEventRecord(e, pool_[k]) != cudaSuccess || cudaStreamWaitEvent(st_, e, 0) != cudaSuccess) {
-                    // never leave work behind that the caller's stream does not wait for
-                    cudaStreamSynchronize(pool_[k]);
-                    rc = VLXB_ECUDA;
-                }
-                if (e) cudaEventDestroy(e);
-                used_[k] = false;
-            }
-        return rc;
-    }
-    ~Fork()
-    {
-        join();
-        if (start_) cudaEventDestroy(start_);
-    }
-
-  private:
-    cudaStream_t st_;
-    cudaStream_t* pool_ = nullptr;
-    cudaEvent_t start_ = nullptr;
-    bool used_[FORK_STREAMS] = {};
-};
 
 constexpr int pair_ab[6][2] = {{0, 0}, {0, 1}, {0, 2}, {1, 1}, {1, 2}, {2, 2}};
 
@@ -238,7 +154,9 @@ extern "C" int vlxb_fockBuild(const VlxbFockBuild* b, void* stream)
     int rc = vlxb::run_build(*b, share, nullptr, st);
     if (rc) return rc;
     share.prepare_only = false;
-    vlxb::Fork fork(*b, st);  // joined before the preparations are handed back on `st`
+    uint64_t outputs = 0;
+    for (int p = 0; p < 9; p++) outputs += (uint64_t)b->j_count[p] + b->k_count[p];
+    vlxb::Fork fork(st, outputs);  // joined before the preparations are handed back on `st`
     rc = vlxb::run_build(*b, share, &fork, st);
     const int jc = fork.join();
     if (!rc) rc = jc;

@@ -28,7 +28,7 @@ NVCC = os.environ.get("NVCC", "nvcc")
 ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ["-std=c++17", "-O3", "-lineinfo", "-Xcompiler", "-fPIC", "-Xptxas", "-v", "-I", CSRC] + ARCH_FLAGS
 
-HOST_HEADERS = ["common.cuh", "engine.cuh", "jk_kernels.cuh", "launch.cuh", "classes.cuh", "prep.cuh", "md.cuh"]
+HOST_HEADERS = ["common.cuh", "engine.cuh", "fork.cuh", "jk_kernels.cuh", "launch.cuh", "classes.cuh", "prep.cuh", "md.cuh"]
 CLASS_HEADERS = ["common.cuh", "engine.cuh", "jk_kernels.cuh", "launch.cuh", "class_launch.cuh", "col_kernels.cuh",
                  "md.cuh", "md_kernels.cuh", "tma.cuh", "jtma_kernels.cuh"]
 RYS_HEADERS = ["common.cuh", "engine.cuh", "jk_kernels.cuh", "launch.cuh", "rys.cuh", "krys_kernels.cuh"]
@@ -46,7 +46,7 @@ def _sources():
     srcs = [os.path.join(CSRC, "prep.cu"), os.path.join(CSRC, "api.cu"), os.path.join(CSRC, "schwarz.cu"),
             os.path.join(CSRC, "noalloc.cu"), os.path.join(CSRC, "aomap.cu"),
             os.path.join(CSRC, "listbuild.cu"), os.path.join(CSRC, "fshell.cu"), os.path.join(CSRC, "rys.cu"),
-            os.path.join(CSRC, "fockbuild.cu"),
+            os.path.join(CSRC, "fockbuild.cu"), os.path.join(CSRC, "fork.cu"),
             os.path.join(GEN, "abi.cu"), os.path.join(GEN, "drivers.cu")]
     srcs += sorted(glob.glob(os.path.join(GEN, "jrys_*.cu"))) + sorted(glob.glob(os.path.join(GEN, "kgrad_*.cu"))) + sorted(glob.glob(os.path.join(GEN, "krys_*.cu"))) + sorted(glob.glob(os.path.join(GEN, "cls_*.cu")))
     return srcs

@@ -86,3 +86,40 @@ def test_calls_on_two_streams_do_not_wait_for_each_other():
     for out in (late, first):
         for part, r in zip(out, ref):
             assert all(torch.equal(part[k], r[k]) for k in r)
+
+
+def test_f_shell_calls_take_no_stream_that_others_may_be_using():
+    """f-shell class calls run on side streams while another thread captures: a
+    stream of torch's pool, which hands the same 32 to everyone, may be the one
+    that is being captured."""
+    import threading
+
+    _, dl = system(2, {0: 1, 3: 1})
+    ref = fock.build_jk(dl)
+    torch.cuda.synchronize()
+    captured, mine = torch.cuda.Stream(), torch.cuda.Stream()
+    outs, errors = [], []
+
+    def builds():
+        try:
+            with torch.cuda.stream(mine):
+                for _ in range(10):  # at four streams a build, more than the pool has
+                    outs.append(fock.build_jk(dl))
+                mine.synchronize()
+        except Exception as e:  # noqa: BLE001 (handed to the test's thread)
+            errors.append(e)
+
+    x = torch.ones(8, device="cuda")
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=captured, capture_error_mode="thread_local"):
+        y = x + 1.0
+        t = threading.Thread(target=builds)
+        t.start()
+        t.join()
+    assert not errors, errors
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y, x + 1.0) and len(outs) == 10
+    for out in outs:
+        for part, r in zip(out, ref):
+            assert all(torch.equal(part[k], r[k]) for k in r)

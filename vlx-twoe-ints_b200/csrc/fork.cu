@@ -9,9 +9,11 @@
 #include "fork.cuh"
 
 #include <mutex>
+#include <new>
 #include <vector>
 
 #include "engine.cuh"
+#include "../../include/vlxb.h"
 
 namespace vlxb {
 
@@ -45,7 +47,8 @@ static void destroy(SideStreams* w)
 
 static SideStreams* create()
 {
-    SideStreams* w = new SideStreams;
+    SideStreams* w = new (std::nothrow) SideStreams;
+    if (!w) return nullptr;
     bool ok = cudaEventCreateWithFlags(&w->start, cudaEventDisableTiming) == cudaSuccess;
     for (int k = 0; ok && k < FORK_STREAMS; k++)
         ok = cudaStreamCreateWithFlags(&w->s[k], cudaStreamNonBlocking) == cudaSuccess &&
@@ -160,3 +163,24 @@ Fork::~Fork()
 }
 
 }  // namespace vlxb
+
+extern "C" void* vlxb_forkBegin(void* stream, uint64_t outputs)
+{
+    vlxb::Fork* f = new (std::nothrow) vlxb::Fork((cudaStream_t)stream, outputs);
+    if (f && f->forked()) return f;
+    delete f;
+    return nullptr;
+}
+
+extern "C" void* vlxb_forkStream(void* fork, int list)
+{
+    return fork && list >= 0 ? (void*)((vlxb::Fork*)fork)->at(list) : nullptr;
+}
+
+extern "C" int vlxb_forkJoin(void* fork)
+{
+    if (!fork) return VLXB_EINVAL;
+    const int rc = ((vlxb::Fork*)fork)->join();
+    delete (vlxb::Fork*)fork;
+    return rc;
+}

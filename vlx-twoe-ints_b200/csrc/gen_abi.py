@@ -327,6 +327,17 @@ def header():
          "    double omega, thr;",
          "} VlxbFockBuild;",
          "int vlxb_fockBuild(const VlxbFockBuild* build, void* stream);", "",
+         "/* Side streams for class calls of one small build (vlxb_fockBuild takes its",
+         "   own): calls that write different output lists may run beside one another.",
+         "   Begin forks from `stream` (outputs: entries of all output lists) and returns",
+         "   a handle, or NULL where a fork does not pay (large lists), is not possible or",
+         "   `stream` is being captured; Stream gives the stream of output list `list`",
+         "   (any number, the same one for calls of one list); Join makes the forked-from",
+         "   stream wait for them and ends the handle, which must not outlive that",
+         "   stream.  No reference counterpart. */",
+         "void* vlxb_forkBegin(void* stream, uint64_t outputs);",
+         "void* vlxb_forkStream(void* fork, int list);",
+         "int vlxb_forkJoin(void* fork);", "",
          "/* Allocation-free variant of vlxb_computeCoulombFockSSSS (same arguments,",
          "   same result) for callers that cannot allocate device memory, e.g. hosts",
          "   whose device memory is owned by their own allocator, or plugins that are",

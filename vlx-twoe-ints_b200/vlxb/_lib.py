@@ -133,6 +133,9 @@ class Lib:
                                                ctypes.c_void_p, ctypes.c_int32, ctypes.c_void_p, ctypes.c_void_p]
         c.vlxb_fockBuild.argtypes = [ctypes.c_void_p, ctypes.c_void_p]
         c.vlxb_fockBuild.restype = ctypes.c_int
+        c.vlxb_forkBegin.argtypes, c.vlxb_forkBegin.restype = [ctypes.c_void_p, ctypes.c_uint64], ctypes.c_void_p
+        c.vlxb_forkStream.argtypes, c.vlxb_forkStream.restype = [ctypes.c_void_p, ctypes.c_int], ctypes.c_void_p
+        c.vlxb_forkJoin.argtypes = [ctypes.c_void_p]
         for fn in (c.vlxb_coulombBatch, c.vlxb_exchangeBatch):
             fn.argtypes = [ctypes.c_int] * 4 + [ctypes.c_void_p, ctypes.c_void_p]
             fn.restype = ctypes.c_int

@@ -226,29 +226,23 @@ def build_jk(dl: DeviceLists, stream: torch.cuda.Stream | None = None, omega: fl
     return matJ, matK
 
 
-FORK_ENTRIES = 400000  # vlxb_fockBuild's bound: larger builds fill the device with single kernels
-
-
 def _fork(dl: DeviceLists, stream: torch.cuda.Stream, calls: int):
     """(at, join): at(list) is the stream (handle) for the class calls that
-    write one output list, four side streams in turn for small builds, else
-    `stream`; join() makes `stream` wait for them.  The calls of one list keep
-    their order; nothing is forked while a graph is captured."""
+    write one output list, side streams of the library's own in turn for small
+    builds (vlxb_forkBegin), else `stream`; join() makes `stream` wait for them.
+    The calls of one list keep their order."""
+    L = lib()
     entries = sum(v["first"].numel() for v in dl.j.values()) + sum(v["i"].numel() for v in dl.kpair.values())
-    if calls < 2 or entries > FORK_ENTRIES or torch.cuda.is_current_stream_capturing():
+    fork = L.cdll.vlxb_forkBegin(stream.cuda_stream, entries) if calls > 1 else None
+    if fork is None:
         return (lambda key: stream.cuda_stream), (lambda: None)
-    side, keys, start = {}, {}, stream.record_event()
+    keys = {}
 
     def at(key):
-        k = keys.setdefault(key, len(keys)) % 4
-        if k not in side:
-            side[k] = torch.cuda.Stream(device=dl.device)
-            side[k].wait_event(start)
-        return side[k].cuda_stream
+        return L.cdll.vlxb_forkStream(fork, keys.setdefault(key, len(keys))) or 0
 
     def join():
-        for st in side.values():
-            stream.wait_stream(st)
+        L.check(L.cdll.vlxb_forkJoin(fork), "vlxb_forkJoin")
 
     return at, join
 

@@ -123,3 +123,29 @@ def test_f_shell_calls_take_no_stream_that_others_may_be_using():
     for out in outs:
         for part, r in zip(out, ref):
             assert all(torch.equal(part[k], r[k]) for k in r)
+
+
+@pytest.mark.parametrize("what", ["build", "coulomb gradient", "exchange gradient"])
+def test_fresh_outputs_are_zeroed_before_another_stream_adds_to_them(what):
+    """Outputs made by the call are zeroed on the current stream, here a late
+    one, and added to on the stream that is asked for."""
+    wl, dl = system(2, {0: 1, 1: 1, 2: 1})
+    side = torch.cuda.Stream()
+    cg, kg = gradient.CoulombGradient(dl, wl.mol), gradient.ExchangeGradient(dl, wl.mol)
+
+    def call(stream):
+        if what == "build":
+            J, K = fock.build_jk(dl, stream=stream)
+            return [J[k] for k in sorted(J)] + [K[k] for k in sorted(K)]
+        if what == "coulomb gradient":
+            return [gradient.pair_gradients(dl, cg.map, stream=stream)]
+        return [gradient.exchange_pair_gradients(dl, kg.map, stream=stream)]
+
+    ref = call(torch.cuda.current_stream())
+    torch.cuda.synchronize()
+    with torch.cuda.stream(torch.cuda.Stream()):
+        torch.cuda._sleep(400_000_000)
+        out = call(side)
+    torch.cuda.synchronize()
+    assert any(float(r.abs().max()) > 0.0 for r in ref)
+    assert all(torch.equal(a, b) for a, b in zip(out, ref))

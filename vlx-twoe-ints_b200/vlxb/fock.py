@@ -199,12 +199,12 @@ def build_jk(dl: DeviceLists, stream: torch.cuda.Stream | None = None, omega: fl
     if stream is None:
         stream = torch.cuda.current_stream(dl.device)
     s = stream.cuda_stream
-    if matJ is None or matK is None:
-        matJ, matK = alloc_outputs(dl)
     jcls = [c for c in ((j_only or j_classes_all()) if do_j else []) if c[:2] in dl.j and c[2:] in dl.j]
     kcls = [c for c in ((k_only or k_classes_all()) if do_k else [])
             if c[0] + c[2] in dl.kpair and c[:2] in dl.kpart and c[2:] in dl.kpart]
     with torch.cuda.stream(stream):
+        if matJ is None or matK is None:
+            matJ, matK = alloc_outputs(dl)  # zeroed on the stream that adds to them
         spd = [c for c in jcls if "f" not in c], [c for c in kcls if "f" not in c]
         if len(spd[0]) == len(set(spd[0])) and len(spd[1]) == len(set(spd[1])):  # a mask holds a class once
             b = build_call(dl, omega)

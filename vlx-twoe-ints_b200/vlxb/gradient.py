@@ -139,9 +139,9 @@ def pair_gradients(dl: DeviceLists, gmap: GradientMap, stream=None, classes=None
     the J classes (all 36 by default), through the class entry points."""
     L = lib()
     st = stream or torch.cuda.current_stream(dl.device)
-    G = torch.zeros((6, max(gmap.total, 1)), dtype=torch.float64, device=dl.device)
     run = [c for c in (classes or j_classes()) if c[:2] in dl.j and c[2:] in dl.j]
     with torch.cuda.stream(st):
+        G = torch.zeros((6, max(gmap.total, 1)), dtype=torch.float64, device=dl.device)
         if len(run) == len(set(run)):  # a mask holds a class once
             b = build_call(dl)
             b.gradient, b.grad_stride = 1, G.shape[1]
@@ -160,10 +160,10 @@ def exchange_pair_gradients(dl: DeviceLists, kmap: GradientMap, stream=None, ome
     space, summed over the K classes (all 54 by default)."""
     L = lib()
     st = stream or torch.cuda.current_stream(dl.device)
-    G = torch.zeros((6, max(kmap.total, 1)), dtype=torch.float64, device=dl.device)
     run = [c for c in (classes or k_classes())
            if c[0] + c[2] in dl.kpair and c[:2] in dl.kpart and c[2:] in dl.kpart]
     with torch.cuda.stream(st):
+        G = torch.zeros((6, max(kmap.total, 1)), dtype=torch.float64, device=dl.device)
         if len(run) == len(set(run)):
             b = build_call(dl, omega)
             b.gradient, b.grad_stride = 1, G.shape[1]

@@ -11,6 +11,7 @@ from __future__ import annotations
 
 import argparse
 import concurrent.futures as cf
+import functools
 import glob
 import os
 import subprocess
@@ -28,13 +29,6 @@ NVCC = os.environ.get("NVCC", "nvcc")
 ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ["-std=c++17", "-O3", "-lineinfo", "-Xcompiler", "-fPIC", "-Xptxas", "-v", "-I", CSRC] + ARCH_FLAGS
 
-HOST_HEADERS = ["common.cuh", "engine.cuh", "fork.cuh", "jk_kernels.cuh", "launch.cuh", "classes.cuh", "prep.cuh", "md.cuh"]
-CLASS_HEADERS = ["common.cuh", "engine.cuh", "jk_kernels.cuh", "launch.cuh", "class_launch.cuh", "col_kernels.cuh",
-                 "md.cuh", "md_kernels.cuh", "tma.cuh", "jtma_kernels.cuh"]
-RYS_HEADERS = ["common.cuh", "engine.cuh", "jk_kernels.cuh", "launch.cuh", "rys.cuh", "krys_kernels.cuh"]
-GRAD_HEADERS = RYS_HEADERS + ["kgrad_kernels.cuh"]
-JRYS_HEADERS = ["common.cuh", "engine.cuh", "jk_kernels.cuh", "launch.cuh", "rys.cuh", "md.cuh", "jrys_kernels.cuh"]
-
 
 def _run_generators():
     subprocess.run([sys.executable, os.path.join(CSRC, "gen_quartets.py"), GEN], check=True)
@@ -48,26 +42,35 @@ def _sources():
             os.path.join(CSRC, "listbuild.cu"), os.path.join(CSRC, "fshell.cu"), os.path.join(CSRC, "rys.cu"),
             os.path.join(CSRC, "fockbuild.cu"), os.path.join(CSRC, "fork.cu"),
             os.path.join(GEN, "abi.cu"), os.path.join(GEN, "drivers.cu")]
-    srcs += sorted(glob.glob(os.path.join(GEN, "jrys_*.cu"))) + sorted(glob.glob(os.path.join(GEN, "kgrad_*.cu"))) + sorted(glob.glob(os.path.join(GEN, "krys_*.cu"))) + sorted(glob.glob(os.path.join(GEN, "cls_*.cu")))
+    for kind in ("jrys", "kgrad", "krys", "cls"):
+        srcs += sorted(glob.glob(os.path.join(GEN, f"{kind}_*.cu")))
     return srcs
 
 
+@functools.lru_cache(maxsize=None)
+def _included(path, mtime):
+    """Files that `path` includes by a quoted name, where the compiler looks for them."""
+    out = []
+    with open(path) as fh:
+        for ln in fh:
+            if ln.startswith("#include \""):
+                name = ln.split('"')[1]
+                for base in (os.path.dirname(path), CSRC):
+                    p = os.path.normpath(os.path.join(base, name))
+                    if os.path.exists(p):
+                        out.append(p)
+                        break
+    return out
+
+
 def _deps(src):
-    base = os.path.basename(src)
-    if base.startswith("jrys_"):
-        return [src] + [os.path.join(CSRC, h) for h in JRYS_HEADERS]
-    if base.startswith("kgrad_"):
-        return [src] + [os.path.join(CSRC, h) for h in GRAD_HEADERS]
-    if base.startswith(("krys_", "rys")):
-        return [src] + [os.path.join(CSRC, h) for h in RYS_HEADERS]
-    deps = [src, os.path.join(GEN, "hrr_pairs.cuh"), os.path.join(REPO_ROOT, "include", "vlxb.h")]
-    deps += [os.path.join(CSRC, h) for h in (CLASS_HEADERS if base.startswith("cls_") else HOST_HEADERS)]
-    if base.startswith("cls_"):
-        deps.append(os.path.join(GEN, f"col_{base.split('_')[1]}.cuh"))
-        with open(src) as fh:  # every generated quartet header the unit includes (its class first)
-            deps += [os.path.join(GEN, ln.split('"')[1]) for ln in fh if ln.startswith('#include "q_')]
-    if base == "prep.cu":
-        deps.append(os.path.join(GEN, "schedule_default.inc"))
+    """The source and every file that it includes, directly or not."""
+    deps, todo = [], [os.path.normpath(src)]
+    while todo:
+        p = todo.pop()
+        if p not in deps:
+            deps.append(p)
+            todo += _included(p, os.path.getmtime(p))
     return deps
 
 

@@ -16,8 +16,8 @@
 // registers (eri_component), rho' = rho for the Coulomb operator and
 // rho w^2 / (rho + w^2) for the attenuated one.  Two atoms 1s1p1d1f (170 f class
 // calls and the s/p/d ones): 209 ms with a Hermite box per component in local
-// memory, 45 ms so, 27 ms with four blocks per SM and wide blocks for short
-// lists, 21 ms with the class calls on side streams.
+// memory, 20.8 ms with a recurrence table per root and direction, 6.2 ms with
+// the pairs' Hermite coefficients folded before the roots (eri_component).
 // Screening is the reference's per-component predicate
 // (|Q_ij Q_kl D_kl| > thr for J, |Q_ij Q_kl max_D| > thr for K), the J ket
 // weights gen_coulomb.py:276-281, the K density gather gen_exchange.py:323.
@@ -34,7 +34,7 @@ namespace vlxb {
 constexpr int FS_THREADS = 128;
 constexpr int FS_WIDE = 512;                // threads per entry of lists too short to fill the device
 constexpr int FS_LMAX = 3;                  // f
-constexpr int FS_N = 2 * FS_LMAX + 1;     // rows and columns of a 1-D table: exponents 0..6 per pair
+constexpr int FS_N = 2 * FS_LMAX + 1;     // 1-D Hermite coefficients of a pair: exponents 0..6
 constexpr int FS_NR = RYS_MAX;            // roots of an (FF|FF) quartet
 
 struct FPrim {
@@ -61,100 +61,91 @@ __device__ __forceinline__ FPrim fprim(const double* __restrict__ info, uint32_t
     return f;
 }
 
-// Coefficients of the 1-D shift (x, y) = sum_n cf[n] (n, 0):
-// binomial(y, n - x) R^(y - n + x), 0 outside n = x .. x + y (y <= 3).
-__device__ __forceinline__ void fs_shift(int x, int y, double R, double* cf)
+// 1-D Hermite coefficients E^{ij}_t of one pair, t = 0..i + j (0 above), raised
+// on the first centre, then on the second (md.cuh's recurrence; indices of
+// arrays are constants throughout).
+__device__ __forceinline__ void fs_hermite(int i, int j, double PA, double PB, double h, double* e)
 {
-    const double R2 = R * R, R3 = R2 * R;
 #pragma unroll
-    for (int n = 0; n < FS_N; n++) {
-        const int k = n - x, j = y - k;
-        double c = j == 0 ? 1.0 : (j == 1 ? R : (j == 2 ? R2 : R3));
-        if ((y == 3 && (k == 1 || k == 2))) c *= 3.0;
-        else if (y == 2 && k == 1) c *= 2.0;
-        cf[n] = k >= 0 && j >= 0 ? c : 0.0;
+    for (int t = 0; t < FS_N; t++) e[t] = t == 0 ? 1.0 : 0.0;
+#pragma unroll
+    for (int k = 0; k < FS_N - 1; k++) {
+        if (k >= i + j) break;
+        const double X = k < i ? PA : PB;
+        double prev = 0.0;  // e[t - 1] before this step
+#pragma unroll
+        for (int t = 0; t <= k + 1; t++) {
+            const double cur = e[t];
+            double v = fma(h, prev, X * cur);
+            if (t + 1 <= k) v = fma((double)(t + 1), e[t + 1], v);
+            prev = cur;
+            e[t] = v;
+        }
     }
 }
 
 // (ab|cd) / (S_ab S_cd) of one Cartesian component quartet by Rys quadrature:
-// per direction the 2-D integrals (a b; c d) at every root, as the shifts of
-// the recurrence table V(n, m), built column by column in registers (indices of
-// arrays are constants throughout; nab, ncd = la + lb, lc + ld bound the rows,
-// and columns stop at c + d).  About a quarter of the operations of the Hermite
-// box it replaces and no local memory.
+// per direction the integral at a root is sum_s G_s H_s, with the product of
+// both pairs' Hermite coefficients G_{t+u} = sum E_t E'_u (-1)^u, which no root
+// changes, and H_0 = 1, H_{s+1} = -2 rho x (PQ H_s + s H_{s-1}).  The pairs'
+// centres enter through P - A and P - B as they are: a recurrence on A shifted
+// to B by powers of A - B loses the digits of a tight b far from a diffuse a
+// (5e-11 of the Schwarz bound, root mean square, for exponents 0.05 to 50 on
+// two centres in a box of 6 bohr; this form 1.2e-16, a Hermite box 6e-16).
 __device__ double eri_component(const FPrim& A, const FPrim& B, const FPrim& C, const FPrim& D, int nab, int ncd,
                                 double omega, const double* __restrict__ rtab)
 {
     const double p = A.alpha + B.alpha, q = C.alpha + D.alpha;
-    const double ip = 1.0 / p, iq = 1.0 / q, inv = 1.0 / (p + q);
-    const double rho = p * q * inv;
+    const double ip = 1.0 / p, iq = 1.0 / q;
+    const double rho = p * q / (p + q);
     const double d2 = omega != 0.0 ? omega * omega / (rho + omega * omega) : 1.0;
     const double rp = rho * d2;
-    double PA[3], QC[3], PQ[3], r2 = 0.0;
+    double PQ[3], r2 = 0.0;
 #pragma unroll
     for (int x = 0; x < 3; x++) {
-        PA[x] = -B.alpha * ip * (A.r[x] - B.r[x]);
-        QC[x] = -D.alpha * iq * (C.r[x] - D.r[x]);
-        PQ[x] = (QC[x] + C.r[x]) - (PA[x] + A.r[x]);
+        PQ[x] = (A.r[x] - B.alpha * ip * (A.r[x] - B.r[x])) - (C.r[x] - D.alpha * iq * (C.r[x] - D.r[x]));
         r2 = fma(PQ[x], PQ[x], r2);
     }
     const int nr = (nab + ncd) / 2 + 1;
-    double x2[FS_NR], prod[FS_NR];
+    double m2[FS_NR], prod[FS_NR];  // -2 rho x, and the product of the weight and the directions so far
 #pragma unroll
     for (int r = 0; r < FS_NR; r++) {
+        m2[r] = prod[r] = 0.0;
         if (r < nr) {
-            double xr, wr;
-            rys_root_rt(nr, rp * r2, rtab, r, xr, wr);
-            x2[r] = xr * d2;
-            prod[r] = wr;
-        } else {
-            x2[r] = prod[r] = 0.0;
+            rys_root_rt(nr, rp * r2, rtab, r, m2[r], prod[r]);
+            m2[r] *= -2.0 * rp;
         }
     }
 #pragma unroll
     for (int x = 0; x < 3; x++) {
-        const int mc = C.c[x] + D.c[x];
-        double cb[FS_N], cd[FS_N];
-        fs_shift(A.c[x], B.c[x], A.r[x] - B.r[x], cb);
-        fs_shift(C.c[x], D.c[x], C.r[x] - D.r[x], cd);
+        const double ab = A.r[x] - B.r[x], cd = C.r[x] - D.r[x];
+        const int na = A.c[x] + B.c[x], nc = C.c[x] + D.c[x];
+        double e[FS_N], f[FS_N], G[2 * FS_N - 1];
+        fs_hermite(A.c[x], B.c[x], -B.alpha * ip * ab, A.alpha * ip * ab, 0.5 * ip, e);
+        fs_hermite(C.c[x], D.c[x], -D.alpha * iq * cd, C.alpha * iq * cd, 0.5 * iq, f);
+#pragma unroll
+        for (int s = 0; s < 2 * FS_N - 1; s++) G[s] = 0.0;
+#pragma unroll
+        for (int u = 0; u < FS_N; u++) {
+            if (u > nc) break;
+            const double g = (u & 1) ? -f[u] : f[u];
+#pragma unroll
+            for (int t = 0; t < FS_N; t++)
+                if (t <= na) G[t + u] = fma(e[t], g, G[t + u]);
+        }
 #pragma unroll
         for (int r = 0; r < FS_NR; r++) {
             if (r >= nr) break;
-            const double zx = q * inv * x2[r], ex = p * inv * x2[r];
-            const double B10 = 0.5 * ip * (1.0 - zx), B01 = 0.5 * iq * (1.0 - ex), B00 = 0.5 * inv * x2[r];
-            const double Cx = fma(zx, PQ[x], PA[x]), Dx = fma(-ex, PQ[x], QC[x]);
-            double v[FS_N], w[FS_N];  // columns m and m - 1
-            v[0] = 1.0;
-            v[1] = Cx;
-            double s = fma(cb[1], v[1], cb[0]);
+            double h = 1.0, h1 = m2[r] * PQ[x], s = G[0];  // H_{s-1}, H_s
 #pragma unroll
-            for (int n = 2; n < FS_N; n++) {
-                v[n] = 0.0;
-                if (n <= nab) {
-                    v[n] = fma(Cx, v[n - 1], (n - 1) * B10 * v[n - 2]);
-                    s = fma(cb[n], v[n], s);
-                }
+            for (int n = 1; n < 2 * FS_N - 1; n++) {
+                if (n > na + nc) break;
+                s = fma(G[n], h1, s);
+                const double h2 = m2[r] * fma(PQ[x], h1, n * h);
+                h = h1;
+                h1 = h2;
             }
-#pragma unroll
-            for (int n = 0; n < FS_N; n++) w[n] = 0.0;
-            double sum = cd[0] * s;
-#pragma unroll
-            for (int m = 1; m < FS_N; m++) {
-                if (m > mc) break;
-                double prev = 0.0;  // v[n - 1] of the column before this one
-                s = 0.0;
-#pragma unroll
-                for (int n = 0; n < FS_N; n++) {
-                    if (n > nab) break;
-                    const double t = fma(Dx, v[n], fma((m - 1) * B01, w[n], n * B00 * prev));
-                    prev = v[n];
-                    w[n] = v[n];
-                    v[n] = t;
-                    s = fma(cb[n], t, s);
-                }
-                sum = fma(cd[m], s, sum);
-            }
-            prod[r] *= sum;
+            prod[r] *= s;
         }
     }
     double sum = 0.0;
@@ -191,9 +182,9 @@ struct FShellJ {
     double thr;
 };
 
-// 128 registers: four blocks of 128 threads per SM or one of 512.  The spills
-// they cost (300 bytes) are repaid by the warps: 170 f class calls of two atoms
-// 1s1p1d1f, 239 registers 43.5 ms, 168 35.5, 128 31.2.
+// 128 registers: four blocks of 128 threads per SM or one of 512 (the spills,
+// 690 bytes here and 80 in the exchange kernel, are mostly the bra's
+// coefficients, which no ket changes).
 __global__ void __launch_bounds__(FS_WIDE, 1)
 coulomb_fshell_kernel(FShellJ a, double* __restrict__ mat_J, const double* __restrict__ tab)
 {

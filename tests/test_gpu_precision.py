@@ -55,3 +55,67 @@ def test_f_coulomb_keeps_its_digits(alpha0, ratio, side):
             bound += abs(w) * float(jl.Q[e]) * float(jl.Q[k])
         err = abs(float(exact - float(got[e])))
         assert bound > 0.0 and err <= 32 * EPS * bound, (e, got[e], err / (EPS * bound))
+
+
+def thin(kp, per_row):
+    """At most `per_row` seeded partners of every row of a partner list."""
+    keep = []
+    for i, (d, c) in enumerate(zip(kp.displs.astype(np.int64), kp.counts.astype(np.int64))):
+        keep.append(np.sort(d + np.random.default_rng(i + 200).choice(c, min(per_row, c), replace=False)))
+    kp.counts = np.array([len(k) for k in keep], dtype=kp.counts.dtype)
+    kp.displs = np.concatenate([[0], np.cumsum(kp.counts[:-1].astype(np.int64))]).astype(kp.displs.dtype)
+    for n in ("Dinds", "Q", "pdata"):
+        setattr(kp, n, np.ascontiguousarray(getattr(kp, n)[np.concatenate(keep)]))
+
+
+# limit: roundings of the bound, two to three times the largest of the same
+# blocks by the Hermite recurrences (46, 4, 8 and 5)
+@pytest.mark.parametrize("cls,alpha0,ratio,side,limit", [
+    ("sdsd", 0.1, 50.0, 2.0, 128), ("dddd", 0.05, 1000.0, 6.0, 16), ("pddd", 0.05, 1000.0, 6.0, 24),
+    ("dddd", 0.05, 2.5, 6.0, 16),
+])
+def test_exchange_gradient_keeps_its_digits(cls, alpha0, ratio, side, limit):
+    """Blocks of one (i, k) entry and two partners a side; the bound of a
+    derivative is the Schwarz bound of the raised and lowered functions."""
+    from vlxb import gradient
+
+    _, rl = system({0: 1, 1: 1, 2: 1}, alpha0, ratio, side)
+    la, lb, lc, ld = (lists.LV[x] for x in cls)
+    ac, kab, kcd = cls[0] + cls[2], rl.kpartners[cls[:2]], rl.kpartners[cls[2:]]
+    thin(kab, 2)
+    if kcd is not kab:
+        thin(kcd, 2)
+    dl = fock.to_device(rl)
+    kq = rl.kpairs[ac]
+    rows = np.random.default_rng(3).choice(len(kq.pair_i), 6, replace=False)
+    ao = lambda l, idx: int(rl.pd.aoinds[l][int(idx) % len(CART[l]), int(idx) // len(CART[l])])  # noqa: E731
+    root = lambda f, u, v: float(f(u, v, u, v)) ** 0.5  # noqa: E731
+    worst = 0.0
+    for r in rows:
+        i, k = int(kq.pair_i[r]), int(kq.pair_k[r])
+        dl.kpair[ac] = {n: torch.tensor([v], dtype=torch.int32, device="cuda") for n, v in (("i", i), ("k", k))}
+        G = torch.zeros((6, 1), dtype=torch.float64, device="cuda")
+        lib().exchange_grad(cls, gradient.kgrad_args(dl, cls, G, 0, 1, torch.cuda.current_stream().cuda_stream))
+        got, exact, bound = G.cpu().numpy()[:, 0], [mp_integrals.mp.mpf(0)] * 6, np.zeros(6)
+        wik = (1.0 if la == lc and i == k else 2.0) * rl.D_AO[ao(la, i), ao(lc, k)]
+        for tj in range(int(kab.displs[i]), int(kab.displs[i]) + int(kab.counts[i])):
+            for tl in range(int(kcd.displs[k]), int(kcd.displs[k]) + int(kcd.counts[k])):
+                j, l = int(kab.Dinds[tj]), int(kcd.Dinds[tl])
+                prims, comps = zip(prim(rl, la, i), prim(rl, lb, j), prim(rl, lc, k), prim(rl, ld, l))
+                w = float(wik * rl.D_AO[ao(lb, j), ao(ld, l)] * kab.pdata[tj] * kcd.pdata[tl])
+                grad = mp_integrals.quartet(prims)[1]
+                for c in (0, 2):
+                    f, o = (mp_integrals.quartet(prims[s:s + 2] * 2)[0] for s in (c, 2 - c))
+                    other = root(o, *comps[2 - c:4 - c])
+                    for x in range(3):
+                        u = [tuple(v + s * (t == x) for t, v in enumerate(comps[c])) for s in (1, -1)]
+                        s = 2.0 * float(prims[c][0]) * root(f, u[0], comps[c + 1])
+                        if comps[c][x]:
+                            s += comps[c][x] * root(f, u[1], comps[c + 1])
+                        at = x if c == 0 else 3 + x
+                        exact[at] += w * grad(c, x, *comps)
+                        bound[at] += abs(w) * s * other
+        for x in range(6):
+            if bound[x] > 0.0:
+                worst = max(worst, abs(float(exact[x] - float(got[x]))) / (EPS * bound[x]))
+    assert 0.0 < worst <= limit, worst

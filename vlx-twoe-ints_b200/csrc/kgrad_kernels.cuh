@@ -53,44 +53,78 @@ struct KGradShape {
     static constexpr int SMEM = 3 * N1 * M1 * THREADS * 8;
 };
 
-// v[m], m < NM: the shift of V(a, .) to b exponent bx (krys_row).
-template <int LB, int M1, int NM, int TH>
-__device__ __forceinline__ void kgrad_shift(const double* V, int a, int bx, double R, double* v)
+// Shifts between the centres of a pair.  The recurrence is on the centre of the
+// tighter shell: the exponent `near` on it and `far` on the other centre are
+// sum_k binomial(far, k) R^(far - k) V(near + k), R = near centre - far centre,
+// whose terms do not cancel as P is nearer to the near centre.  From a diffuse a
+// to a tight b two shifts cancel: blocks of (SD|SD), exponents 0.1 and 5 at 2
+// bohr, were 304 roundings off in units of the bound where the Hermite tables
+// before were 16 (as here).  One shift costs no more than P - B = (P - A) + (A -
+// B) does anyway ((PP|PP): 8 either way), so s and p shells b (d) keep a (c).
+// 5 atoms 4s3p2d: 55 -> 59 ms.
+//
+// v[m], m < NM, for the exponents a and b; `swap`: the recurrence is on b.
+template <int LA, int LB, int M1, int NM, int TH>
+__device__ __forceinline__ void kgrad_shift(const double* V, bool swap, int a, int b, double R, double* v)
 {
-    const double* p = V + a * M1 * TH;
-    if (LB == 0 || bx == 0) {
+    // lanes of a warp mostly agree in `swap`: their quartets share the bra's record
+    const int near = LB > 1 && swap ? b : a, far = LB > 1 && swap ? a : b;
+    const double* p = V + near * M1 * TH;
+    if (LB == 0 || far == 0) {
 #pragma unroll
         for (int m = 0; m < NM; m++) v[m] = p[m * TH];
-    } else if (LB == 1 || bx == 1) {
+    } else if (LB == 1 || far == 1) {
 #pragma unroll
         for (int m = 0; m < NM; m++) v[m] = fma(R, p[m * TH], p[(M1 + m) * TH]);
-    } else {
+    } else if (LA < 2 || far == 2) {
         const double R2 = R * R, RR = R + R;
 #pragma unroll
+        for (int m = 0; m < NM; m++) v[m] = fma(R2, p[m * TH], fma(RR, p[(M1 + m) * TH], p[(2 * M1 + m) * TH]));
+    } else {  // a + 1 = 3
+        const double R3 = R * R * R, T2 = 3.0 * R * R, T1 = 3.0 * R;
+#pragma unroll
         for (int m = 0; m < NM; m++)
-            v[m] = fma(R2, p[m * TH],
-                       fma(RR, p[(M1 + m) * TH], p[(2 * M1 + m) * TH]));
+            v[m] = fma(R3, p[m * TH], fma(T2, p[(M1 + m) * TH], fma(T1, p[(2 * M1 + m) * TH], p[(3 * M1 + m) * TH])));
+    }
+}
+
+// h(c, d) from v[m], m <= LC + LD (shift_ket; `swap`: the recurrence is on d).
+template <int LC, int LD>
+__device__ __forceinline__ void kgrad_shift_ket(bool swap, double* v, double R, double* out)
+{
+    if (LD < 2 || !swap) {
+        shift_ket<LC, LD>(v, R, out);
+    } else {
+#pragma unroll
+        for (int c = 0; c <= LC; c++) {
+#pragma unroll
+            for (int d = 0; d <= LD; d++) out[c * (LD + 1) + d] = v[d];
+            if (c < LC) {
+#pragma unroll
+                for (int d = 0; d < LC + LD - c; d++) v[d] = fma(R, v[d], v[d + 1]);
+            }
+        }
     }
 }
 
 // The two centres' derivative sums of one direction for sensitivities S(c, d)
 // of the extended integrals H(c, d), c <= LC + 1.
-template <int LB, int LC, int LD, int M1, int TH>
-__device__ __forceinline__ void kgrad_direction(const double* V, int ax, int bx, double R, double Rk, double al2,
-                                                double ga2, const double* S, const double* H, double& gA, double& gC)
+template <int LA, int LB, int LC, int LD, int M1, int TH>
+__device__ __forceinline__ void kgrad_direction(const double* V, int base, int ax, int bx, double R, double Rk,
+                                                double al2, double ga2, const double* S, const double* H, double& gA, double& gC)
 {
     constexpr int D1 = LD + 1, NM = LC + LD + 1;
     double p[NM], h[(LC + 1) * D1];
-    kgrad_shift<LB, M1, NM, TH>(V, ax + 1, bx, R, p);
+    kgrad_shift<LA, LB, M1, NM, TH>(V, base & 1, ax + 1, bx, R, p);
 #pragma unroll
     for (int m = 0; m < NM; m++) p[m] *= al2;
     if (ax > 0) {
         double q[NM];
-        kgrad_shift<LB, M1, NM, TH>(V, ax - 1, bx, R, q);
+        kgrad_shift<LA, LB, M1, NM, TH>(V, base & 1, ax - 1, bx, R, q);
 #pragma unroll
         for (int m = 0; m < NM; m++) p[m] = fma(-(double)ax, q[m], p[m]);
     }
-    shift_ket<LC, LD>(p, Rk, h);
+    kgrad_shift_ket<LC, LD>(base & 2, p, Rk, h);
     double s1 = 0.0, s2 = 0.0;
 #pragma unroll
     for (int c = 0; c <= LC; c++)
@@ -105,7 +139,7 @@ __device__ __forceinline__ void kgrad_direction(const double* V, int ax, int bx,
 
 // The six sums of one root with per-component S and component masks.
 template <int LA, int LB, int LC, int LD>
-__device__ __noinline__ void kgrad_masked(const KPartnerRecs& ab, const KPartnerRecs& cd, int jr, int lr,
+__device__ __noinline__ void kgrad_masked(const KPartnerRecs& ab, const KPartnerRecs& cd, int jr, int lr, int base,
                                           const KDensity& dm, const double* Dw, const double* V, double al2,
                                           double ga2, double* g)
 {
@@ -118,7 +152,13 @@ __device__ __noinline__ void kgrad_masked(const KPartnerRecs& ab, const KPartner
     for (int x = 0; x < 3; x++) {
         R[x] = __ldg(ab.geo + (G_RX + x) * ab.sp_stride + spj);
         Rk[x] = __ldg(cd.geo + (G_RX + x) * cd.sp_stride + spl);
+        if (base & 1) R[x] = -R[x];
+        if (base & 2) Rk[x] = -Rk[x];
     }
+    const bool sb = base & 1, sd = base & 2;
+    auto value = [&](const double* Vx, int a, int b, int c, int d, int x) {
+        return krys_value<M1, TH>(Vx, sb ? b : a, sb ? a : b, sd ? d : c, sd ? c : d, R[x], Rk[x]);
+    };
     for (int ij = 0; ij < ncart(LA) * ncart(LB); ij++) {
         if (!((mj >> ij) & 1ull)) continue;
         const double Sij = isnan(suj) ? __ldg(ab.S + ij * ab.sp_stride + spj) : suj;
@@ -138,11 +178,11 @@ __device__ __noinline__ void kgrad_masked(const KPartnerRecs& ab, const KPartner
             double I[3], dA[3], dC[3];
             for (int x = 0; x < 3; x++) {
                 const double* Vx = V + x * N1 * M1 * TH;
-                I[x] = krys_value<M1, TH>(Vx, a[x], b[x], c[x], d[x], R[x], Rk[x]);
-                dA[x] = al2 * krys_value<M1, TH>(Vx, a[x] + 1, b[x], c[x], d[x], R[x], Rk[x]);
-                if (a[x] > 0) dA[x] -= a[x] * krys_value<M1, TH>(Vx, a[x] - 1, b[x], c[x], d[x], R[x], Rk[x]);
-                dC[x] = ga2 * krys_value<M1, TH>(Vx, a[x], b[x], c[x] + 1, d[x], R[x], Rk[x]);
-                if (c[x] > 0) dC[x] -= c[x] * krys_value<M1, TH>(Vx, a[x], b[x], c[x] - 1, d[x], R[x], Rk[x]);
+                I[x] = value(Vx, a[x], b[x], c[x], d[x], x);
+                dA[x] = al2 * value(Vx, a[x] + 1, b[x], c[x], d[x], x);
+                if (a[x] > 0) dA[x] -= a[x] * value(Vx, a[x] - 1, b[x], c[x], d[x], x);
+                dC[x] = ga2 * value(Vx, a[x], b[x], c[x] + 1, d[x], x);
+                if (c[x] > 0) dC[x] -= c[x] * value(Vx, a[x], b[x], c[x] - 1, d[x], x);
             }
             for (int x = 0; x < 3; x++) {
                 const double o = w * I[(x + 1) % 3] * I[(x + 2) % 3];
@@ -166,9 +206,10 @@ __device__ __forceinline__ void kgrad_lane(const KPartnerRecs& ab, const KPartne
     KVTable<N1 * M1, false, TH> Vx{V}, Vy{V + VX}, Vz{V + 2 * VX};
     krys_tables<S::NR, N1, M1, NS>(sc, root, rtab, Vx, Vy, Vz);
     const double al2 = 2.0 * sc[KF_AL * NS], ga2 = 2.0 * sc[KF_GA * NS];
+    const int base = st.base[q];
     if (st.jr[q] < 0) {
         double h[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-        kgrad_masked<LA, LB, LC, LD>(ab, cd, ~st.jr[q], st.lr[q], dm, Dw, V, al2, ga2, h);
+        kgrad_masked<LA, LB, LC, LD>(ab, cd, ~st.jr[q], st.lr[q], base, dm, Dw, V, al2, ga2, h);
 #pragma unroll
         for (int x = 0; x < 6; x++) g[x] += h[x];
         return;
@@ -197,12 +238,12 @@ __device__ __forceinline__ void kgrad_lane(const KPartnerRecs& ab, const KPartne
             int ax, ay, az;
             cart_exps(LA, a, ax, ay, az);
             double X[CE], Y[CE], Z[CE], v[M1];
-            kgrad_shift<LB, M1, M1, TH>(V, ax, bx, R[0], v);
-            shift_ket<LC + 1, LD>(v, Rk[0], X);
-            kgrad_shift<LB, M1, M1, TH>(V + VX, ay, by, R[1], v);
-            shift_ket<LC + 1, LD>(v, Rk[1], Y);
-            kgrad_shift<LB, M1, M1, TH>(V + 2 * VX, az, bz, R[2], v);
-            shift_ket<LC + 1, LD>(v, Rk[2], Z);
+            kgrad_shift<LA, LB, M1, M1, TH>(V, base & 1, ax, bx, R[0], v);
+            kgrad_shift_ket<LC + 1, LD>(base & 2, v, Rk[0], X);
+            kgrad_shift<LA, LB, M1, M1, TH>(V + VX, base & 1, ay, by, R[1], v);
+            kgrad_shift_ket<LC + 1, LD>(base & 2, v, Rk[1], Y);
+            kgrad_shift<LA, LB, M1, M1, TH>(V + 2 * VX, base & 1, az, bz, R[2], v);
+            kgrad_shift_ket<LC + 1, LD>(base & 2, v, Rk[2], Z);
             double Xb[CD], Yb[CD], Zb[CD];
 #pragma unroll
             for (int k = 0; k < CD; k++) Xb[k] = Yb[k] = Zb[k] = 0.0;
@@ -243,9 +284,9 @@ __device__ __forceinline__ void kgrad_lane(const KPartnerRecs& ab, const KPartne
                         Zb[z * D1 + dz] = fma(Tb[k], Dv[k], Zb[z * D1 + dz]);
                     }
             }
-            kgrad_direction<LB, LC, LD, M1, TH>(V, ax, bx, R[0], Rk[0], al2, ga2, Xb, X, g[0], g[3]);
-            kgrad_direction<LB, LC, LD, M1, TH>(V + VX, ay, by, R[1], Rk[1], al2, ga2, Yb, Y, g[1], g[4]);
-            kgrad_direction<LB, LC, LD, M1, TH>(V + 2 * VX, az, bz, R[2], Rk[2], al2, ga2, Zb, Z, g[2], g[5]);
+            kgrad_direction<LA, LB, LC, LD, M1, TH>(V, base, ax, bx, R[0], Rk[0], al2, ga2, Xb, X, g[0], g[3]);
+            kgrad_direction<LA, LB, LC, LD, M1, TH>(V + VX, base, ay, by, R[1], Rk[1], al2, ga2, Yb, Y, g[1], g[4]);
+            kgrad_direction<LA, LB, LC, LD, M1, TH>(V + 2 * VX, base, az, bz, R[2], Rk[2], al2, ga2, Zb, Z, g[2], g[5]);
         }
     }
 }
@@ -302,7 +343,7 @@ exchange_grad_kernel(KOutBlocks out, KPartnerRecs ab, KPartnerRecs cd, KDensity 
                 const int n = min(batch, total - w0), w = w0 + lane;
                 if (lane < n) {
                     while (s_c64[jj + 1] <= w) jj++;
-                    krys_setup<true>(ab, cd, jb + jj, c0 + w - s_c64[jj], omega, set, lane);
+                    krys_setup<true, (LB > 1), (LD > 1)>(ab, cd, jb + jj, c0 + w - s_c64[jj], omega, set, lane);
                 }
                 __syncwarp();
                 if (slot < S::QW)

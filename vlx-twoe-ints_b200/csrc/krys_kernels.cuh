@@ -73,9 +73,12 @@ struct KWarpSetup {
     double sc[KF_N * NS];
     int jsh[NS], lsh[NS];  // partner shells
     int jr[NS], lr[NS];    // records; jr < 0: no single S (per-component path)
+    uint8_t base[NS];      // gradient only: bit 0 the bra's recurrence is on b, bit 1 the ket's on d
 };
 
-template <bool GRAD, typename ST>
+// SB, SD (gradient): the recurrence of a pair may be on b (d), its tighter shell;
+// PA, AB (QC, CD) are then P - B, B - A (Q - D, D - C).
+template <bool GRAD, bool SB, bool SD, typename ST>
 __device__ __forceinline__ void krys_setup(const KPartnerRecs& ab, const KPartnerRecs& cd, int jr, int lr, double omega,
                                            ST& s, int q)
 {
@@ -105,8 +108,23 @@ __device__ __forceinline__ void krys_setup(const KPartnerRecs& ab, const KPartne
     sc[KF_I2Z * NS] = bg.i2z;
     sc[KF_I2E * NS] = kg.i2z;
     sc[KF_HI * NS] = 0.5 * inv * d2;
-    const double PA[3] = {bg.Ax, bg.Ay, bg.Az}, QC[3] = {kg.Ax, kg.Ay, kg.Az};
-    const double AB[3] = {bg.Rx, bg.Ry, bg.Rz}, CD[3] = {kg.Rx, kg.Ry, kg.Rz};
+    double PA[3] = {bg.Ax, bg.Ay, bg.Az}, QC[3] = {kg.Ax, kg.Ay, kg.Az};
+    double AB[3] = {bg.Rx, bg.Ry, bg.Rz}, CD[3] = {kg.Rx, kg.Ry, kg.Rz};
+    if (GRAD) {
+        const bool sb = SB && s.sc[KF_AL * NS + q] < 0.5 * bg.z, sd = SD && s.sc[KF_GA * NS + q] < 0.5 * kg.z;
+        s.base[q] = (uint8_t)((sb ? 1 : 0) | (sd ? 2 : 0));
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            if (sb) {
+                PA[k] += AB[k];
+                AB[k] = -AB[k];
+            }
+            if (sd) {
+                QC[k] += CD[k];
+                CD[k] = -CD[k];
+            }
+        }
+    }
 #pragma unroll
     for (int k = 0; k < 3; k++) {
         sc[(KF_PQ + k) * NS] = PQ[k];
@@ -256,10 +274,10 @@ __device__ __forceinline__ double krys_value(const double* V, int a, int b, int 
 {
     double s = 0.0;
     for (int k = 0; k <= b; k++) {
-        double cb = (k == 0 || k == b) ? 1.0 : 2.0;
+        double cb = (k == 0 || k == b) ? 1.0 : (double)b;  // binomial(b, k), b <= 3
         for (int j = 0; j < b - k; j++) cb *= R;
         for (int l = 0; l <= d; l++) {
-            double cd = (l == 0 || l == d) ? cb : cb * 2.0;
+            double cd = (l == 0 || l == d) ? cb : cb * (double)d;
             for (int j = 0; j < d - l; j++) cd *= Rk;
             s = fma(cd, V[((a + k) * M1 + c + l) * STRIDE], s);
         }
@@ -496,7 +514,7 @@ exchange_rys_kernel(KOutBlocks out, KPartnerRecs ab, KPartnerRecs cd, KGroups ga
                 const int n = __popc(taken);
                 if (grouped && qcount && lane == 0) atomicAdd(qcount, (unsigned long long)n);
                 if (mine)
-                    krys_setup<false>(ab, cd, jb + jj, l, omega, set, __popc(taken & ((1u << lane) - 1)));
+                    krys_setup<false, false, false>(ab, cd, jb + jj, l, omega, set, __popc(taken & ((1u << lane) - 1)));
                 __syncwarp();
                 if (slot < S::QW)
                     for (int q = slot; q < n; q += S::QW)

@@ -85,11 +85,11 @@ int launch_exchange_mixed(int grid, cudaStream_t st, const KOutBlocks& out, cons
 {
     constexpr int V = k_mixed(LA, LB, LC, LD);
     if constexpr (V == 3 || V == 4)
-        exchange_colc_kernel<LA, LB, LC, LD, V - 3, 1><<<grid, K_THREADS, 0, st>>>(
+        exchange_colc_kernel<LA, LB, LC, LD, V - 3><<<grid, K_THREADS, 0, st>>>(
             out, ab, cd, gab, gcd, dm, maxD, omega, thr, mat_K, tab, qk, cut, budget);
     else if constexpr (V != 0)
-        exchange_col_kernel<LA, LB, LC, LD, (V == 7 ? 4 : 0), 1><<<grid, K_THREADS, 0, st>>>(
-            out, ab, cd, dm, maxD, omega, thr, mat_K, tab, qk, cut, budget);
+        exchange_col_kernel<LA, LB, LC, LD, (V == 7 ? 4 : 0)><<<grid, K_THREADS, 0, st>>>(
+            out, ab, cd, dm, maxD, omega, thr, mat_K, tab, cut, budget);
     else
         exchange_kernel<LA, LB, LC, LD, 1><<<grid, K_THREADS, 0, st>>>(out, ab, cd, dm, maxD, omega, thr, mat_K, tab,
                                                                        qk, cut, budget);

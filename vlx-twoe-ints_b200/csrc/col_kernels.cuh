@@ -233,11 +233,12 @@ __device__ __forceinline__ void kcol_quartet(bool act, int jr, int lr, const KPa
     __syncwarp();
 }
 
-template <int LA, int LB, int LC, int LD, int ORI, int PM>
+// The FP32 quartets of a class (exchange_rys_kernel evaluates and counts the others
+// and counts these).
+template <int LA, int LB, int LC, int LD, int ORI>
 __global__ void __launch_bounds__(K_THREADS)
 exchange_col_kernel(KOutBlocks out, KPartnerRecs ab, KPartnerRecs cd, KDensity dm, double maxD, double omega,
-                    double thr, double* __restrict__ mat_K, BoysTabs tabs, unsigned long long* __restrict__ qcount,
-                    double fp32_cut, double fp32_budget)
+                    double thr, double* __restrict__ mat_K, BoysTabs tabs, double fp32_cut, double fp32_budget)
 {
     using S = KColShape<LA, LB, LC, LD, ORI>;
     constexpr int NA = S::NA, NB = S::NB, NC = S::NC, ND = S::ND;
@@ -272,20 +273,7 @@ exchange_col_kernel(KOutBlocks out, KPartnerRecs ab, KPartnerRecs cd, KDensity d
         for (int jb = a0; jb < a1; jb += K_JCHUNK) {
             const int nj = min(K_JCHUNK, a1 - jb);
             k_chunk_scan(ab, cd, jb, nj, c0, c1, mD, thr, fp32_cut, ch, a1 - a0, fp32_budget);
-            const int t64 = s_c64[nj], t32 = s_c32[nj];
-            if (qcount && PM == 0 && threadIdx.x == 0) atomicAdd(qcount, (unsigned long long)(t64 + t32));
-            const int n64 = PM == 0 ? (t64 + NW * P - 1) / (NW * P) : 0;
-            for (int it = 0; it < n64; it++) {
-                const int w = it * (NW * P) + warp * P + grp;
-                const bool act = lane_ok && w < t64;
-                const int wq = act ? w : 0;
-                const int jj = k_find(s_c64, nj, wq);
-                const int jr = jb + jj;
-                const int lr = c0 + (wq - s_c64[jj]);
-                kcol_quartet<LA, LB, LC, LD, ORI, double>(act, jr, act ? lr : c0, ab, cd, dm, omega, tabs, ln,
-                                                          lane_ok, lig, U[warp][gsel], Kacc);
-            }
-            const int n32 = PM == 1 ? (t32 + NW * P - 1) / (NW * P) : 0;
+            const int t32 = s_c32[nj], n32 = (t32 + NW * P - 1) / (NW * P);
             for (int it = 0; it < n32; it++) {
                 const int w = it * (NW * P) + warp * P + grp;
                 const bool act = lane_ok && w < t32;
@@ -470,13 +458,10 @@ __device__ __forceinline__ int kcolc_group(bool act, int jg, int lg, const KPart
 // Contracted-partner exchange kernel: exchange_col_kernel's output blocks and
 // flattened partner enumeration, over partner groups instead of records (the
 // screen on group maxima selects a superset; kcolc_group applies the exact
-// per-member screen).  PM as for coulomb_kernel, split on the group maxima.
-// Registers are capped for 3 CTAs per SM (168) for the plain plans: the
-// heaviest classes spill a little; a 2-CTA cap (no spills, fewer warps)
-// measured no faster.  The packed plans (two or five quartets per warp, the
-// tower in registers) get the 2-CTA cap.
-template <int LA, int LB, int LC, int LD, int ORI, int PM>
-__global__ void __launch_bounds__(K_THREADS, ORI >= 2 ? 2 : 3)
+// per-member screen).  The FP32 groups, split from the others on the group
+// maxima; counts its own quartets.  Registers are capped for 3 CTAs per SM (168).
+template <int LA, int LB, int LC, int LD, int ORI>
+__global__ void __launch_bounds__(K_THREADS, 3)
 exchange_colc_kernel(KOutBlocks out, KPartnerRecs ab, KPartnerRecs cd, KGroups gab, KGroups gcd, KDensity dm,
                      double maxD, double omega, double thr, double* __restrict__ mat_K, BoysTabs tabs,
                      unsigned long long* __restrict__ qcount, double fp32_cut, double fp32_budget)
@@ -516,19 +501,7 @@ exchange_colc_kernel(KOutBlocks out, KPartnerRecs ab, KPartnerRecs cd, KGroups g
             const int nj = min(K_JCHUNK, a1 - jb);
             k_chunk_scan(gab.q, gcd.q, jb, nj, c0, c1, mD, thr, fp32_cut, ch, gab.qa, gcd.qpre, a1 - a0,
                          fp32_budget);
-            const int t64 = s_c64[nj], t32 = s_c32[nj];
-            const int n64 = PM == 0 ? (t64 + NW * P - 1) / (NW * P) : 0;
-            for (int it = 0; it < n64; it++) {
-                const int w = it * (NW * P) + warp * P + grp;
-                const bool act = lane_ok && w < t64;
-                const int wq = act ? w : 0;
-                const int jj = k_find(s_c64, nj, wq);
-                const int np = kcolc_group<LA, LB, LC, LD, ORI, double>(
-                    act, jb + jj, c0 + (wq - s_c64[jj]), ab, cd, gab, gcd, dm, mD, thr, omega, tabs, ln, lane_ok,
-                    lig, U[warp][gsel], Kacc);
-                if (act && lig == 0) nq += (unsigned long long)np;
-            }
-            const int n32 = PM == 1 ? (t32 + NW * P - 1) / (NW * P) : 0;
+            const int t32 = s_c32[nj], n32 = (t32 + NW * P - 1) / (NW * P);
             for (int it = 0; it < n32; it++) {
                 const int w = it * (NW * P) + warp * P + grp;
                 const bool act = lane_ok && w < t32;

@@ -326,11 +326,12 @@ def k_fits(plan: ColumnPlan) -> bool:
 
 
 def k_variants(la, lb, lc, ld, spilling=False):
-    """Exchange kernel variants (schedule values) built for a class: 0 thread
+    """Exchange schedule values that name a plan which fits a class: 0 thread
     per quartet (unless its code spills), 1 / 2 column with bra / ket lanes,
-    3 / 4 the contracted-partner column kernels, 5 / 6 packed column plans
-    (kinds 2 / 3), 7 / 8 packed plans on the second centre (kinds 4 / 5),
-    9..12 the contracted-partner kernels of kinds 2..5."""
+    3 / 4 with contracted partners, 5 / 6 packed column plans (kinds 2 / 3),
+    7 / 8 packed plans on the second centre (kinds 4 / 5), 9..12 kinds 2..5 with
+    contracted partners.  The library accepts them all; which kernel runs is a
+    rule of the class (k_rys and k_mixed of launch.cuh), not of the value."""
     out = [] if spilling else [0]
     for ori in (0, 1):
         if k_fits(ColumnPlan(la, lb, lc, ld, ori)):
@@ -345,12 +346,13 @@ def _yname(y):
     return f"{y[0]}{y[1]}{y[2]}"
 
 
-def emit_cuda(plan: ColumnPlan, T: str = "double", with_tables: bool = True, acc: bool = False):
+def emit_cuda(plan: ColumnPlan, T: str | None = "double", with_tables: bool = True, acc: bool = False):
     """Device function col_vrr<LA,LB,LC,LD,ORI>(q, F, ln, out): out[t] = [x|y_t]^0 for
     the lane's component x and the step-side targets y_t (plan.ytargets order).
     Also the lane table col_tab<...> (plan.NL rows of 20 int8).  With acc, the
     function is col_vrr_acc(q, F, ln, out, w) and adds w * [x|y_t]^0 to out[t]
-    (primitive quartets summed before the HRR)."""
+    (primitive quartets summed before the HRR).  T None: the flags alone, for a
+    plan that no kernel runs."""
     la, lb, lc, ld = plan.cls
     ori = plan.ori
     TT = T
@@ -382,6 +384,8 @@ def emit_cuda(plan: ColumnPlan, T: str = "double", with_tables: bool = True, acc
         L.append(f"    static constexpr bool K_FITS = {'true' if k_fits(plan) else 'false'};"
                  f"  // exchange kernel shared memory: {k_smem_bytes(plan)} bytes")
         L.append("};")
+        if TT is None:
+            return "\n".join(L)
         L.append(f"__device__ const int8_t col_tab_{plan.name()}[{plan.NL}][20] = {{" + ", ".join(rows) + "};")
         L.append(f"template <> __device__ __forceinline__ const int8_t* col_tab_ptr<{T}>() "
                  f"{{ return &col_tab_{plan.name()}[0][0]; }}")
@@ -478,6 +482,11 @@ def emit_cuda(plan: ColumnPlan, T: str = "double", with_tables: bool = True, acc
     return "\n".join(L)
 
 
+# (type, acc) of the device functions of each plan kind that some kernel calls
+# (class_launch.cuh): Coulomb columns in both precisions, exchange in FP32.
+EMITTED = {0: [("double", False), ("float", False), ("float", True)], 1: [("float", True)], 4: [("float", False)]}
+
+
 def column_classes():
     """Classes generated with column kernels (both orientations)."""
     out = []
@@ -529,16 +538,10 @@ def main(outdir):
         parts = ["// Generated by gen_column.py -- do not edit.", "#pragma once", "namespace vlxb {", ""]
         for ori in PLAN_KINDS:
             plan = ColumnPlan(*cls, ori)
-            parts.append(emit_cuda(plan, "double", True))
-            parts.append("")
-            if not plan.applies:
-                continue
-            parts.append(emit_cuda(plan, "float", False))
-            parts.append("")
-            parts.append(emit_cuda(plan, "double", False, acc=True))
-            parts.append("")
-            parts.append(emit_cuda(plan, "float", False, acc=True))
-            parts.append("")
+            forms = EMITTED.get(ori, [(None, False)])
+            for n, (T, acc) in enumerate(forms if plan.applies else forms[:1]):
+                parts.append(emit_cuda(plan, T, n == 0, acc=acc))
+                parts.append("")
         parts.append("}  // namespace vlxb")
         text = "\n".join(parts) + "\n"
         path = os.path.join(outdir, f"col_{name}.cuh")

@@ -562,7 +562,7 @@ def run_batched(args, L, dev, cut):
     """Batched leg: many small molecules (1 atom per 30 bohr^3, the 4s3p2d
     recipe), all resident.  plain = the molecules' FP64 builds one after the
     other through the C ABI; batched = one CUDA graph replay per iteration (all
-    molecules' class calls on 8 capture streams), FP64 and with FP32 below
+    molecules' builds on 8 capture streams), FP64 and with FP32 below
     `cut`.  Device time with CUDA events; builds/s = molecules/s."""
     import torch
     from vlxb import basis, fock, lists
@@ -603,7 +603,7 @@ def run_batched(args, L, dev, cut):
     t_bmx = timed(bb.run, 3)
     L.set_fp32_cut(0.0)
     got = energies()
-    # fused: one class call per class for each union of up to --fuse-group
+    # fused: one build call for each union of up to --fuse-group
     # molecules, one graph per iteration
     from vlxb.batchfuse import FusedBatchGroups
 
@@ -639,9 +639,9 @@ def run_batched(args, L, dev, cut):
             "max_abs_dK": max(float(np.abs(a[1] - b[1]).max()) for a, b in zip(got, ref)),
             "max_abs_dE_Eh": max(abs(a[2] - b[2]) for a, b in zip(got, ref)),
             "timing": ("device (CUDA events), best of 2-3 iterations; plain = sequential per-molecule builds; "
-                       "batched = every molecule's class calls in one graph on 8 streams; fused = one class "
-                       "call per class per union of up to --fuse-group molecules (vlxb_coulombBatch / "
-                       "vlxb_exchangeBatch), one graph")}
+                       "batched = every molecule's build in one graph on 8 streams; fused = one build call "
+                       "per union of up to --fuse-group molecules (vlxb_fockBuild; class by class through "
+                       "vlxb_coulombBatch / vlxb_exchangeBatch above its memory bound), one graph")}
 
 
 def run_served(args, L, dev, cut):

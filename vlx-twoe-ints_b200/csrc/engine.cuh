@@ -298,10 +298,12 @@ struct PrepShare {
     bool prepare_only = false;  // the class calls prepare their lists and launch nothing
 };
 
-// Kernel variant per class: kind 0 = Coulomb (0 thread-per-quartet, 1 column),
-// kind 1 = exchange (0 thread-per-quartet, 1 column with bra lanes, 2 column
-// with ket lanes).  Defaults come from the generator; the autotuner
-// overrides them through vlxb_setSchedule.
+// Schedule value per class.  Kind 0 = Coulomb: the kernel variant (0 thread per
+// quartet, 1 column, 2 McMurchie-Davidson, 3 thread with TMA-staged kets) of the
+// classes without a Rys kernel, and of the others' FP32 quartets.  Kind 1 =
+// exchange: kept and returned, but each class has one kernel (launch.cuh).
+// Defaults come from the generator; the autotuner overrides them through
+// vlxb_setSchedule.
 int schedule_get(int kind, int la, int lb, int lc, int ld);
 int schedule_set(int kind, int la, int lb, int lc, int ld, int variant);
 

@@ -499,11 +499,9 @@ def column_classes():
 
 
 def default_schedule():
-    """Kernel variant per class before autotuning.  J: 0 thread-per-quartet,
-    1 column.  K: 0 thread-per-quartet, 1 column with bra lanes, 2 column with
-    ket lanes.  Column kernels for the classes whose thread kernels spill
-    (total angular momentum >= 6 for J, >= 5 for K); for K the orientation that
-    keeps more lanes busy and fits in shared memory."""
+    """Schedule value per class before autotuning.  J: 0 thread-per-quartet,
+    1 column, for the classes whose thread kernels spill (total angular momentum
+    >= 6).  K: a plan that fits the class; the value selects nothing (k_variants)."""
     j, k = {}, {}
     for cls in column_classes():
         L = sum(cls)

@@ -19,8 +19,9 @@
 // (some components below the threshold) has its density rebuilt there by its
 // lane with the exact per-component screen.
 //
-// Bound: FP64 issue (lane efficiency 30 of 32 at worst), then for kets with two
-// d shells the rebuilding of screened densities.  10 atoms 4s3p2d, ms per class
+// Bound: FP64 issue (pipe 40 to 51 % busy, lane efficiency 30 of 32 at worst); for
+// kets with two d shells the unrolled rebuilding of screened densities, which
+// waits for instructions as often as for results.  10 atoms 4s3p2d, ms per class
 // call: (DD|DD) 7.9 -> 1.8, (PD|DD) 9.8 -> 2.6, (DD|PD) 6.0 -> 1.7, (PD|PD) 5.5
 // -> 2.8; the gradient of all classes 444 -> 78.
 //
@@ -53,7 +54,10 @@ struct JRysShape {
     static constexpr int NW = J_THREADS / 32;
     static constexpr int NHB = nherm(LE), NHK = nherm(LF);
     static constexpr int BATCH = 32 / QW * QW;  // kets set up together
-    // CTAs per SM: the NHB partials are the registers that count
+    // CTAs per SM: the NHB partials are the registers that count.  8 atoms 4s3p2d,
+    // ms for the Coulomb classes / the gradient classes of one NHB with 2, 3 and 4
+    // CTAs: NHB 10 5.1 4.3 4.1 / 9.2 7.9 7.2; 20 5.2 4.5 4.3 / 14.8 12.8 11.9;
+    // 35 3.2 3.1 3.6 / 10.3 9.2 10.3; 56 (gradient) 6.3 7.8 11.3.
     static constexpr int MINB = NHB > 20 ? 2 : (NHB > 12 ? 3 : 4);
 };
 

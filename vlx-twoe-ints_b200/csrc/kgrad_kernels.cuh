@@ -23,10 +23,10 @@
 // Loops over b and a are not unrolled; the 27 sensitivities of one (a, b), the
 // 1-D integrals and the six sums are all that a lane keeps in registers.  The
 // VRR table in shared memory has one more row and column than the energy's.
-// Bound: FP64 issue and shared-memory loads together, with eight warps per SM
-// (255 registers).  5 atoms 4s3p2d: 717 -> 70 ms for the 54 classes against the
-// Hermite-table kernel it replaces (shared-memory bound at 91 %), DDDD class
-// call 4.0, PDDD 4.2 ms with the list preparation.
+// Bound: FP64 issue and the latency of dependent multiply-adds, with eight warps
+// per SM (255 registers; seven for two d-d pairs): FP64 pipe 42 to 50 % busy, the
+// shared-memory pipe 27 to 52 %.  5 atoms 4s3p2d, all 54 classes: 741 ms with the
+// Hermite-table kernel it replaces (shared-memory bound at 91 %), 54.5 ms now.
 //
 // Layout follows the exchange kernels: one CTA per (i, k) primitive shell
 // block, fixed-order reduction, no atomics on the output.  Screening is the K
@@ -44,7 +44,10 @@ struct KGradShape {
     static constexpr int L = LA + LB + LC + LD;
     static constexpr int NR = (L + 1) / 2 + 1;
     static constexpr int QW = 32 / NR;
-    static constexpr int BATCH = L >= 3 ? QW : 32 / QW * QW;  // quartets set up together
+    // quartets set up together: as many as one pass takes, for shared memory's sake
+    // (full batches up to L = 4: 4 atoms 4s3p2d, 3.9 and 5.9 ms for the classes of
+    // L = 3 and 4 against 4.0 and 5.7); below L = 3 either way the same
+    static constexpr int BATCH = L >= 3 ? QW : 32 / QW * QW;
     static constexpr int N1 = LA + LB + 2, M1 = LC + LD + 2;
     // two CTAs of four warps (255 registers); the tables of two d-d pairs leave
     // room for seven warps, taken as one CTA

@@ -18,6 +18,11 @@
 // quartet by one lane for up to 32 quartets at a time and read back from
 // shared memory by the lanes of the roots.
 //
+// Precision: the shift to the second centre loses digits from a diffuse to a
+// tight shell, as a horizontal recurrence does, but fewer: 1.3e-15 of the Schwarz
+// bound (root mean square over d-rich quartets, exponents 0.4 to 3, a box of 4
+// bohr) against 4.6e-15 for VRR and HRR as in the thread and column kernels.
+//
 // Bound: FP64 issue.  (SD|DD) on 10 atoms 4s3p2d runs the FP64 pipe at 57 %
 // ((PD|DP) 65 %), the rest being arithmetic latency that two warps per scheduler do not
 // cover, with two CTAs of 128 threads per SM (registers); with the tables in shared
@@ -49,9 +54,10 @@ struct KRysShape {
     static constexpr int N1 = LA + LB + 1, M1 = LC + LD + 1;
     static constexpr int NAC = ncart(LA) * ncart(LC);
     // The VRR tables (3 N1 M1 values), the (a, c) partials and the x and y
-    // slices stay in registers with the loop over b unrolled; (DD|DD) alone
-    // does not fit and keeps the tables in shared memory, b not unrolled.  10
-    // atoms 4s3p2d, registers / shared memory, ms: (PD|DD) 9.2 / 11.7, (PD|PD)
+    // slices stay in registers with the loop over b unrolled.  Where they do not
+    // fit, (PD|DD), (DP|DD) and (DD|DP) spill 0.65 to 1.1 KB and are faster all
+    // the same; (DD|DD), 4 KB, keeps the tables in shared memory, b not unrolled.
+    // 10 atoms 4s3p2d, registers / shared memory, ms: (PD|DD) 9.2 / 11.7, (PD|PD)
     // 3.8 / 5.8, (DD|DP) 6.1 / 6.6, (DD|DD) 27.6 / 10.3.
     static constexpr bool REG = L < 8;
     static constexpr int SMEM_ROWS = REG ? 0 : 3 * N1 * M1;

@@ -1,8 +1,8 @@
 """Batched J/K builds of many independent molecules, one CUDA graph per iteration.
 
 Every molecule keeps its reference-format lists resident on the device
-(`DeviceLists`).  One iteration = the 36 Coulomb and 54 exchange class calls of
-every molecule.  All of them are captured once into a single CUDA graph: the
+(`DeviceLists`).  One iteration = the 36 Coulomb and 54 exchange classes of
+every molecule, a build call each.  All of them are captured once into a single CUDA graph: the
 molecules are spread round-robin over `streams` capture streams forked from
 and joined back into the capture origin, so their kernels are independent
 graph branches that run concurrently and fill the GPU (a 3-atom molecule's

@@ -1,12 +1,13 @@
-"""Fused batches: one class call per class for many molecules.
+"""Fused batches: each class once for many molecules.
 
-`batch.BatchedBuilder` replays every molecule's 90 class calls inside one
-CUDA graph.  `FusedBatch` instead concatenates the molecules' reference-format
-lists into one union (primitives of each type numbered molecule after
-molecule, no pair across two molecules) and runs each class ONCE for the whole
-batch through `vlxb_coulombBatch` / `vlxb_exchangeBatch`: one device-side
-regrouping and one persistent kernel launch (two with FP32 below a cutoff)
-per class per iteration, whatever the number of molecules.
+`batch.BatchedBuilder` replays every molecule's build inside one CUDA graph.
+`FusedBatch` instead concatenates the molecules' reference-format lists into one
+union (primitives of each type numbered molecule after molecule, no pair across
+two molecules) and runs each class ONCE for the whole batch: one
+`vlxb_fockBuild` over the union regroups each list once and launches one
+persistent kernel (two with FP32 below a cutoff) per class per iteration,
+whatever the number of molecules; above its memory bound the classes go one by
+one through `vlxb_coulombBatch` / `vlxb_exchangeBatch`.
 
 Molecule boundaries reach the kernels as data: a Coulomb bra only meets the
 kets of its own molecule (per-molecule ket segments sorted by bound), and an
@@ -263,7 +264,7 @@ class FusedBatch:
         self.L.check(self.L.cdll.vlxb_exchangeBatch(*l4, ctypes.byref(c), stream), f"vlxb_exchangeBatch {cls}")
 
     def issue(self, stream=None):
-        """Zero the outputs and queue one batched iteration (90 class calls)."""
+        """Zero the outputs and queue one batched iteration."""
         st = stream or torch.cuda.current_stream(self.device)
         with torch.cuda.stream(st):
             for t in list(self.matJ.values()) + list(self.matK.values()):

@@ -1,10 +1,11 @@
 """J/K builds through the C ABI (the drop-in path).
 
 `DeviceLists` holds the reference-format arrays of one system on the GPU
-(torch tensors used as plain device buffers); `build_jk` calls the 36 Coulomb
-and 54 exchange entry points exactly as the reference's host would call the
-emitted kernels, accumulating mat_J per bra list ("ab") and mat_K per (i, k)
-list ("ac").
+(torch tensors used as plain device buffers); `build_jk` runs the 36 Coulomb
+and 54 exchange classes in one call (vlxb_fockBuild), or entry point by entry
+point, as the reference's host would call the emitted kernels, where that call
+declines; it accumulates mat_J per bra list ("ab") and mat_K per (i, k) list
+("ac").
 """
 from __future__ import annotations
 
@@ -194,7 +195,8 @@ def build_jk(dl: DeviceLists, stream: torch.cuda.Stream | None = None, omega: fl
     """Launch every J and K class through the C ABI on `stream` (asynchronous):
     the s, p and d classes in one vlxb_fockBuild, which prepares each list once,
     classes with f shells through their entry points.  Returns (matJ, matK):
-    device tensors in prim-cart pair space."""
+    device tensors in prim-cart pair space (made and zeroed on `stream` unless
+    given)."""
     L = lib()
     if stream is None:
         stream = torch.cuda.current_stream(dl.device)

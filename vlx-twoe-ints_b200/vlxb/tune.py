@@ -3,7 +3,8 @@
 For each class and each compiled variant (thread-per-quartet, column,
 McMurchie-Davidson, thread-per-quartet with TMA-staged kets) the class
 entry point is timed with CUDA events on a given system's lists (best of
-`reps`), and the fastest variant is kept; every K class has one kernel.  The result is a JSON schedule
+`reps`), and the fastest variant is kept; every K class has one kernel, its
+number is carried along.  The result is a JSON schedule
 ({"J": {class: variant}, "K": {...}}) that `apply_schedule` loads into the
 library's table (vlxb_setSchedule).  Every variant computes the same J/K to
 rounding, so the choice only changes speed.
@@ -25,7 +26,8 @@ DEFAULT_SCHEDULE = os.path.join(HERE, "schedule_b200.json")
 
 # Thread-per-quartet kernels whose code does not fit in registers (ptxas
 # keeps them at 32 registers with 15-87 KB of local memory per thread); they
-# are 5-10x slower than the column kernels and are not timed.
+# are 5-10x slower than the column kernels and are not timed (K: not offered as
+# a schedule value; those classes run by Rys quadrature).
 SPILLING_THREAD_KERNELS = {
     "J": {"dddd"},
     "K": {"ddds", "dpdp", "ppdd", "pddp", "sddd", "pdpd", "dpdd", "dddp", "pddd", "dddd"},

@@ -119,3 +119,18 @@ def test_exchange_gradient_keeps_its_digits(cls, alpha0, ratio, side, limit):
             if bound[x] > 0.0:
                 worst = max(worst, abs(float(exact[x] - float(got[x]))) / (EPS * bound[x]))
     assert 0.0 < worst <= limit, worst
+
+
+@pytest.mark.parametrize("omega", [0.0, 0.4])
+def test_exchange_gradient_per_component_path_on_either_centre(omega):
+    """Records without a common S (the per-component path) whose pairs have a
+    tighter shell on either centre, so that the recurrence is on b or d for some;
+    FP64 bar of the suite, 1e-10 of the largest element."""
+    from test_gpu_rys import close, system as rys_system
+    from vlxb import gradient
+
+    wl, rl = rys_system(2, 2, 2.0, 11, True)
+    dl = fock.to_device(rl)
+    g = gradient.ExchangeGradient(dl, wl.mol).compute(omega=omega).cpu().numpy()
+    go, _ = helpers.oracle_exchange_gradient(rl, wl.mol.natoms, omega)
+    assert float(np.abs(go).max()) > 1e-3 and close(g, go), float(np.abs(g - go).max())
